@@ -88,8 +88,53 @@ __device__ __forceinline__ double compat_fac(int k, int ng, double b, double nor
   return normfac * exp(K * K * b * 0.25);
 }
 
+// fac(k0 + r stride), r = 0..R-1, of one radix-R butterfly's outputs (R = 16,
+// or the only stage's radix).  Float evaluates each (one approximate exp).
+// Double takes an exp at every fourth output only and forms the three between
+// by exp(c (k + d)^2) = exp(c k^2) exp(2 c k d) exp(c d^2), c = b / (4 ng^2):
+// five FP64 exps per butterfly instead of sixteen, at most four roundings each
+// (the FP64 pipe bounds the double row pass).  hs: exp(c j d^2)
+// for the butterfly's output stride d and j = 1, 4, 9, 8 (the last: the growth
+// of exp(2 c k d) from one anchor to the next), per CTA.
+__device__ __forceinline__ void compat_fac_steps(int stride, int ng, double b, double *hs) {
+  if (threadIdx.x < 4) {
+    const double D = (double)stride / (double)ng;
+    const int j = threadIdx.x;
+    hs[j] = exp(b * 0.25 * D * D * (double)(j == 0 ? 1 : (j == 1 ? 4 : (j == 2 ? 9 : 8))));
+  }
+}
+__device__ __forceinline__ void compat_fac_steps(int, int, float, float *) {}
+template <int R>
+__device__ __forceinline__ void compat_facs(int k0, int stride, int ng, float b, float normfac, const float *,
+                                            float *f) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) f[r] = compat_fac(k0 + r * stride, ng, b, normfac);
+}
+template <int R>
+__device__ __forceinline__ void compat_facs(int k0, int stride, int ng, double b, double normfac, const double *hs,
+                                            double *f) {
+  if constexpr (R < 16) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) f[r] = compat_fac(k0 + r * stride, ng, b, normfac);
+  } else {
+    const double inv = 1.0 / (double)ng, D = (double)stride * inv, c = b * 0.25;
+    const double h1 = hs[0], h2 = hs[1], h3 = hs[2], g4 = hs[3];
+    double g = exp(2.0 * c * ((double)k0 * inv) * D);  // exp(2 c k d) at the anchor
+#pragma unroll
+    for (int a = 0; a < R; a += 4) {
+      const double K = (double)(k0 + a * stride) * inv;
+      const double e = normfac * exp(K * K * c);
+      const double g2 = g * g;
+      f[a] = e;
+      f[a + 1] = e * (g * h1);
+      f[a + 2] = e * (g2 * h2);
+      f[a + 3] = e * (g2 * g * h3);
+      g *= g4;
+    }
+  }
+}
+
 __device__ __forceinline__ float cpow(float a, int m) { return powf(a, m); }
-__device__ __forceinline__ double cpow(double a, int m) { return pow(a, m); }
 
 // Reference cell j = (int)((x + 0.5) * (ng - 1)) (double arithmetic,
 // src/gridding.cu:43,93) and the tap bounds of :53-58.  Returns false when the
@@ -192,10 +237,56 @@ __device__ __forceinline__ void compat_coefs(const typename RecOf<T>::type &rc, 
   }
 }
 
-constexpr int kCompatThreads = 256;
+// All taps of one record into the tile: cell m0 + m for m in [lo, hi), scaled
+// by sc.  Float: powf of the fast-math build per tap, two approximate
+// instructions, the reference's own bits.
+template <typename A>
+__device__ __forceinline__ void compat_record(A *acc, int m0, int lo, int hi, int rf, float E1, float E2, float val,
+                                              float sc, const float *e3, const float *E3g) {
+  for (int m = lo; m < hi; ++m) {
+    const int mp = m < 0 ? -m : m;
+    const float e3m = mp < kCompatMaxRf ? e3[mp] : E3g[mp];
+    const float w = val * (E1 * cpow(E2, m) * e3m);
+    FixAccWide<float>::add(acc + m0 + m, FixAccWide<float>::to_fix(w * sc));
+  }
+}
+// Double: E2^m by a running product up and down from m = 0, kept as an
+// unevaluated sum (p + pl) with FMA-exact products, so each power is the
+// correctly rounded one to a few 2^-100 before it enters the tap; seven FP64
+// operations per tap where pow() takes over a hundred.  The FP64 pipe (two
+// FMA per clock and SM) bounds this kernel (1e5 samples on 2^19 cells: the
+// whole transform 746 us with pow(), 588 of them here, and an exp per output;
+// 193 us now).  The two chains are independent, which hides half of the FP64
+// latency.
+template <typename A>
+__device__ __forceinline__ void compat_record(A *acc, int m0, int lo, int hi, int rf, double E1, double E2,
+                                              double val, double sc, const double *e3, const double *E3g) {
+  const double vs = val * sc;
+  if (lo <= 0 && 0 < hi) FixAccWide<double>::add(acc + m0, FixAccWide<double>::to_fix(vs * (E1 * e3[0])));
+  const double q = 1.0 / E2, ql = fma(-q, E2, 1.0) * q;  // 1/E2 = q + ql
+  double p = 1.0, pl = 0.0, r = 1.0, rl = 0.0;
+#pragma unroll 2
+  for (int k = 1; k < rf; ++k) {
+    const double t = E1 * (k < kCompatMaxRf ? e3[k] : E3g[k]);
+    const double p1 = p * E2, r1 = r * q;
+    pl = fma(pl, E2, fma(p, E2, -p1));
+    rl = fma(rl, q, fma(r, ql, fma(r, q, -r1)));
+    p = p1;
+    r = r1;
+    if (lo <= k && k < hi) FixAccWide<double>::add(acc + m0 + k, FixAccWide<double>::to_fix(vs * fma(t, pl, t * p)));
+    if (lo <= -k && -k < hi)
+      FixAccWide<double>::add(acc + m0 - k, FixAccWide<double>::to_fix(vs * fma(t, rl, t * r)));
+  }
+}
 
-template <typename T, bool BOOT>
-__global__ void __launch_bounds__(kCompatThreads) k_grid_compat(const typename RecOf<T>::type *__restrict__ recs,
+// Threads per tile: 256, or 1024 where the tiles and resamples of the call do
+// not fill the SMs twice (a tile's records are then the serial chain: 128
+// tiles of 780 records each for 1e5 samples on 2^19 cells).
+constexpr int kCompatThreads = 256;
+constexpr int kCompatThreadsFew = 1024;
+
+template <typename T, bool BOOT, int NT>
+__global__ void __launch_bounds__(NT) k_grid_compat(const typename RecOf<T>::type *__restrict__ recs,
                                                                 const int *__restrict__ off,
                                                                 typename CxOf<T>::type *f_hat, int ng,
                                                                 const typename FpOf<T>::type *fp,
@@ -207,8 +298,8 @@ __global__ void __launch_bounds__(kCompatThreads) k_grid_compat(const typename R
   A *acc = reinterpret_cast<A *>(smem_raw);
   T *e3 = reinterpret_cast<T *>(acc + (1 << kCompatLogTL));
   int *hist = reinterpret_cast<int *>(e3 + kCompatMaxRf);
-  __shared__ float red[kCompatThreads / 32];
-  __shared__ int redi[kCompatThreads / 32];
+  __shared__ float red[NT / 32];
+  __shared__ int redi[NT / 32];
   __shared__ T scale_s;
   const int tile = blockIdx.x, slab = blockIdx.y;
   const int base = tile << kCompatLogTL;
@@ -219,14 +310,14 @@ __global__ void __launch_bounds__(kCompatThreads) k_grid_compat(const typename R
   int logBS = 4;
   while ((1 << logBS) < 2 * rf) ++logBS;
   const int NB = ((tl + 2 * rf) >> logBS) + 1;
-  for (int c = threadIdx.x; c < tl; c += kCompatThreads) acc[c] = 0;
-  for (int m = threadIdx.x; m < rf && m < kCompatMaxRf; m += kCompatThreads) e3[m] = E3g[m];
-  for (int q = threadIdx.x; q < NB; q += kCompatThreads) hist[q] = 0;
+  for (int c = threadIdx.x; c < tl; c += NT) acc[c] = 0;
+  for (int m = threadIdx.x; m < rf && m < kCompatMaxRf; m += NT) e3[m] = E3g[m];
+  for (int q = threadIdx.x; q < NB; q += NT) hist[q] = 0;
   __syncthreads();
   const int r0 = off[tile], r1 = off[tile + 1];
   // bound pass: records per bucket and the largest |value| (NaN if any is not finite)
   float ym = 0.f;
-  for (int r = r0 + threadIdx.x; r < r1; r += kCompatThreads) {
+  for (int r = r0 + threadIdx.x; r < r1; r += NT) {
     const Rec rc = recs[r];
     atomicAdd(&hist[(rc.cell - base + rf) >> logBS], 1);
     T E1, E2, val;
@@ -235,7 +326,7 @@ __global__ void __launch_bounds__(kCompatThreads) k_grid_compat(const typename R
   }
   __syncthreads();
   int hmax = 0;
-  for (int q = threadIdx.x; q < NB; q += kCompatThreads) hmax = max(hmax, hist[q]);
+  for (int q = threadIdx.x; q < NB; q += NT) hmax = max(hmax, hist[q]);
   for (int o = 16; o > 0; o >>= 1) {
     hmax = max(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
     const float u = __shfl_xor_sync(0xffffffffu, ym, o);
@@ -250,7 +341,7 @@ __global__ void __launch_bounds__(kCompatThreads) k_grid_compat(const typename R
     int h = 0;
     float v = 0.f;
     bool bad = false;
-    for (int w = 0; w < kCompatThreads / 32; ++w) {
+    for (int w = 0; w < NT / 32; ++w) {
       h = max(h, redi[w]);
       bad |= isnan(red[w]);
       v = fmaxf(v, red[w]);
@@ -266,7 +357,7 @@ __global__ void __launch_bounds__(kCompatThreads) k_grid_compat(const typename R
   __syncthreads();
   const T sc = scale_s;
   if (sc > (T)0) {
-    for (int r = r0 + threadIdx.x; r < r1; r += kCompatThreads) {
+    for (int r = r0 + threadIdx.x; r < r1; r += NT) {
       const Rec rc = recs[r];
       const int j = rc.cell;
       int ms = -rf + 1, me = rf;
@@ -275,22 +366,17 @@ __global__ void __launch_bounds__(kCompatThreads) k_grid_compat(const typename R
       T E1, E2, val;
       compat_coefs<T, BOOT>(rc, E1g, E2g, y, n, seed, slab, E1, E2, val);
       const int lo = max(ms, base - j), hi = min(me, base + tl - j);
-      for (int m = lo; m < hi; ++m) {
-        const int mp = m < 0 ? -m : m;
-        const T e3m = mp < kCompatMaxRf ? e3[mp] : E3g[mp];
-        const T w = val * (E1 * cpow(E2, m) * e3m);
-        FA::add(&acc[j + m - base], FA::to_fix(w * sc));
-      }
+      compat_record(acc, j - base, lo, hi, rf, E1, E2, val, sc, e3, E3g);
     }
   }
   __syncthreads();
   typename CxOf<T>::type *out = f_hat + (int64_t)slab * ng + base;
   if (isnan(sc)) {  // a non-finite value: the tile is NaN, as the float sums would spread it
-    for (int c = threadIdx.x; c < tl; c += kCompatThreads) out[c].x += (T)NAN;
+    for (int c = threadIdx.x; c < tl; c += NT) out[c].x += (T)NAN;
     return;
   }
   const T inv = sc > (T)0 ? (T)1 / sc : (T)0;
-  for (int c = threadIdx.x; c < tl; c += kCompatThreads) {
+  for (int c = threadIdx.x; c < tl; c += NT) {
     const A v = acc[c];
     if (v != 0) out[c].x += (T)v * inv;
   }
@@ -375,13 +461,15 @@ template <typename T, int LOG1> struct CtFacDst {
   typename CxOf<T>::type *p;  // slab
   int ng, r0, norm;
   T b, nf;
+  const T *hs;  // compat_fac_steps
   template <int R, int LOGNS>
   __device__ __forceinline__ void store(int seq, int idxD, typename CxOf<T>::type *v) const {
+    const int k0 = r0 + seq + (idxD << LOG1);
+    constexpr int S = 1 << (LOGNS + LOG1);
+    T fac[R];
+    if (norm) compat_facs<R>(k0, S, ng, b, nf, hs, fac);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int k = r0 + seq + ((idxD + (r << LOGNS)) << LOG1);
-      p[k] = norm ? cscale(v[r], compat_fac(k, ng, b, nf)) : v[r];
-    }
+    for (int r = 0; r < R; ++r) p[k0 + r * S] = norm ? cscale(v[r], fac[r]) : v[r];
   }
 };
 
@@ -397,7 +485,10 @@ __global__ void __launch_bounds__(PassCfg<T>::THREADS) k_ct_rowpass_compat(const
   C *s = reinterpret_cast<C *>(smem_raw);
   const int r0 = blockIdx.x << LOGB;
   CtRowSrc<T, LOG2> src{in + blockIdx.y * slab_stride + ((int64_t)r0 << LOG2)};
-  CtFacDst<T, LOG1> dst{out + blockIdx.y * slab_stride, 1 << LOGL, r0, norm, fp->b, fp->normfac};
+  __shared__ T hs[4];  // read by the storing stage, after at least one barrier
+  static_assert(LOG2 > 4, "the row transform has more than one stage");
+  compat_fac_steps(1 << (last_logns<LOG2>() + LOG1), 1 << LOGL, fp->b, hs);
+  CtFacDst<T, LOG1> dst{out + blockIdx.y * slab_stride, 1 << LOGL, r0, norm, fp->b, fp->normfac, hs};
   // rows are read point-fastest (contiguous), outputs written row-fastest
   ct_fft<T, LOG2, LOGB, true, false, true>(s, f.tw2, src, dst);
 }
@@ -680,10 +771,13 @@ int compat_grid(const T *x, const T *y, typename CxOf<T>::type *f_hat, int n, in
   CUNA_TRY(compat_bin<T>(x, y, n, ng, dfp, boot, cw, st));
   Rec *recs = (Rec *)cw.recs;
   const size_t smg = compat_grid_smem<T>();
-  if (boot)
-    k_grid_compat<T, true><<<dim3(ntiles, nbs), 256, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
-  else
-    k_grid_compat<T, false><<<dim3(ntiles, 1), 256, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
+  const dim3 gg(ntiles, boot ? nbs : 1);
+  constexpr int NF = kCompatThreadsFew, NM = kCompatThreads;
+  const bool few = (int64_t)gg.x * gg.y < 2 * (int64_t)device_sm_count();
+  if (boot && few) k_grid_compat<T, true, NF><<<gg, NF, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
+  else if (boot) k_grid_compat<T, true, NM><<<gg, NM, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
+  else if (few) k_grid_compat<T, false, NF><<<gg, NF, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
+  else k_grid_compat<T, false, NM><<<gg, NM, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
   CUNA_CK(cudaGetLastError());
   return CUNA2_SUCCESS;
 }
@@ -1065,7 +1159,7 @@ int compat_adjoint_noalloc(const float *x, const float *y, float2 *f_hat, int n,
     k_bin_scatter<<<gscat, 512, 2 * smc, st>>>(sp, offsets, cursor, recs, ntiles);
     CUNA_CK(cudaGetLastError());
     const size_t smg = compat_grid_smem<float>();
-    k_grid_compat<float, false><<<dim3(ntiles, 1), 256, smg, st>>>(recs, offsets, f_hat, ng, dfp, y, n, 0u);
+    k_grid_compat<float, false, kCompatThreadsFew><<<dim3(ntiles, 1), kCompatThreadsFew, smg, st>>>(recs, offsets, f_hat, ng, dfp, y, n, 0u);
     CUNA_CK(cudaGetLastError());
   }
   const int logL = ilog2i(ng);
