@@ -30,6 +30,7 @@ CORE_UNITS = [
     ("runtime.cu", []),
     ("compat.cu", ["--use_fast_math"]),
     ("accurate.cu", []),
+    ("backward.cu", []),
     ("batch.cu", []),
     ("lombscargle.cu", []),
 ]

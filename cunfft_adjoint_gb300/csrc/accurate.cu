@@ -31,6 +31,7 @@
 #include <mutex>
 #include <vector>
 #include "accurate_kernels.cuh"
+#include "backward.h"
 #include "fftpass.cuh"
 
 struct cuna2_plan_st {
@@ -1053,15 +1054,6 @@ int backward_run(cuna2_plan_st *p, const double *t, const T *y, const typename C
       return fail(CUNA2_ERROR_INVALID_VALUE, "series %d: T = %g, t0 = %g", s, Ts[s], t0s[s]);
   if (n > ((int64_t)1 << 30)) return fail(CUNA2_ERROR_UNSUPPORTED, "n > 2^30 samples per series");
   if (n == 0 || (!gy && !gt)) return CUNA2_SUCCESS;
-  const AccParams<T> e = make_params<T>(p);
-  const FftDev<T> f = to_dev<T>(p->geom);
-  BwdSpec<T> sp;
-  sp.G = G;
-  sp.ng = p->ng;
-  sp.K = p->nf / 2;
-  sp.c0b = (T)(1.0 / sqrt(4.0 * kPi * p->tau));
-  sp.c1 = (T)(4.0 * kPi * kPi * p->tau / ((double)p->ng * (double)p->ng));
-  sp.twk = (T)(2.0 / (double)p->ng);
   const int L = 1 << p->geom.logL;
   const int group = std::min(nser, kBwdSeries);
   BwdSeries *ser = new BwdSeries();  // 8 KB of launch parameters, filled per group
@@ -1086,45 +1078,16 @@ int backward_run(cuna2_plan_st *p, const double *t, const T *y, const typename C
     z = (C *)p->bws;
     r = z + (size_t)L * group;
   }
-  static char attr;
-  if (!setup_done(&attr)) {
-    CUNA_CK(cudaFuncSetAttribute(k_bwd_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    CUNA_CK(cudaFuncSetAttribute(k_bwd_colpass<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUNA_CK(cudaFuncSetAttribute(k_bwd_rowpass<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    mark_setup_done(&attr);
-  }
   for (int s0 = 0; s0 < nser; s0 += group) {
     const int ns = std::min(group, nser - s0);
     for (int s = 0; s < ns; ++s) {
       ser->pm[s] = phase_setup(t0s[s0 + s], Ts[s0 + s]);
       ser->tscale[s] = (double)p->ng / Ts[s0 + s];
     }
-    const double *tg = t + (int64_t)s0 * n;
-    const T *yg = y ? y + (int64_t)s0 * n : nullptr;
-    T *gyg = gy ? gy + (int64_t)s0 * n : nullptr;
-    double *gtg = gt ? gt + (int64_t)s0 * n : nullptr;
-    BwdSpec<T> spg = sp;
-    spg.G = G + (int64_t)s0 * p->nf;
-    if (p->small) {
-      const size_t smem = sizeof(C) * (size_t)fft_pitch(L, 1);
-      const int threads = std::max(32, std::min(sizeof(T) == 4 ? 1024 : 512, L / kFftE));
-      k_bwd_small<T><<<ns, threads, smem, st>>>(tg, yg, n, *ser, e, spg, f, gyg, gtg);
-      CUNA_CK(cudaGetLastError());
-      continue;
-    }
-    const int elems = sizeof(T) == 4 ? kPassElemsF32 : kPassElemsF64;
-    const int threads = elems / kFftE;
-    const int L1 = 1 << p->geom.logL1, L2 = 1 << p->geom.logL2;
-    const int BA = elems / L1, BB = elems / L2;
-    const size_t smemA = sizeof(C) * (size_t)BA * fft_pitch(L1, BA);
-    const size_t smemB = sizeof(C) * (size_t)BB * fft_pitch(L2, BB);
-    k_bwd_colpass<T><<<dim3(L2 / BA, ns), threads, smemA, st>>>(spg, z, f);
-    CUNA_CK(cudaGetLastError());
-    k_bwd_rowpass<T><<<dim3(L1 / BB, ns), threads, smemB, st>>>(z, r, f);
-    CUNA_CK(cudaGetLastError());
-    const int64_t tot = n * ns;
-    k_bwd_interp<T><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(tg, yg, n, ns, *ser, e, (const T *)r, gyg, gtg);
-    CUNA_CK(cudaGetLastError());
+    const int64_t o = (int64_t)s0 * n;
+    BwdArgs<T> a{t + o, y ? y + o : nullptr, G + (int64_t)s0 * p->nf, gy ? gy + o : nullptr, gt ? gt + o : nullptr,
+                 n, p->ng, p->nf, ns, p->m, p->tau, p->small, p->geom, z, r, ser};
+    CUNA_TRY(backward_group<T>(a, st));
   }
   return CUNA2_SUCCESS;
 }

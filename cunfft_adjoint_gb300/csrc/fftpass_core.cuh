@@ -37,13 +37,27 @@ template <class X> struct in_smem<X, std::void_t<decltype(X::kShared)>> : std::b
 template <typename T> struct PassCfg {
   static constexpr int ELEMS = sizeof(T) == 4 ? kPassElemsF32 : kPassElemsF64;
   static constexpr int THREADS = ELEMS / kFftE;
+  static constexpr int LOGE = ilog2c(ELEMS);
 };
+
+// log2 of the elements a pass's CTA holds: PassCfg<T>::LOGE where the launch
+// then fills the SMs, else PassFew: a quarter of it (half of it for 2^19 and
+// 2^20 points, whose columns would otherwise be read in pieces below 16
+// bytes), so that a single transform of middling length runs on four times
+// the CTAs.  The arithmetic per element does not depend on it.
+template <typename T, int LOGL> struct PassFew {
+  static constexpr int LOGE = PassCfg<T>::LOGE - (LOGL <= 18 ? 2 : (LOGL <= 20 ? 1 : 0));
+};
+template <typename T> inline bool pass_few(int logL, int nslab) {
+  return logL <= 20 && ((int64_t)nslab << logL) >> PassCfg<T>::LOGE < device_sm_count();
+}
 
 // One Stockham stage of radix R over the 2^LOGS sequences of length 2^LOGN a
 // CTA holds; 2^LOGNS points already transformed.  IN_G / OUT_G: the stage
 // reads from src / writes to dst instead of shared memory.  SEQ_FAST: thread
-// g takes sequence g mod 2^LOGS (else point-fastest).
-template <typename T, int R, int LOGN, int LOGNS, int LOGS, bool IN_G, bool OUT_G, bool SEQ_FAST, class Src,
+// g takes sequence g mod 2^LOGS (else point-fastest).  FTW: every twiddle is
+// read from the table (see below).
+template <typename T, int R, int LOGN, int LOGNS, int LOGS, bool IN_G, bool OUT_G, bool SEQ_FAST, bool FTW, class Src,
           class Dst>
 __device__ __forceinline__ void ct_stage(typename CxOf<T>::type *s, const typename CxOf<T>::type *__restrict__ tw,
                                          const Src &src, const Dst &dst) {
@@ -75,7 +89,7 @@ __device__ __forceinline__ void ct_stage(typename CxOf<T>::type *s, const typena
       // w_12, with w_{a + 4b} = w_a w_{4b} (one rounding more than a table
       // value); double reads all 15 (the FP64 pipe, not the loads, bounds it).
       const int step = (j & ((1 << LOGNS) - 1)) << TWSH;
-      if (sizeof(T) == 8) {
+      if (FTW) {
 #pragma unroll
         for (int r = 1; r < R; ++r) v[u][r] = cmul(v[u][r], ldtw(tw + r * step));
       } else {
@@ -117,29 +131,31 @@ __device__ __forceinline__ void ct_stage(typename CxOf<T>::type *s, const typena
 }
 
 // radix-16 stages from LOGNS on; the last one writes to dst when TO_GLOBAL
-template <typename T, int LOGN, int LOGS, int LOGNS, bool TO_GLOBAL, bool FSF, bool LSF, class Src, class Dst>
+template <typename T, int LOGN, int LOGS, int LOGNS, bool TO_GLOBAL, bool FSF, bool LSF, bool FTW, class Src,
+          class Dst>
 __device__ __forceinline__ void ct_rest(typename CxOf<T>::type *s, const typename CxOf<T>::type *__restrict__ tw,
                                         const Src &src, const Dst &dst) {
   if constexpr (LOGNS + 4 >= LOGN) {
-    ct_stage<T, 16, LOGN, LOGNS, LOGS, false, TO_GLOBAL, TO_GLOBAL ? LSF : FSF>(s, tw, src, dst);
+    ct_stage<T, 16, LOGN, LOGNS, LOGS, false, TO_GLOBAL, TO_GLOBAL ? LSF : FSF, FTW>(s, tw, src, dst);
   } else {
-    ct_stage<T, 16, LOGN, LOGNS, LOGS, false, false, FSF>(s, tw, src, dst);
-    ct_rest<T, LOGN, LOGS, LOGNS + 4, TO_GLOBAL, FSF, LSF>(s, tw, src, dst);
+    ct_stage<T, 16, LOGN, LOGNS, LOGS, false, false, FSF, FTW>(s, tw, src, dst);
+    ct_rest<T, LOGN, LOGS, LOGNS + 4, TO_GLOBAL, FSF, LSF, FTW>(s, tw, src, dst);
   }
 }
 
 // Src -> stages -> Dst (TO_GLOBAL) or -> shared memory s[seq*PITCH + pad16(k)]
 // followed by a barrier.  FSF / LSF: thread mapping of the loading stages /
 // of the storing stage.
-template <typename T, int LOGN, int LOGS, bool TO_GLOBAL, bool FSF, bool LSF, class Src, class Dst>
+template <typename T, int LOGN, int LOGS, bool TO_GLOBAL, bool FSF, bool LSF, bool FTW = (sizeof(T) == 8), class Src,
+          class Dst>
 __device__ __forceinline__ void ct_fft(typename CxOf<T>::type *s, const typename CxOf<T>::type *__restrict__ tw,
                                        const Src &src, const Dst &dst) {
   constexpr int R0L = (LOGN & 3) == 0 ? 4 : (LOGN & 3);
   if constexpr (R0L == LOGN) {
-    ct_stage<T, (1 << R0L), LOGN, 0, LOGS, true, TO_GLOBAL, TO_GLOBAL ? LSF : FSF>(s, tw, src, dst);
+    ct_stage<T, (1 << R0L), LOGN, 0, LOGS, true, TO_GLOBAL, TO_GLOBAL ? LSF : FSF, FTW>(s, tw, src, dst);
   } else {
-    ct_stage<T, (1 << R0L), LOGN, 0, LOGS, true, false, FSF>(s, tw, src, dst);
-    ct_rest<T, LOGN, LOGS, R0L, TO_GLOBAL, FSF, LSF>(s, tw, src, dst);
+    ct_stage<T, (1 << R0L), LOGN, 0, LOGS, true, false, FSF, FTW>(s, tw, src, dst);
+    ct_rest<T, LOGN, LOGS, R0L, TO_GLOBAL, FSF, LSF, FTW>(s, tw, src, dst);
   }
 }
 
@@ -181,12 +197,12 @@ template <int LOGN> __host__ __device__ constexpr int last_logns() {
 // column block `cblock` of one packed grid (L1 x L2 complex, row-major), from
 // `in` to `out` (in == out allowed: every read precedes the first barrier,
 // every write follows it)
-template <typename T, int LOGL>
+template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE>
 __device__ __forceinline__ void ct_colpass_body(const typename MemOf<T>::type *in, typename MemOf<T>::type *out,
                                                 const FftDev<T> &f, int cblock) {
   typedef typename CxOf<T>::type C;
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
-  constexpr int LOGB = ilog2c(PassCfg<T>::ELEMS) - LOG1;
+  constexpr int LOGB = LOGE - LOG1;
   constexpr int B = 1 << LOGB;
   constexpr int PITCH = fft_pitch(1 << LOG1, B);
   constexpr int LNS = last_logns<LOG1>();
@@ -196,7 +212,7 @@ __device__ __forceinline__ void ct_colpass_body(const typename MemOf<T>::type *i
   const int c0 = cblock * B;
   pdl_trigger();
   // stride 17 so that the columns of one row of the table fall in different banks
-  for (int i = threadIdx.x; i < 16 * B; i += PassCfg<T>::THREADS)
+  for (int i = threadIdx.x; i < 16 * B; i += 1 << (LOGE - 4))
     steps[(i >> 4) * 17 + (i & 15)] = twiddle_L(f, (c0 + (i >> 4)) * ((i & 15) << LNS));
   // the steps table is read only by the storing stage, after at least one barrier
   pdl_wait();  // the grid comes from the gridding
@@ -206,16 +222,16 @@ __device__ __forceinline__ void ct_colpass_body(const typename MemOf<T>::type *i
   ct_fft<T, LOG1, LOGB, true, true, true>(s, f.tw1, src, dst);
 }
 
-template <typename T, int LOGL>
-__global__ void __launch_bounds__(PassCfg<T>::THREADS) k_ct_colpass(typename MemOf<T>::type *grid, FftDev<T> f,
-                                                                    int64_t slab_stride) {
+template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE>
+__global__ void __launch_bounds__(1 << (LOGE - 4)) k_ct_colpass(typename MemOf<T>::type *grid, FftDev<T> f,
+                                                                int64_t slab_stride) {
   typename MemOf<T>::type *z = grid + blockIdx.y * slab_stride;
-  ct_colpass_body<T, LOGL>(z, z, f, blockIdx.x);
+  ct_colpass_body<T, LOGL, LOGE>(z, z, f, blockIdx.x);
 }
 
-template <typename T, int LOGL> constexpr size_t ct_colpass_smem() {
+template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE> constexpr size_t ct_colpass_smem() {
   constexpr int LOG1 = (LOGL + 1) / 2;
-  constexpr int B = PassCfg<T>::ELEMS >> LOG1;
+  constexpr int B = 1 << (LOGE - LOG1);
   return sizeof(typename CxOf<T>::type) * ((size_t)fft_pitch(1 << LOG1, B) * B + 17 * B);
 }
 
