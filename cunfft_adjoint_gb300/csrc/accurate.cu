@@ -146,21 +146,21 @@ inline void mark(Prof *pr, const char *name, cudaStream_t st) {
 // Both four-step passes with the compile-time kernels of fftpass.cuh for the
 // lengths that have an instance: returns 1 when launched, 0 when logL has no
 // instance, -1 on a launch error.
-template <typename T, int LOGL>
-int ct_passes_at(typename MemOf<T>::type *z, const FftDev<T> &f, const AccParams<typename AccOf<T>::type> &e,
-                 typename MemOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
+template <typename T, int LOGL, int LOGE>
+int ct_passes_sized(typename MemOf<T>::type *z, const FftDev<T> &f, const AccParams<typename AccOf<T>::type> &e,
+                    typename MemOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
-  constexpr int BA = PassCfg<T>::ELEMS >> LOG1;
-  constexpr size_t smA = ct_colpass_smem<T, LOGL>(), smB = ct_rowpass_smem<T, LOGL>();
+  constexpr int BA = 1 << (LOGE - LOG1), TH = 1 << (LOGE - 4);
+  constexpr size_t smA = ct_colpass_smem<T, LOGL, LOGE>(), smB = ct_rowpass_smem<T, LOGL, LOGE>();
   static char attr;
   if (!setup_done(&attr)) {
-    if (cudaFuncSetAttribute(k_ct_colpass<T, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
-        cudaFuncSetAttribute(k_ct_rowpass_acc<T, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB))
+    if (cudaFuncSetAttribute(k_ct_colpass<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
+        cudaFuncSetAttribute(k_ct_rowpass_acc<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB))
       return -1;
     mark_setup_done(&attr);
   }
   bool tma = false;
-  if constexpr (sizeof(T) == 4 && TmaCol<LOGL>::ok) {
+  if constexpr (sizeof(T) == 4 && TmaCol<LOGL>::ok && LOGE == PassCfg<T>::LOGE) {
     // column pass through TMA boxes when the CUDA driver encodes the tensor map
     int *tmo = tma_enabled() ? wait_timeout_counter() : nullptr;
     alignas(64) CUtensorMap map;
@@ -172,21 +172,30 @@ int ct_passes_at(typename MemOf<T>::type *z, const FftDev<T> &f, const AccParams
           return -1;
         mark_setup_done(&attr_tma);
       }
-      k_ct_colpass_tma<LOGL><<<dim3((1 << LOG2) / BA, nslab), PassCfg<T>::THREADS, ct_colpass_tma_smem<LOGL>(), st>>>(
+      k_ct_colpass_tma<LOGL><<<dim3((1 << LOG2) / BA, nslab), TH, ct_colpass_tma_smem<LOGL>(), st>>>(
           map, f, tmo);
       tma = true;
     }
   }
-  if (!tma && launch_pdl(k_ct_colpass<T, LOGL>, dim3((1 << LOG2) / BA, nslab), dim3(PassCfg<T>::THREADS), smA, st, z,
-                         f, (int64_t)1 << LOGL) != cudaSuccess)
+  if (!tma && launch_pdl(k_ct_colpass<T, LOGL, LOGE>, dim3((1 << LOG2) / BA, nslab), dim3(TH), smA, st, z, f,
+                         (int64_t)1 << LOGL) != cudaSuccess)
     return -1;
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
   mark(pr, "fft_colpass", st);
-  if (launch_pdl(k_ct_rowpass_acc<T, LOGL>, dim3(ct_rowpass_ctas<T, LOGL>(), nslab), dim3(PassCfg<T>::THREADS), smB,
-                 st, z, f, e, F) != cudaSuccess)
+  if (launch_pdl(k_ct_rowpass_acc<T, LOGL, LOGE>, dim3(ct_rowpass_ctas<T, LOGL, LOGE>(), nslab), dim3(TH), smB, st,
+                 (const typename MemOf<T>::type *)z, f, e, F) != cudaSuccess)
     return -1;
   mark(pr, "fft_rowpass", st);
   return 1;
+}
+
+template <typename T, int LOGL>
+int ct_passes_at(typename MemOf<T>::type *z, const FftDev<T> &f, const AccParams<typename AccOf<T>::type> &e,
+                 typename MemOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
+  if constexpr (sizeof(T) == 4)
+    if (pass_few<T>(LOGL, nslab, 4) && !tma_enabled())
+      return ct_passes_sized<T, LOGL, PassFew<T, LOGL>::LOGE>(z, f, e, F, nslab, st, pr);
+  return ct_passes_sized<T, LOGL, PassCfg<T>::LOGE>(z, f, e, F, nslab, st, pr);
 }
 
 template <typename T>

@@ -398,7 +398,7 @@ int bwd_passes_sized(const BwdSpec<T> &sp, typename CxOf<T>::type *z, typename C
 template <typename T, int LOGL>
 int bwd_passes_at(const BwdSpec<T> &sp, typename CxOf<T>::type *z, typename CxOf<T>::type *r, const FftDev<T> &f,
                   int ns, cudaStream_t st) {
-  if (pass_few<T>(LOGL, ns)) return bwd_passes_sized<T, LOGL, PassFew<T, LOGL>::LOGE>(sp, z, r, f, ns, st);
+  if (pass_few<T>(LOGL, ns, sizeof(T) == 4 ? 4 : 1)) return bwd_passes_sized<T, LOGL, PassFew<T, LOGL>::LOGE>(sp, z, r, f, ns, st);
   return bwd_passes_sized<T, LOGL, PassCfg<T>::LOGE>(sp, z, r, f, ns, st);
 }
 

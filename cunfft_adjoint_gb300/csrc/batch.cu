@@ -163,42 +163,48 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256) k_browpass(const T
 
 // Four-step passes with compile-time geometry for one size class of large
 // series: blockIdx.y indexes the class's series list.
-template <typename T, int LOGL>
-__global__ void __launch_bounds__(PassCfg<T>::THREADS) k_bct_colpass(T *grid, const BDesc<T> *__restrict__ D,
-                                                                     const int *__restrict__ list) {
+template <typename T, int LOGL, int LOGE>
+__global__ void __launch_bounds__(1 << (LOGE - 4)) k_bct_colpass(T *grid, const BDesc<T> *__restrict__ D,
+                                                                 const int *__restrict__ list) {
   typedef typename CxOf<T>::type C;
   const int s = list[blockIdx.y];
   C *z = reinterpret_cast<C *>(grid + D[s].g_off);
-  ct_colpass_body<T, LOGL>(z, z, D[s].f, blockIdx.x);
+  ct_colpass_body<T, LOGL, LOGE>(z, z, D[s].f, blockIdx.x);
 }
 
-template <typename T, int LOGL>
-__global__ void __launch_bounds__(PassCfg<T>::THREADS) k_bct_rowpass(const T *grid, const BDesc<T> *__restrict__ D,
-                                                                     const int *__restrict__ list,
-                                                                     typename CxOf<T>::type *F) {
+template <typename T, int LOGL, int LOGE>
+__global__ void __launch_bounds__(1 << (LOGE - 4)) k_bct_rowpass(const T *grid, const BDesc<T> *__restrict__ D,
+                                                                 const int *__restrict__ list,
+                                                                 typename CxOf<T>::type *F) {
   typedef typename CxOf<T>::type C;
   const int s = list[blockIdx.y];
-  ct_rowpass_body<T, LOGL>(reinterpret_cast<const C *>(grid + D[s].g_off), D[s].f, D[s].e, F + D[s].f_off,
-                           blockIdx.x);
+  ct_rowpass_body<T, LOGL, LOGE>(reinterpret_cast<const C *>(grid + D[s].g_off), D[s].f, D[s].e, F + D[s].f_off,
+                                 blockIdx.x);
 }
 
-template <typename T, int LOGL>
-int bct_at(T *grid, const BDesc<T> *D, const int *list, int cnt, typename CxOf<T>::type *F, cudaStream_t st) {
+template <typename T, int LOGL, int LOGE>
+int bct_sized(T *grid, const BDesc<T> *D, const int *list, int cnt, typename CxOf<T>::type *F, cudaStream_t st) {
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
-  constexpr int BA = PassCfg<T>::ELEMS >> LOG1;
-  constexpr size_t smA = ct_colpass_smem<T, LOGL>(), smB = ct_rowpass_smem<T, LOGL>();
+  constexpr int BA = 1 << (LOGE - LOG1), TH = 1 << (LOGE - 4);
+  constexpr size_t smA = ct_colpass_smem<T, LOGL, LOGE>(), smB = ct_rowpass_smem<T, LOGL, LOGE>();
   static char attr;
   if (!setup_done(&attr)) {
-    if (cudaFuncSetAttribute(k_bct_colpass<T, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
-        cudaFuncSetAttribute(k_bct_rowpass<T, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB))
+    if (cudaFuncSetAttribute(k_bct_colpass<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
+        cudaFuncSetAttribute(k_bct_rowpass<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB))
       return -1;
     mark_setup_done(&attr);
   }
-  k_bct_colpass<T, LOGL><<<dim3((1 << LOG2) / BA, cnt), PassCfg<T>::THREADS, smA, st>>>(grid, D, list);
+  k_bct_colpass<T, LOGL, LOGE><<<dim3((1 << LOG2) / BA, cnt), TH, smA, st>>>(grid, D, list);
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
-  k_bct_rowpass<T, LOGL><<<dim3(ct_rowpass_ctas<T, LOGL>(), cnt), PassCfg<T>::THREADS, smB, st>>>(grid, D, list, F);
+  k_bct_rowpass<T, LOGL, LOGE><<<dim3(ct_rowpass_ctas<T, LOGL, LOGE>(), cnt), TH, smB, st>>>(grid, D, list, F);
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
   return 1;
+}
+template <typename T, int LOGL>
+int bct_at(T *grid, const BDesc<T> *D, const int *list, int cnt, typename CxOf<T>::type *F, cudaStream_t st) {
+  if constexpr (sizeof(T) == 4)
+    if (pass_few<T>(LOGL, cnt, 4)) return bct_sized<T, LOGL, PassFew<T, LOGL>::LOGE>(grid, D, list, cnt, F, st);
+  return bct_sized<T, LOGL, PassCfg<T>::LOGE>(grid, D, list, cnt, F, st);
 }
 
 // 1: launched, 0: no compiled instance for logL, -1: launch error

@@ -443,11 +443,11 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256) k_fft_rowpass_comp
 // Compile-time four-step passes of the compat transform: column pass from
 // f_hat into scratch (twiddled), row pass from scratch back into f_hat in
 // natural order with the reference normalisation fused in.
-template <typename T, int LOGL>
-__global__ void __launch_bounds__(PassCfg<T>::THREADS) k_ct_colpass_oop(const typename CxOf<T>::type *in,
-                                                                        typename CxOf<T>::type *out, FftDev<T> f,
-                                                                        int64_t slab_stride) {
-  ct_colpass_body<T, LOGL>(in + blockIdx.y * slab_stride, out + blockIdx.y * slab_stride, f, blockIdx.x);
+template <typename T, int LOGL, int LOGE>
+__global__ void __launch_bounds__(1 << (LOGE - 4)) k_ct_colpass_oop(const typename CxOf<T>::type *in,
+                                                                    typename CxOf<T>::type *out, FftDev<T> f,
+                                                                    int64_t slab_stride) {
+  ct_colpass_body<T, LOGL, LOGE>(in + blockIdx.y * slab_stride, out + blockIdx.y * slab_stride, f, blockIdx.x);
 }
 
 template <typename T, int LOG2> struct CtRowSrc {
@@ -473,14 +473,14 @@ template <typename T, int LOG1> struct CtFacDst {
   }
 };
 
-template <typename T, int LOGL>
-__global__ void __launch_bounds__(PassCfg<T>::THREADS) k_ct_rowpass_compat(const typename CxOf<T>::type *in,
-                                                                           typename CxOf<T>::type *out, FftDev<T> f,
-                                                                           const typename FpOf<T>::type *fp,
-                                                                           int64_t slab_stride, int norm) {
+template <typename T, int LOGL, int LOGE>
+__global__ void __launch_bounds__(1 << (LOGE - 4)) k_ct_rowpass_compat(const typename CxOf<T>::type *in,
+                                                                       typename CxOf<T>::type *out, FftDev<T> f,
+                                                                       const typename FpOf<T>::type *fp,
+                                                                       int64_t slab_stride, int norm) {
   typedef typename CxOf<T>::type C;
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
-  constexpr int LOGB = ilog2c(PassCfg<T>::ELEMS) - LOG2;
+  constexpr int LOGB = LOGE - LOG2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *s = reinterpret_cast<C *>(smem_raw);
   const int r0 = blockIdx.x << LOGB;
@@ -493,27 +493,36 @@ __global__ void __launch_bounds__(PassCfg<T>::THREADS) k_ct_rowpass_compat(const
   ct_fft<T, LOG2, LOGB, true, false, true>(s, f.tw2, src, dst);
 }
 
-template <typename T, int LOGL>
-int compat_ct_at(typename CxOf<T>::type *f_hat, typename CxOf<T>::type *scratch, const FftDev<T> &f,
-                 const typename FpOf<T>::type *dfp, int nbs, bool norm, cudaStream_t st) {
+template <typename T, int LOGL, int LOGE>
+int compat_ct_sized(typename CxOf<T>::type *f_hat, typename CxOf<T>::type *scratch, const FftDev<T> &f,
+                    const typename FpOf<T>::type *dfp, int nbs, bool norm, cudaStream_t st) {
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
-  constexpr int BA = PassCfg<T>::ELEMS >> LOG1, BB = PassCfg<T>::ELEMS >> LOG2;
-  constexpr size_t smA = ct_colpass_smem<T, LOGL>();
+  constexpr int BA = 1 << (LOGE - LOG1), BB = 1 << (LOGE - LOG2), TH = 1 << (LOGE - 4);
+  constexpr size_t smA = ct_colpass_smem<T, LOGL, LOGE>();
   constexpr size_t smB = sizeof(typename CxOf<T>::type) * (size_t)fft_pitch(1 << LOG2, BB) * BB;
   static char attr;
   if (!setup_done(&attr)) {
-    if (cudaFuncSetAttribute(k_ct_colpass_oop<T, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
-        cudaFuncSetAttribute(k_ct_rowpass_compat<T, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB))
+    if (cudaFuncSetAttribute(k_ct_colpass_oop<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
+        cudaFuncSetAttribute(k_ct_rowpass_compat<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smB))
       return -1;
     mark_setup_done(&attr);
   }
   const int64_t L = (int64_t)1 << LOGL;
-  k_ct_colpass_oop<T, LOGL><<<dim3((1 << LOG2) / BA, nbs), PassCfg<T>::THREADS, smA, st>>>(f_hat, scratch, f, L);
+  k_ct_colpass_oop<T, LOGL, LOGE><<<dim3((1 << LOG2) / BA, nbs), TH, smA, st>>>(f_hat, scratch, f, L);
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
-  k_ct_rowpass_compat<T, LOGL><<<dim3((1 << LOG1) / BB, nbs), PassCfg<T>::THREADS, smB, st>>>(scratch, f_hat, f, dfp,
-                                                                                            L, norm ? 1 : 0);
+  k_ct_rowpass_compat<T, LOGL, LOGE><<<dim3((1 << LOG1) / BB, nbs), TH, smB, st>>>(scratch, f_hat, f, dfp, L,
+                                                                                   norm ? 1 : 0);
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
   return 1;
+}
+template <typename T, int LOGL>
+int compat_ct_at(typename CxOf<T>::type *f_hat, typename CxOf<T>::type *scratch, const FftDev<T> &f,
+                 const typename FpOf<T>::type *dfp, int nbs, bool norm, cudaStream_t st) {
+  if constexpr (sizeof(T) == 4)
+    if (pass_few<T>(LOGL, nbs, 4))
+      return compat_ct_sized<T, LOGL, PassFew<T, LOGL>::LOGE>(f_hat, scratch, f, dfp, nbs, norm, st);
+  return compat_ct_sized<T, LOGL, PassCfg<T>::LOGE>(f_hat, scratch, f, dfp, nbs, norm, st);
 }
 
 // 1: launched, 0: no compiled instance, -1: launch error

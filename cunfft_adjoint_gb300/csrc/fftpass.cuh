@@ -39,7 +39,7 @@ struct CtNoDst {
 };
 
 // row-pair block `pblock` of one packed grid z; outputs Fs[0 .. nf)
-template <typename T, int LOGL>
+template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE>
 __device__ __forceinline__ void ct_rowpass_body(const typename MemOf<T>::type *slab, const FftDev<T> &f,
                                                 const AccParams<typename AccOf<T>::type> &e,
                                                 typename MemOf<T>::type *Fs, int pblock) {
@@ -47,10 +47,10 @@ __device__ __forceinline__ void ct_rowpass_body(const typename MemOf<T>::type *s
   typedef typename AccOf<T>::type A;
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
   constexpr int L2 = 1 << LOG2;
-  constexpr int LOGB = ilog2c(PassCfg<T>::ELEMS) - LOG2;
+  constexpr int LOGB = LOGE - LOG2;
   constexpr int B = 1 << LOGB, LOGP = LOGB - 1, P = B >> 1;
   constexpr int PITCH = fft_pitch(L2, B);
-  constexpr int THREADS = PassCfg<T>::THREADS;
+  constexpr int THREADS = 1 << (LOGE - 4);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *s = reinterpret_cast<C *>(smem_raw);
   // unpack twiddles W_ng^k = W_ng^{k1} W_ng^{k2 L1} from two small tables
@@ -86,21 +86,25 @@ __device__ __forceinline__ void ct_rowpass_body(const typename MemOf<T>::type *s
 
 // three CTAs per SM for the short rows of many small grids (bootstrap), where
 // the pass streams from HBM and more bytes in flight pay
-template <typename T, int LOGL>
-__global__ void __launch_bounds__(PassCfg<T>::THREADS, (sizeof(T) == 4 && LOGL <= 15) ? 3 : 2) k_ct_rowpass_acc(const typename MemOf<T>::type *grid,
-                                                                        FftDev<T> f, AccParams<typename AccOf<T>::type> e,
-                                                                        typename MemOf<T>::type *F) {
-  ct_rowpass_body<T, LOGL>(grid + ((int64_t)blockIdx.y << LOGL), f, e, F + (int64_t)blockIdx.y * e.nf, blockIdx.x);
+template <typename T, int LOGL, int LOGE> constexpr int ct_rowpass_min_ctas() {
+  return LOGE < PassCfg<T>::LOGE ? 1 : ((sizeof(T) == 4 && LOGL <= 15) ? 3 : 2);
+}
+template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE>
+__global__ void __launch_bounds__(1 << (LOGE - 4), ct_rowpass_min_ctas<T, LOGL, LOGE>()) k_ct_rowpass_acc(
+    const typename MemOf<T>::type *grid, FftDev<T> f, AccParams<typename AccOf<T>::type> e,
+    typename MemOf<T>::type *F) {
+  ct_rowpass_body<T, LOGL, LOGE>(grid + ((int64_t)blockIdx.y << LOGL), f, e, F + (int64_t)blockIdx.y * e.nf,
+                                 blockIdx.x);
 }
 
 // CTAs per packed grid of the row pass: L1/2 slots, B/2 per CTA
-template <typename T, int LOGL> constexpr int ct_rowpass_ctas() {
-  return ((1 << ((LOGL + 1) / 2)) / 2) / ((PassCfg<T>::ELEMS >> (LOGL / 2)) / 2);
+template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE> constexpr int ct_rowpass_ctas() {
+  return ((1 << ((LOGL + 1) / 2)) / 2) / ((1 << (LOGE - LOGL / 2)) / 2);
 }
 
-template <typename T, int LOGL> constexpr size_t ct_rowpass_smem() {
+template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE> constexpr size_t ct_rowpass_smem() {
   constexpr int LOG2 = LOGL / 2;
-  constexpr int B = PassCfg<T>::ELEMS >> LOG2;
+  constexpr int B = 1 << (LOGE - LOG2);
   return sizeof(typename CxOf<T>::type) * ((size_t)fft_pitch(1 << LOG2, B) * B + B + (1 << LOG2));
 }
 

@@ -40,16 +40,20 @@ template <typename T> struct PassCfg {
   static constexpr int LOGE = ilog2c(ELEMS);
 };
 
-// log2 of the elements a pass's CTA holds: PassCfg<T>::LOGE where the launch
-// then fills the SMs, else PassFew: a quarter of it (half of it for 2^19 and
-// 2^20 points, whose columns would otherwise be read in pieces below 16
-// bytes), so that a single transform of middling length runs on four times
-// the CTAs.  The arithmetic per element does not depend on it.
+// log2 of the elements a pass's CTA holds: PassCfg<T>::LOGE, or PassFew (a
+// quarter of it; half of it for 2^19 and 2^20 points, whose columns would
+// otherwise be read in pieces below 16 bytes) where a launch leaves most SMs
+// idle.  The arithmetic per element does not depend on it.  Float passes take
+// it below a quarter of the SMs (one transform of 2^14 points: 6.4 + 7.0 us on
+// 2 CTAs each, 4.9 + 4.4 on 8; from 64 CTAs on it gains nothing); the double
+// backward below one CTA per SM (its FP64 pipes are then the bound).  The
+// forward's FP64 passes lose with it (their code is fetched by more CTAs of
+// fewer warps).
 template <typename T, int LOGL> struct PassFew {
   static constexpr int LOGE = PassCfg<T>::LOGE - (LOGL <= 18 ? 2 : (LOGL <= 20 ? 1 : 0));
 };
-template <typename T> inline bool pass_few(int logL, int nslab) {
-  return logL <= 20 && ((int64_t)nslab << logL) >> PassCfg<T>::LOGE < device_sm_count();
+template <typename T> inline bool pass_few(int logL, int nslab, int part) {
+  return logL <= 20 && part * (((int64_t)nslab << logL) >> PassCfg<T>::LOGE) <= device_sm_count();
 }
 
 // One Stockham stage of radix R over the 2^LOGS sequences of length 2^LOGN a
