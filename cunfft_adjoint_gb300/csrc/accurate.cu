@@ -332,9 +332,9 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
       CUNA_CK(cudaFuncSetAttribute(k_nfft_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
       mark_setup_done(&attr);
     }
-    const size_t smem = sizeof(C) * (size_t)fft_pitch(L, 1) + sizeof(T) * (2 * p->m + 2);
-    const int threads = std::max(32, std::min(1024, L / kFftE));
-    k_nfft_small<T><<<nslab, threads, smem, st>>>(t, y, n, pm, e, f, F, wts);
+    const bool alone = nslab <= nsm, gather = small_gather(L, alone, sizeof(T) == 4);
+    k_nfft_small<T><<<nslab, small_threads<T>(L, alone, gather), small_smem<T>(L, p->m, gather), st>>>(
+        t, y, n, pm, e, f, F, wts, gather);
     CUNA_CK(cudaGetLastError());
     mark(pr, "nfft_small", st);
     return CUNA2_SUCCESS;

@@ -128,71 +128,7 @@ __device__ __forceinline__ void acc_output_tw(const AccParams<typename AccOf<T>:
   if (k >= 1) F[e.K - k] = cconj(Fk);
 }
 
-// ---------------------------------------------------------------------------
-// single-CTA transform for small grids
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ int real_slot(int c) { return 2 * pad16(c >> 1) + (c & 1); }
-
-// Whole transform of one series in one CTA: gridding straight into shared
-// memory (the grid is the packed complex FFT buffer), FFT, epilogue.
-template <typename T>
-__device__ __forceinline__ void nfft_small_body(const double *__restrict__ t, const T *__restrict__ y,
-                                                int64_t n, const PhaseMul &pm, const AccParams<T> &e,
-                                                const FftDev<T> &f, typename CxOf<T>::type *F) {
-  typedef typename CxOf<T>::type C;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int L = 1 << f.logL;
-  const int pitch = fft_pitch(L, 1);
-  C *s = reinterpret_cast<C *>(smem_raw);
-  T *sr = reinterpret_cast<T *>(smem_raw);
-  T *e3 = reinterpret_cast<T *>(s + pitch);
-  const int m = e.m, ng = (int)e.ng;
-  for (int i = threadIdx.x; i < 2 * pitch; i += blockDim.x) sr[i] = (T)0;
-  for (int d = threadIdx.x; d <= 2 * m; d += blockDim.x) e3[d] = exp_t(e.e3c * (T)((d - m) * (d - m)));
-  __syncthreads();
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    int cell;
-    T fr;
-    reduce_sample<T>(t[i], pm, e.ng, cell, fr);
-    const T E1 = exp2_t(-e.k1 * fr * fr), E2 = exp2_t(e.k2 * fr);
-    const T w0 = y[i] * E1;
-    T w = w0;
-    for (int d = 0; d <= m; ++d) {
-      int c = cell + d;
-      if (c >= ng) c -= ng;
-      atomicAdd(&sr[real_slot(c)], w * e3[d + m]);
-      w *= E2;
-    }
-    const T E2i = (T)1 / E2;
-    w = w0 * E2i;
-    for (int d = -1; d > -m; --d) {
-      int c = cell + d;
-      if (c < 0) c += ng;
-      atomicAdd(&sr[real_slot(c)], w * e3[d + m]);
-      w *= E2i;
-    }
-  }
-  __syncthreads();
-  smem_fft<T>(s, pitch, f.logL, 1, f.tw1);
-  for (int64_t k = threadIdx.x; k <= e.K; k += blockDim.x) {
-    const C Zk = s[pad16((int)(k & (L - 1)))];
-    const C Zm = cconj(s[pad16((int)((L - k) & (L - 1)))]);
-    acc_output<T>(e, k, Zk, Zm, F);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_nfft_small(const double *__restrict__ t, const T *__restrict__ y,
-                                                     int64_t n, PhaseMul pm, AccParams<T> e, FftDev<T> f,
-                                                     typename CxOf<T>::type *F, const T *__restrict__ wts) {
-  // one CTA per output slab: slab b grids wts[b*n + j] when wts is given
-  // (bootstrap resample b), else y[j]
-  if (wts) {
-    y = wts + (int64_t)blockIdx.x * n;
-    F += (int64_t)blockIdx.x * e.nf;
-  }
-  nfft_small_body<T>(t, y, n, pm, e, f, F);
-}
 
 // ---------------------------------------------------------------------------
 // binning sampler, tiled gridding, last FFT pass
@@ -381,6 +317,214 @@ __device__ __forceinline__ void gauss_acc(T y, T x, T k1, const GaussCW<T, CW> &
     if (MASKED) a[H - j] = fma((unsigned)(rel - H + j) < (unsigned)w2 ? u : (T)0, g.c[j], a[H - j]);
     else a[H - j] = fma(u, g.c[j], a[H - j]);
   }
+}
+
+// ---------------------------------------------------------------------------
+// single-CTA transform for small grids
+// ---------------------------------------------------------------------------
+// Whole transform of one series in one CTA: gridding straight into shared
+// memory (the grid is the packed complex FFT buffer), FFT, epilogue.
+//
+// Two griddings.  Scatter: a thread per sample adds its 2m taps with shared
+// atomics (float: compare-and-swap loops, 3 adds per clock and SM).  Gather
+// (float): the samples go in chunks of up to small_cap(ng) records; a chunk is
+// counting-sorted in shared memory by group of four cells (one atomic per
+// record ranks it, the gather reads it through an index), then every thread
+// sums its groups of four cells over the records in reach, as the tiled gather
+// does, with no floating-point atomics.  The gather visits every group once
+// per chunk, so it pays on small grids: in a batch (four samples per grid of
+// 16 to 32 cells) 21 -> 11 us for 2^10-cell grids and 20 -> 18 us at 2^12
+// cells, but 29 -> 34 us at 2^13 and 114 -> 171 us at 2^15; a transform with an
+// SM to itself takes it to 2^14 cells.  One transform of n = 1000, Nf = 2048,
+// R = 2, m = 8: 28.7 us per call with L / 16 threads and the scatter, 14.1 us
+// here.
+inline bool small_gather(int L, bool alone, bool is_float) { return is_float && L <= (alone ? 8192 : 2048); }
+constexpr int kSmallCapMax = 2048;
+__host__ __device__ __forceinline__ int small_cap(int64_t ng) {
+  const int64_t c = ng / 4;
+  return (int)(c < 32 ? 32 : (c > kSmallCapMax ? kSmallCapMax : c));
+}
+// shared bytes: FFT buffer | gather: records, index, group starts; scatter: E3
+template <typename T> size_t small_smem(int L, int m, bool gather) {
+  const size_t fft = sizeof(typename CxOf<T>::type) * (size_t)fft_pitch(L, 1);
+  if (!gather) return fft + sizeof(T) * (2 * m + 2);
+  const int cap = small_cap(2 * (int64_t)L);
+  return ((fft + 15) & ~(size_t)15) + (size_t)cap * (sizeof(SRec<float>) + sizeof(int)) +
+         sizeof(int) * ((size_t)(2 * L) / 4 + 1);
+}
+// threads of a small transform: the FFT keeps L / 16 busy, the samples, groups
+// and outputs more; `alone`: the launch has an SM per transform
+template <typename T> int small_threads(int L, bool alone, bool gather) {
+  const int most = sizeof(T) == 4 ? 1024 : 512;
+  const int want = gather ? (alone ? L / 2 : L / 8) : (alone ? most : L / kFftE);
+  return std::max(std::max(32, std::min(most, L / kFftE)), std::min(most, want));
+}
+
+// exclusive scan in place of v[0..n), v[n] = total, by the whole CTA; ends
+// with a barrier
+__device__ __forceinline__ void cta_scan_in_place(int *v, int n) {
+  __shared__ int wsum[32];
+  const int nt = blockDim.x, tid = threadIdx.x;
+  const int per = (n + nt - 1) / nt;
+  const int beg = min(tid * per, n), end = min(beg + per, n);
+  int sum = 0;
+  for (int i = beg; i < end; ++i) sum += v[i];
+  const int lane = tid & 31, w = tid >> 5;
+  int x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += u;
+  }
+  if (lane == 31) wsum[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    int q = lane < (nt >> 5) ? wsum[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, q, o);
+      if (lane >= o) q += u;
+    }
+    wsum[lane] = q;
+  }
+  __syncthreads();
+  int run = x - sum + (w > 0 ? wsum[w - 1] : 0);
+  for (int i = beg; i < end; ++i) {
+    const int u = v[i];
+    v[i] = run;
+    run += u;
+  }
+  if (tid == nt - 1) v[n] = wsum[(nt >> 5) - 1];
+  __syncthreads();
+}
+
+// the four cells of group g from the sorted records of one chunk, added to
+// a[]: records of the groups that hold cells 4g - m .. 4g + m + 2, whose
+// indices wrap around the periodic grid (images o = -1, 0, 1)
+template <bool MASKED>
+__device__ __forceinline__ void small_gather4(const SRec<float> *srec, const int *order, const int *start, int g, int NG,
+                                              int ng, int m, float k1, const GaussCW<float, 4> &gw, float *a) {
+  const int c0 = 4 * g;
+  const int glo = (c0 - m) >> 2, ghi = (c0 + m + 2) >> 2;
+#pragma unroll 1
+  for (int o = -1; o <= 1; ++o) {
+    const int lo = max(glo, o * NG) - o * NG, hi = min(ghi, o * NG + NG - 1) - o * NG;
+    if (lo > hi) continue;
+    const int c = c0 - o * ng;  // the group's first cell as this image sees it
+    const int re = start[hi + 1];
+    for (int r = start[lo]; r < re; ++r) {
+      const SRec<float> q = srec[order[r]];
+      const int dc = c - q.lc;
+      gauss_acc<float, 4, MASKED>(q.y, (float)dc - q.f, k1, gw, m - dc, 2 * m, a);
+    }
+  }
+}
+
+__device__ __forceinline__ void small_grid_gather(const double *__restrict__ t, const float *__restrict__ y, int64_t n,
+                                                  const PhaseMul &pm, const AccParams<float> &e, float *sr,
+                                                  SRec<float> *srec, int *order, int *start) {
+  const int ng = (int)e.ng, NG = ng / 4, m = e.m, cap = small_cap(ng);
+  const GaussCW<float, 4> gw(e.k1);
+  // as tail_free_gather: exp(-m^2 / (4 tau)) < 1e-8
+  const bool masked = e.k1 * (float)(m * m) < 26.6f;
+  int64_t c0 = 0;
+  do {
+    const int cnt = (int)min((int64_t)cap, n - c0);
+    if (c0 > 0) __syncthreads();  // the previous chunk's gather is done with the starts and records
+    for (int i = threadIdx.x; i < NG; i += blockDim.x) start[i] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+      SRec<float> r;
+      reduce_sample<float>(t[c0 + i], pm, e.ng, r.lc, r.f);
+      r.y = y[c0 + i];
+      r.pad = atomicAdd(&start[r.lc >> 2], 1);  // rank within its group
+      srec[i] = r;
+    }
+    __syncthreads();
+    cta_scan_in_place(start, NG);
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) order[start[srec[i].lc >> 2] + srec[i].pad] = i;
+    __syncthreads();
+    for (int g = threadIdx.x; g < NG; g += blockDim.x) {
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+      if (masked) small_gather4<true>(srec, order, start, g, NG, ng, m, e.k1, gw, a);
+      else small_gather4<false>(srec, order, start, g, NG, ng, m, e.k1, gw, a);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float &d = sr[real_slot(4 * g + i)];
+        d = c0 == 0 ? a[i] : d + a[i];
+      }
+    }
+    c0 += cap;
+  } while (c0 < n);
+}
+
+template <typename T>
+__device__ __forceinline__ void nfft_small_body(const double *__restrict__ t, const T *__restrict__ y,
+                                                int64_t n, const PhaseMul &pm, const AccParams<T> &e,
+                                                const FftDev<T> &f, typename CxOf<T>::type *F, bool gather) {
+  typedef typename CxOf<T>::type C;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int L = 1 << f.logL;
+  const int pitch = fft_pitch(L, 1);
+  C *s = reinterpret_cast<C *>(smem_raw);
+  T *sr = reinterpret_cast<T *>(smem_raw);
+  if (sizeof(T) == 4 && gather) {
+    if constexpr (sizeof(T) == 4) {
+      const int cap = small_cap(e.ng);
+      SRec<float> *srec = reinterpret_cast<SRec<float> *>(smem_raw + ((sizeof(C) * pitch + 15) & ~(size_t)15));
+      int *order = reinterpret_cast<int *>(srec + cap);
+      small_grid_gather(t, y, n, pm, e, sr, srec, order, order + cap);
+    }
+  } else {
+    T *e3 = reinterpret_cast<T *>(s + pitch);
+    const int m = e.m, ng = (int)e.ng;
+    for (int i = threadIdx.x; i < 2 * pitch; i += blockDim.x) sr[i] = (T)0;
+    for (int d = threadIdx.x; d <= 2 * m; d += blockDim.x) e3[d] = exp_t(e.e3c * (T)((d - m) * (d - m)));
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+      int cell;
+      T fr;
+      reduce_sample<T>(t[i], pm, e.ng, cell, fr);
+      const T E1 = exp2_t(-e.k1 * fr * fr), E2 = exp2_t(e.k2 * fr);
+      const T w0 = y[i] * E1;
+      T w = w0;
+      for (int d = 0; d <= m; ++d) {
+        int c = cell + d;
+        if (c >= ng) c -= ng;
+        atomicAdd(&sr[real_slot(c)], w * e3[d + m]);
+        w *= E2;
+      }
+      const T E2i = (T)1 / E2;
+      w = w0 * E2i;
+      for (int d = -1; d > -m; --d) {
+        int c = cell + d;
+        if (c < 0) c += ng;
+        atomicAdd(&sr[real_slot(c)], w * e3[d + m]);
+        w *= E2i;
+      }
+    }
+  }
+  __syncthreads();
+  smem_fft<T, sizeof(T) == 4>(s, pitch, f.logL, 1, f.tw1);
+  for (int64_t k = threadIdx.x; k <= e.K; k += blockDim.x) {
+    const C Zk = s[pad16((int)(k & (L - 1)))];
+    const C Zm = cconj(s[pad16((int)((L - k) & (L - 1)))]);
+    acc_output<T>(e, k, Zk, Zm, F);
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_nfft_small(const double *__restrict__ t, const T *__restrict__ y,
+                                                     int64_t n, PhaseMul pm, AccParams<T> e, FftDev<T> f,
+                                                     typename CxOf<T>::type *F, const T *__restrict__ wts,
+                                                     bool gather) {
+  // one CTA per output slab: slab b grids wts[b*n + j] when wts is given
+  // (bootstrap resample b), else y[j]
+  if (wts) {
+    y = wts + (int64_t)blockIdx.x * n;
+    F += (int64_t)blockIdx.x * e.nf;
+  }
+  nfft_small_body<T>(t, y, n, pm, e, f, F, gather);
 }
 
 __device__ __forceinline__ void store4(float *p, float a, float b, float c, float d) {

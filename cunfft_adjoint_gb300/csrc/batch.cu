@@ -227,9 +227,9 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_bsmall(const do
                                                                         const T *__restrict__ y,
                                                                         const BDesc<T> *__restrict__ D,
                                                                         const int *__restrict__ list,
-                                                                        typename CxOf<T>::type *F) {
+                                                                        typename CxOf<T>::type *F, bool gather) {
   const BDesc<T> d = D[list[blockIdx.x]];
-  nfft_small_body<T>(t + d.s_off, y + d.s_off, d.n, d.pm, d.e, d.f, F + d.f_off);
+  nfft_small_body<T>(t + d.s_off, y + d.s_off, d.n, d.pm, d.e, d.f, F + d.f_off, gather);
 }
 
 template <typename T> AccParams<T> series_params(int64_t nf, int R, int m, double tau, int logTL) {
@@ -475,9 +475,9 @@ int batch_run(cuna2_batch_plan_st *p, const double *t, const T *y, typename CxOf
     for (size_t c = 0; c < p->small_classes.size(); ++c) {
       const int logL = p->small_classes[c].first, cnt = p->small_classes[c].second;
       const int L = 1 << logL;
-      const size_t smem = sizeof(C) * (size_t)fft_pitch(L, 1) + sizeof(T) * (2 * p->m_max + 2);
-      const int threads = std::max(32, std::min(1024, L / kFftE));
-      k_bsmall<T><<<cnt, threads, smem, p->side>>>(t, y, D, (const int *)p->d_small_list + p->small_class_off[c], F);
+      const bool alone = cnt <= device_sm_count(), gather = small_gather(L, alone, sizeof(T) == 4);
+      k_bsmall<T><<<cnt, small_threads<T>(L, alone, gather), small_smem<T>(L, p->m_max, gather), p->side>>>(
+          t, y, D, (const int *)p->d_small_list + p->small_class_off[c], F, gather);
       CUNA_CK(cudaGetLastError());
     }
     CUNA_CK(cudaEventRecord(p->ev_join, p->side));

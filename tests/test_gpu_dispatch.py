@@ -37,3 +37,64 @@ def test_compat_double_powers_and_factors(mods, oracle_lib, n, ng):
     f_hat = torch.zeros(ng, dtype=torch.complex128, device="cuda")
     cuna.cunfft_adjoint_raw(xd, yd, f_hat, n, ng, fp)
     assert rel_l2(f_hat.cpu().numpy(), oracle_lib.compat_adjoint(x, y, ng, "d")) < 1e-13
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.float64, 1e-9)])
+@pytest.mark.parametrize("R,m,nf,ns", [(2, 1, 1 << 15, 1), (2, 12, 1 << 15, 2), (4, 13, 1 << 14, 1), (8, 16, 1 << 13, 3),
+                                       (4, 6, 256, 2)])
+def test_backward_windows(mods, dtype, tol, R, m, nf, ns):
+    """The backward's windows at every alignment and over the grid's seam, for
+    narrow and wide filters, one and several series, against the exact
+    adjointness relation: <G, F(y)> = <dL/dy, y> for the plan's own forward,
+    whose gridding and FFT passes are other kernels (relative to the norms:
+    one plan precision's rounding of sums, 2e-5 and 1e-9)."""
+    _, nfft = mods
+    rng = np.random.default_rng(m)
+    n, T = 1001, 7.0
+    ng = R * nf
+    t = rng.uniform(0, T, (ns, n))
+    cells = np.concatenate([np.arange(20), ng - 1 - np.arange(20), rng.integers(0, ng, 160)])
+    t[:, :200] = (cells + rng.uniform(0.01, 0.99, 200)) / ng * T
+    y = rng.normal(0, 1, (ns, n))
+    G = rng.normal(0, 1, (ns, nf)) + 1j * rng.normal(0, 1, (ns, nf))
+    plan = nfft.AdjointNFFT(nf, R, m, dtype)
+    td, yd = torch.as_tensor(t, device="cuda"), torch.as_tensor(y, dtype=dtype, device="cuda")
+    Gd = torch.as_tensor(G, dtype=plan.cdtype, device="cuda")
+    gy, gt = plan.backward_batch(td, yd, Gd, 0.0, T)
+    for s in range(ns):
+        F = plan(td[s], yd[s], 0.0, T).to(torch.complex128)
+        Gs = Gd[s].to(torch.complex128)
+        lhs = float((Gs.conj() * F).real.sum())
+        rhs = float((gy[s].double() * yd[s].double()).sum())
+        assert abs(lhs - rhs) < tol * float(Gs.abs().square().sum().sqrt() * F.abs().square().sum().sqrt())
+        # dL/dt_j = dL/ds_j of moving one sample's time, by the same relation on
+        # the sample's own spectrum: y_j * d/dt of the field; its sum over all
+        # samples moved together is the derivative of <G, F> under a shift,
+        # which multiplies F_k by exp(2 pi i k dt / T)
+        k = torch.arange(-nf // 2, nf // 2, device="cuda", dtype=torch.float64)
+        dF = F * (2j * np.pi / T) * k
+        lhs = float((Gs.conj() * dF).real.sum())
+        rhs = float(gt[s].sum())
+        bound = float(Gs.abs().square().sum().sqrt() * dF.abs().square().sum().sqrt())
+        kernel = np.exp(-np.pi * m * np.sqrt(1 - 1 / R))
+        assert abs(lhs - rhs) < (tol + 20 * kernel) * bound
+
+
+@pytest.mark.parametrize("n,nf,R,m", [(0, 64, 2, 8), (1, 4, 4, 4), (3, 8, 4, 2), (40, 64, 2, 8), (33, 16, 2, 7),
+                                      (1000, 2048, 2, 8), (2049, 2048, 4, 12), (5000, 512, 2, 3), (300, 4096, 2, 16)])
+def test_small_gather(mods, oracle_lib, n, nf, R, m):
+    """One-CTA float transforms: windows wider than a third of the grid (the
+    gather's periodic images), one and several chunks of records, samples on
+    the seam, empty input; against the oracle's double restatement of the same
+    sums (float rounding of about 2m n terms, 2e-6)."""
+    _, nfft = mods
+    rng = np.random.default_rng(n + nf)
+    t = rng.uniform(0, 3.0, n)
+    t[:2] = [0.0, np.nextafter(3.0, 0)][:min(n, 2)]
+    y = rng.normal(0, 1, n).astype(np.float32)
+    plan = nfft.AdjointNFFT(nf, R, m, torch.float32)
+    F = plan(torch.as_tensor(t, device="cuda"), torch.as_tensor(y, device="cuda"), 0.0, 3.0).cpu().numpy()
+    if n == 0:
+        assert not F.any()
+        return
+    assert rel_l2(F, oracle_lib.accurate_adjoint(t, y.astype(np.float64), 0.0, 3.0, nf, R, m)) < 2e-6
