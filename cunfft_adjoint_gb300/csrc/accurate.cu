@@ -33,6 +33,7 @@
 #include "accurate_kernels.cuh"
 #include "backward.h"
 #include "fftpass.cuh"
+#include "fftpass_df.cuh"
 
 struct cuna2_plan_st {
   int dtype;
@@ -147,8 +148,8 @@ inline void mark(Prof *pr, const char *name, cudaStream_t st) {
 // lengths that have an instance: returns 1 when launched, 0 when logL has no
 // instance, -1 on a launch error.
 template <typename T, int LOGL, int LOGE>
-int ct_passes_sized(typename MemOf<T>::type *z, const FftDev<T> &f, const AccParams<typename AccOf<T>::type> &e,
-                    typename MemOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
+int ct_passes_sized(typename CxOf<T>::type *z, const FftDev<T> &f, const AccParams<T> &e,
+                    typename CxOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
   constexpr int BA = 1 << (LOGE - LOG1), TH = 1 << (LOGE - 4);
   constexpr size_t smA = ct_colpass_smem<T, LOGL, LOGE>(), smB = ct_rowpass_smem<T, LOGL, LOGE>();
@@ -183,15 +184,15 @@ int ct_passes_sized(typename MemOf<T>::type *z, const FftDev<T> &f, const AccPar
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
   mark(pr, "fft_colpass", st);
   if (launch_pdl(k_ct_rowpass_acc<T, LOGL, LOGE>, dim3(ct_rowpass_ctas<T, LOGL, LOGE>(), nslab), dim3(TH), smB, st,
-                 (const typename MemOf<T>::type *)z, f, e, F) != cudaSuccess)
+                 (const typename CxOf<T>::type *)z, f, e, F) != cudaSuccess)
     return -1;
   mark(pr, "fft_rowpass", st);
   return 1;
 }
 
 template <typename T, int LOGL>
-int ct_passes_at(typename MemOf<T>::type *z, const FftDev<T> &f, const AccParams<typename AccOf<T>::type> &e,
-                 typename MemOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
+int ct_passes_at(typename CxOf<T>::type *z, const FftDev<T> &f, const AccParams<T> &e,
+                 typename CxOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
   if constexpr (sizeof(T) == 4)
     if (pass_few<T>(LOGL, nslab, 4) && !tma_enabled())
       return ct_passes_sized<T, LOGL, PassFew<T, LOGL>::LOGE>(z, f, e, F, nslab, st, pr);
@@ -199,8 +200,8 @@ int ct_passes_at(typename MemOf<T>::type *z, const FftDev<T> &f, const AccParams
 }
 
 template <typename T>
-int ct_passes(int logL, typename MemOf<T>::type *z, const FftDev<T> &f, const AccParams<typename AccOf<T>::type> &e,
-              typename MemOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
+int ct_passes(int logL, typename CxOf<T>::type *z, const FftDev<T> &f, const AccParams<T> &e,
+              typename CxOf<T>::type *F, int nslab, cudaStream_t st, Prof *pr) {
 #define CUNA_CT(LG) \
   case LG: return ct_passes_at<T, LG>(z, f, e, F, nslab, st, pr);
   if constexpr (sizeof(T) == 4) {
@@ -480,17 +481,20 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   // packed complex view of the real grid slabs
   C *z = reinterpret_cast<C *>(grid);
   {
-    int h;
     if constexpr (sizeof(T) == 8) {
-      // double plans compute both passes in float-float (the FP32 pipe) and
-      // keep the grid and the spectrum in double
-      if (p->has_df && !fp64_passes_forced())
-        h = ct_passes<dfl>(p->geom.logL, z, to_dev<dfl>(p->geom_df), e, F, nslab, st, pr);
-      else
-        h = ct_passes<T>(p->geom.logL, z, f, e, F, nslab, st, pr);
-    } else {
-      h = ct_passes<T>(p->geom.logL, z, f, e, F, nslab, st, pr);
+      // double plans compute both passes in float-float (the FP32 pipe); the
+      // grid and the spectrum are double, the values between the passes
+      // float-float in the grid's memory
+      if (p->has_df && !fp64_passes_forced()) {
+        const FftDev<dfl> fd = to_dev<dfl>(p->geom_df);
+        CUNA_TRY(df_colpass(z, fd, nslab, st));
+        mark(pr, "fft_colpass", st);
+        CUNA_TRY(df_rowpass(z, fd, e, F, nslab, st));
+        mark(pr, "fft_rowpass", st);
+        return CUNA2_SUCCESS;
+      }
     }
+    const int h = ct_passes<T>(p->geom.logL, z, f, e, F, nslab, st, pr);
     if (h < 0) return fail_cuda(cudaGetLastError(), "FFT pass launch");
     if (h == 1) return CUNA2_SUCCESS;
   }

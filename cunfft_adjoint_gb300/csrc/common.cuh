@@ -111,45 +111,22 @@ __device__ __forceinline__ dfl df_rcp(dfl a) {
   const dfl e = dfl(1.0f, 0.f) - a * r0;
   return r0 + r0 * e;
 }
+// A float-float complex value: the two parts' high floats packed in one
+// 64-bit register pair, their low floats in another (re in the low half).
 struct __align__(16) dcx {
-  dfl x, y;
+  unsigned long long h, l;
 };
 
 template <typename T> struct CxOf;
 template <> struct CxOf<float> { typedef float2 type; };
 template <> struct CxOf<double> { typedef double2 type; };
 template <> struct CxOf<dfl> { typedef dcx type; };
-// the element type a complex array of the plan type is stored as in memory
-// (the float-float passes read and write double)
-template <typename T> struct MemOf { typedef typename CxOf<T>::type type; };
-template <> struct MemOf<dfl> { typedef double2 type; };
-// the scalar the plan's epilogue parameters are kept in
-template <typename T> struct AccOf { typedef T type; };
-template <> struct AccOf<dfl> { typedef double type; };
-
 __host__ __device__ __forceinline__ float2 cmk(float a, float b) { return make_float2(a, b); }
 __host__ __device__ __forceinline__ double2 cmk(double a, double b) { return make_double2(a, b); }
-__host__ __device__ __forceinline__ dcx cmk(dfl a, dfl b) {
-  dcx c;
-  c.x = a;
-  c.y = b;
-  return c;
-}
 
-// memory <-> computation forms of a complex value, and read-only twiddle loads
-template <typename C, typename M> __device__ __forceinline__ C cx_load(M v) { return v; }
-template <> __device__ __forceinline__ dcx cx_load<dcx, double2>(double2 v) {
-  return cmk(df_from_double(v.x), df_from_double(v.y));
-}
-__device__ __forceinline__ float2 cx_to_mem(float2 v) { return v; }
-__device__ __forceinline__ double2 cx_to_mem(double2 v) { return v; }
-__device__ __forceinline__ double2 cx_to_mem(dcx v) { return make_double2(df_to_double(v.x), df_to_double(v.y)); }
+// read-only twiddle loads
 __device__ __forceinline__ float2 ldtw(const float2 *p) { return __ldg(p); }
 __device__ __forceinline__ double2 ldtw(const double2 *p) { return __ldg(p); }
-__device__ __forceinline__ dcx ldtw(const dcx *p) {
-  const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
-  return cmk(dfl(v.x, v.y), dfl(v.z, v.w));
-}
 
 template <typename C> __host__ __device__ __forceinline__ C cadd(C a, C b) { return cmk(a.x + b.x, a.y + b.y); }
 template <typename C> __host__ __device__ __forceinline__ C csub(C a, C b) { return cmk(a.x - b.x, a.y - b.y); }

@@ -168,15 +168,15 @@ __device__ __forceinline__ void ct_fft(typename CxOf<T>::type *s, const typename
 // (row-major L1 x L2), times W_L^{c k1}, stored in place.
 // ---------------------------------------------------------------------------
 template <typename T, int LOG1, int LOG2> struct CtColSrc {
-  const typename MemOf<T>::type *p;  // slab + c0
+  const typename CxOf<T>::type *p;  // slab + c0
   __device__ __forceinline__ typename CxOf<T>::type load(int seq, int j, int dr) const {
     // through L2: the gridding may still have been writing when this kernel started
-    return cx_load<typename CxOf<T>::type>(__ldcg(p + ((j + dr) << LOG2) + seq));
+    return __ldcg(p + ((j + dr) << LOG2) + seq);
   }
 };
 
 template <typename T, int LOG1, int LOG2, int LOGB> struct CtColDst {
-  typename MemOf<T>::type *p;             // slab + c0
+  typename CxOf<T>::type *p;             // slab + c0
   const typename CxOf<T>::type *steps;    // shared: steps[seq * 17 + r] = W_L^{c (r << LOGNS_last)}
   FftDev<T> f;
   int c0;
@@ -188,7 +188,7 @@ template <typename T, int LOG1, int LOG2, int LOGB> struct CtColDst {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const C w = r == 0 ? w0 : cmul(w0, steps[seq * 17 + r]);
-      p[((idxD + (r << LOGNS)) << LOG2) + seq] = cx_to_mem(cmul(v[r], w));
+      p[((idxD + (r << LOGNS)) << LOG2) + seq] = cmul(v[r], w);
     }
   }
 };
@@ -202,7 +202,7 @@ template <int LOGN> __host__ __device__ constexpr int last_logns() {
 // `in` to `out` (in == out allowed: every read precedes the first barrier,
 // every write follows it)
 template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE>
-__device__ __forceinline__ void ct_colpass_body(const typename MemOf<T>::type *in, typename MemOf<T>::type *out,
+__device__ __forceinline__ void ct_colpass_body(const typename CxOf<T>::type *in, typename CxOf<T>::type *out,
                                                 const FftDev<T> &f, int cblock) {
   typedef typename CxOf<T>::type C;
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
@@ -227,9 +227,9 @@ __device__ __forceinline__ void ct_colpass_body(const typename MemOf<T>::type *i
 }
 
 template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE>
-__global__ void __launch_bounds__(1 << (LOGE - 4)) k_ct_colpass(typename MemOf<T>::type *grid, FftDev<T> f,
+__global__ void __launch_bounds__(1 << (LOGE - 4)) k_ct_colpass(typename CxOf<T>::type *grid, FftDev<T> f,
                                                                 int64_t slab_stride) {
-  typename MemOf<T>::type *z = grid + blockIdx.y * slab_stride;
+  typename CxOf<T>::type *z = grid + blockIdx.y * slab_stride;
   ct_colpass_body<T, LOGL, LOGE>(z, z, f, blockIdx.x);
 }
 

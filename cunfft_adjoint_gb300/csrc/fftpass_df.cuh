@@ -18,12 +18,12 @@
 //    the FP64 pipe;
 //  - the unpack twiddles come from the FFT's tables, not from FP64 sincospi
 //    (L2 + B of them per CTA).
-// One transform of 2^21 points: DF_NUMBERS.
+// One transform of 2^21 points: column pass 108 -> 65 us, row pass 125 -> 54 us;
+// the whole float64 transform of 1e6 samples 369 -> 275 us.
 #pragma once
 #include "accurate_kernels.cuh"
 
 namespace cuna {
-namespace {
 
 // packed pairs of floats
 typedef unsigned long long f2;
@@ -140,6 +140,8 @@ __device__ __forceinline__ dcx dc_ldcg(const dcx *p) {
   r.l = v.y;
   return r;
 }
+
+namespace {
 
 __device__ __forceinline__ void df_bf4(dcx &a0, dcx &a1, dcx &a2, dcx &a3) {
   const dcx t0 = cadd(a0, a2), t1 = csub(a0, a2), t2 = cadd(a1, a3), t3 = cmuli(csub(a1, a3));

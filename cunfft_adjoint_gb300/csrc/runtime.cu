@@ -94,15 +94,6 @@ struct TwEntry {
 std::mutex g_tw_mu;
 std::map<std::tuple<int, int, int>, TwEntry> *g_tw = new std::map<std::tuple<int, int, int>, TwEntry>();
 
-// float-float table entries: the double value as its nearest float and the
-// remainder, laid out as the device's float-float complex (re.hi, re.lo,
-// im.hi, im.lo)
-struct DfPair {
-  float hi, lo;
-  DfPair() = default;
-  explicit DfPair(double d) : hi((float)d), lo((float)(d - (double)(float)d)) {}
-};
-
 template <typename T>
 int upload_table(int64_t count, int64_t step_num, int64_t denom, const void **out) {
   // entries exp(+2 pi i * q * step_num / denom), q < count, in double then rounded
@@ -116,6 +107,29 @@ int upload_table(int64_t count, int64_t step_num, int64_t denom, const void **ou
   }
   void *d = nullptr;
   size_t bytes = sizeof(T) * h.size();
+  cudaError_t e = cudaMalloc(&d, bytes);
+  if (e != cudaSuccess) return fail_cuda(e, "cudaMalloc(twiddles)");
+  e = cudaMemcpy(d, h.data(), bytes, cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return fail_cuda(e, "cudaMemcpy(twiddles)");
+  *out = d;
+  return CUNA2_SUCCESS;
+}
+
+// The same table in float-float, laid out as the device's float-float complex:
+// (re.hi, im.hi, re.lo, im.lo), each double as its nearest float and the
+// remainder.
+int upload_table_df(int64_t count, int64_t step_num, int64_t denom, const void **out) {
+  std::vector<float> h(4 * (size_t)count);
+  for (int64_t q = 0; q < count; ++q) {
+    const int64_t num = (q * step_num) % denom;
+    const double a = 2.0 * M_PI * (double)num / (double)denom, v[2] = {cos(a), sin(a)};
+    for (int k = 0; k < 2; ++k) {
+      h[4 * q + k] = (float)v[k];
+      h[4 * q + 2 + k] = (float)(v[k] - (double)(float)v[k]);
+    }
+  }
+  void *d = nullptr;
+  const size_t bytes = sizeof(float) * h.size();
   cudaError_t e = cudaMalloc(&d, bytes);
   if (e != cudaSuccess) return fail_cuda(e, "cudaMalloc(twiddles)");
   e = cudaMemcpy(d, h.data(), bytes, cudaMemcpyHostToDevice);
@@ -144,10 +158,10 @@ int fft_geometry_df(int logL, FftGeom *g) {
   const int64_t L = int64_t(1) << logL, L1 = int64_t(1) << G.logL1, L2 = int64_t(1) << G.logL2;
   const int64_t nlo = L < 2048 ? L : 2048, nhi = L / nlo;
   int st;
-  if ((st = upload_table<DfPair>(L1, 1, L1, &G.tw1))) return st;
-  if ((st = upload_table<DfPair>(L2, 1, L2, &G.tw2))) return st;
-  if ((st = upload_table<DfPair>(nlo, 1, L, &G.twlo))) return st;
-  if ((st = upload_table<DfPair>(nhi, nlo, L, &G.twhi))) return st;
+  if ((st = upload_table_df(L1, 1, L1, &G.tw1))) return st;
+  if ((st = upload_table_df(L2, 1, L2, &G.tw2))) return st;
+  if ((st = upload_table_df(nlo, 1, L, &G.twlo))) return st;
+  if ((st = upload_table_df(nhi, nlo, L, &G.twhi))) return st;
   (*g_tw)[key] = TwEntry{G};
   *g = G;
   return CUNA2_SUCCESS;

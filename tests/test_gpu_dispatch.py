@@ -98,3 +98,19 @@ def test_small_gather(mods, oracle_lib, n, nf, R, m):
         assert not F.any()
         return
     assert rel_l2(F, oracle_lib.accurate_adjoint(t, y.astype(np.float64), 0.0, 3.0, nf, R, m)) < 2e-6
+
+
+@pytest.mark.parametrize("nf,R,m", [(1 << 13, 4, 12), (1 << 15, 2, 16), (1 << 17, 2, 10), (1 << 17, 8, 16), (1 << 19, 4, 12)])
+def test_float_float_passes_lengths(mods, oracle_lib, nf, R, m):
+    """Float-float FFT passes at lengths of every leading radix (2, 4, 8) in
+    either pass, against the oracle's double restatement of the same sums (a
+    float-float pass rounds at about 2^-46 per operation, log2(ng) of them:
+    below 1e-12)."""
+    _, nfft = mods
+    rng = np.random.default_rng(nf + R)
+    n = 3000
+    t = rng.uniform(0, 50.0, n)
+    y = rng.normal(0, 1, n)
+    plan = nfft.AdjointNFFT(nf, R, m, torch.float64)
+    F = plan(torch.as_tensor(t, device="cuda"), torch.as_tensor(y, device="cuda"), 0.0, 50.0).cpu().numpy()
+    assert rel_l2(F, oracle_lib.accurate_adjoint(t, y, 0.0, 50.0, nf, R, m)) < 1e-12
