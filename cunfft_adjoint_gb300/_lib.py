@@ -145,3 +145,15 @@ def check(status):
 
 def library_paths():
     return [os.path.join(LIB_DIR, n) for n in ("libcuna_gb300.so", "libcunaf.so", "libcunad.so")]
+
+
+def stream_handle(stream, device):
+    """The CUDA stream handle of `stream`, or of the current stream of `device`
+    (read without making a Stream object, which costs as much as a launch)."""
+    if stream is not None:
+        return stream.cuda_stream or None
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return torch.cuda.current_stream(device).cuda_stream or None
+    return raw(torch.cuda.current_device() if device.index is None else device.index) or None

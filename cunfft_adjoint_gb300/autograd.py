@@ -17,7 +17,7 @@ import torch
 class AdjointNFFTFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, t, y, plan, t0, T):
-        F = plan.adjoint(t.detach(), y.detach(), t0, T)
+        F = plan.adjoint(t, y, t0, T)
         ctx.save_for_backward(t, y)
         ctx.plan, ctx.t0, ctx.T = plan, t0, T
         return F
@@ -26,7 +26,7 @@ class AdjointNFFTFunction(torch.autograd.Function):
     def backward(ctx, grad_F):
         t, y = ctx.saved_tensors
         need_t, need_y = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-        gy, gt = ctx.plan.backward(t.detach(), y.detach(), grad_F, ctx.t0, ctx.T, need_y, need_t)
+        gy, gt = ctx.plan.backward(t, y, grad_F, ctx.t0, ctx.T, need_y, need_t)
         return gt, gy, None, None, None
 
 
@@ -38,7 +38,7 @@ def adjoint_nfft(t, y, plan, t0, T):
 class _BatchFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, t, y, op):
-        F = op.bplan(t.detach().reshape(-1), y.detach().reshape(-1)).view(op.B, op.nf)
+        F = op.bplan(t, y).view(op.B, op.nf)
         ctx.save_for_backward(t, y)
         ctx.op = op
         return F
@@ -49,7 +49,7 @@ class _BatchFunction(torch.autograd.Function):
         op = ctx.op
         need_t, need_y = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         # all series' vector-Jacobian products in one batched execution
-        gy, gt = op.plan.backward_batch(t.detach(), y.detach(), grad_F, op.t0, op.T, need_y, need_t)
+        gy, gt = op.plan.backward_batch(t, y, grad_F, op.t0, op.T, need_y, need_t)
         return gt, gy, None
 
 

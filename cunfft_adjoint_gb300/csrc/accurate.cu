@@ -153,7 +153,7 @@ int ct_passes_sized(typename CxOf<T>::type *z, const FftDev<T> &f, const AccPara
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
   constexpr int BA = 1 << (LOGE - LOG1), TH = 1 << (LOGE - 4);
   constexpr size_t smA = ct_colpass_smem<T, LOGL, LOGE>(), smB = ct_rowpass_smem<T, LOGL, LOGE>();
-  static char attr;
+  static SetupFlag attr;
   if (!setup_done(&attr)) {
     if (cudaFuncSetAttribute(k_ct_colpass<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
         cudaFuncSetAttribute(k_ct_rowpass_acc<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB))
@@ -166,7 +166,7 @@ int ct_passes_sized(typename CxOf<T>::type *z, const FftDev<T> &f, const AccPara
     int *tmo = tma_enabled() ? wait_timeout_counter() : nullptr;
     alignas(64) CUtensorMap map;
     if (tmo && ct_colpass_tma_map<LOGL>(&map, z, nslab)) {
-      static char attr_tma;
+      static SetupFlag attr_tma;
       if (!setup_done(&attr_tma)) {
         if (cudaFuncSetAttribute(k_ct_colpass_tma<LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ct_colpass_tma_smem<LOGL>()))
@@ -315,7 +315,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     return fail(CUNA2_ERROR_UNSUPPORTED, "record inspection needs a tiled plan with the global binning form");
   mark(pr, "start", st);
   if (nbs > 0) {
-    static char attrw;
+    static SetupFlag attrw;
     if (!setup_done(&attrw)) {
       CUNA_CK(cudaFuncSetAttribute(k_boot_weights<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)(sizeof(int) * kBootSmemN)));
@@ -328,7 +328,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     mark(pr, "boot_weights", st);
   }
   if (small) {
-    static char attr;
+    static SetupFlag attr;
     if (!setup_done(&attr)) {
       CUNA_CK(cudaFuncSetAttribute(k_nfft_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
       mark_setup_done(&attr);
@@ -352,7 +352,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     // count (caching each sample's phase) and reserve, then scan + scatter
     SampAcc<T> smp{t, y, n, pm, e, phases};
     SampAccS<T> sms{phases, y, n, e};
-    static char attrs;
+    static SetupFlag attrs;
     if (!setup_done(&attrs)) {
       CUNA_CK(cudaFuncSetAttribute(k_bin_scatter_resv<SampAccS<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)(sizeof(int) * (3 * kScanFuseTiles + 1))));
@@ -404,7 +404,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   const int ch2 = 2 * CH;
   // gather: 8 cells per thread on tiles of 2048 cells, else 4
   const bool cw8 = (1 << p->logTL) == 2048;
-  static char attr_done;
+  static SetupFlag attr_done;
   if (!setup_done(&attr_done)) {
     const int mx = 200 * 1024;
     CUNA_CK(cudaFuncSetAttribute(k_grid_acc<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
@@ -504,7 +504,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   const int BA = elems / L1, BB = elems / L2, PB = BB / 2;
   const size_t smemA = sizeof(C) * (size_t)BA * fft_pitch(L1, BA);
   const size_t smemB = sizeof(C) * (size_t)BB * fft_pitch(L2, BB);
-  static char attr2;
+  static SetupFlag attr2;
   if (!setup_done(&attr2)) {
     CUNA_CK(cudaFuncSetAttribute(k_fft_colpass<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUNA_CK(cudaFuncSetAttribute(k_fft_rowpass_acc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

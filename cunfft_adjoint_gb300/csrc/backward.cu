@@ -383,7 +383,7 @@ int bwd_passes_sized(const BwdSpec<T> &sp, typename CxOf<T>::type *z, typename C
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2, BA = 1 << (LOGE - LOG1), BB = 1 << (LOGE - LOG2);
   constexpr size_t smA = ct_colpass_smem<T, LOGL, LOGE>() + sizeof(C) * 2 * BA;
   constexpr size_t smB = sizeof(C) * (size_t)fft_pitch(1 << LOG2, BB) * BB;
-  static char attr;
+  static SetupFlag attr;
   if (!setup_done(&attr)) {
     CUNA_CK(cudaFuncSetAttribute(k_ct_bwd_col<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA));
     CUNA_CK(cudaFuncSetAttribute(k_ct_bwd_row<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB));
@@ -453,7 +453,7 @@ template <typename T> int backward_group(const BwdArgs<T> &a, cudaStream_t st) {
   cf.k1 = (T)(1.0 / (4.0 * a.tau * log(2.0)));
   cf.inv2tau = (T)2.0 * (T)(1.0 / (4.0 * a.tau));
   if (a.small) {
-    static char attr;
+    static SetupFlag attr;
     if (!setup_done(&attr)) {
       CUNA_CK(cudaFuncSetAttribute(k_bwd_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
       mark_setup_done(&attr);

@@ -187,7 +187,7 @@ int bct_sized(T *grid, const BDesc<T> *D, const int *list, int cnt, typename CxO
   constexpr int LOG1 = (LOGL + 1) / 2, LOG2 = LOGL / 2;
   constexpr int BA = 1 << (LOGE - LOG1), TH = 1 << (LOGE - 4);
   constexpr size_t smA = ct_colpass_smem<T, LOGL, LOGE>(), smB = ct_rowpass_smem<T, LOGL, LOGE>();
-  static char attr;
+  static SetupFlag attr;
   if (!setup_done(&attr)) {
     if (cudaFuncSetAttribute(k_bct_colpass<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
         cudaFuncSetAttribute(k_bct_rowpass<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB))
@@ -456,7 +456,7 @@ int batch_run(cuna2_batch_plan_st *p, const double *t, const T *y, typename CxOf
   typedef typename RecOf<T>::type Rec;
   if ((p->n_total > 0 && (!t || !y)) || !F) return fail(CUNA2_ERROR_INVALID_VALUE, "NULL array");
   const BDesc<T> *D = (const BDesc<T> *)p->d_desc;
-  static char attr;
+  static SetupFlag attr;
   if (!setup_done(&attr)) {
     CUNA_CK(cudaFuncSetAttribute(k_bsmall<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     CUNA_CK(cudaFuncSetAttribute(k_bgrid<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -469,18 +469,23 @@ int batch_run(cuna2_batch_plan_st *p, const double *t, const T *y, typename CxOf
     mark_setup_done(&attr);
   }
   // small series on the side stream, overlapping the large-series pipeline
+  // (on the caller's where there is none: no fork, no events)
+  const bool fork = !p->small_classes.empty() && p->tiles_total > 0;
   if (!p->small_classes.empty()) {
-    CUNA_CK(cudaEventRecord(p->ev_fork, st));
-    CUNA_CK(cudaStreamWaitEvent(p->side, p->ev_fork, 0));
+    const cudaStream_t ss = fork ? p->side : st;
+    if (fork) {
+      CUNA_CK(cudaEventRecord(p->ev_fork, st));
+      CUNA_CK(cudaStreamWaitEvent(p->side, p->ev_fork, 0));
+    }
     for (size_t c = 0; c < p->small_classes.size(); ++c) {
       const int logL = p->small_classes[c].first, cnt = p->small_classes[c].second;
       const int L = 1 << logL;
       const bool alone = cnt <= device_sm_count(), gather = small_gather(L, alone, sizeof(T) == 4);
-      k_bsmall<T><<<cnt, small_threads<T>(L, alone, gather), small_smem<T>(L, p->m_max, gather), p->side>>>(
+      k_bsmall<T><<<cnt, small_threads<T>(L, alone, gather), small_smem<T>(L, p->m_max, gather), ss>>>(
           t, y, D, (const int *)p->d_small_list + p->small_class_off[c], F, gather);
       CUNA_CK(cudaGetLastError());
     }
-    CUNA_CK(cudaEventRecord(p->ev_join, p->side));
+    if (fork) CUNA_CK(cudaEventRecord(p->ev_join, p->side));
   }
   if (p->tiles_total > 0) {
     const int ntl = p->tiles_total;
@@ -540,7 +545,7 @@ int batch_run(cuna2_batch_plan_st *p, const double *t, const T *y, typename CxOf
       CUNA_CK(cudaGetLastError());
     }
   }
-  if (!p->small_classes.empty()) CUNA_CK(cudaStreamWaitEvent(st, p->ev_join, 0));
+  if (fork) CUNA_CK(cudaStreamWaitEvent(st, p->ev_join, 0));
   return CUNA2_SUCCESS;
 }
 

@@ -500,7 +500,7 @@ int compat_ct_sized(typename CxOf<T>::type *f_hat, typename CxOf<T>::type *scrat
   constexpr int BA = 1 << (LOGE - LOG1), BB = 1 << (LOGE - LOG2), TH = 1 << (LOGE - 4);
   constexpr size_t smA = ct_colpass_smem<T, LOGL, LOGE>();
   constexpr size_t smB = sizeof(typename CxOf<T>::type) * (size_t)fft_pitch(1 << LOG2, BB) * BB;
-  static char attr;
+  static SetupFlag attr;
   if (!setup_done(&attr)) {
     if (cudaFuncSetAttribute(k_ct_colpass_oop<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA) ||
         cudaFuncSetAttribute(k_ct_rowpass_compat<T, LOGL, LOGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -632,7 +632,7 @@ int compat_fft(typename CxOf<T>::type *f_hat, int ng, int nbs, const typename Fp
     const int L = 1 << logL;
     const int threads = max(32, L / kFftE);
     const size_t smem = sizeof(C) * (size_t)fft_pitch(L, 1);
-    static char attr;
+    static SetupFlag attr;
     if (!setup_done(&attr)) {
       CUNA_CK(cudaFuncSetAttribute(k_fft_single_compat<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    200 * 1024));
@@ -653,7 +653,7 @@ int compat_fft(typename CxOf<T>::type *f_hat, int ng, int nbs, const typename Fp
   const int BA = elems / L1, BB = elems / L2;
   const size_t smemA = sizeof(C) * (size_t)BA * fft_pitch(L1, BA);
   const size_t smemB = sizeof(C) * (size_t)BB * fft_pitch(L2, BB);
-  static char attr2;
+  static SetupFlag attr2;
   if (!setup_done(&attr2)) {
     CUNA_CK(cudaFuncSetAttribute(k_fft_colpass<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUNA_CK(cudaFuncSetAttribute(k_fft_rowpass_compat<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -737,7 +737,7 @@ int compat_bin(const T *x, const T *y, int n, int ng, const typename FpOf<T>::ty
     // count + reserve, then scan + scatter without global atomics (binning.cuh)
     const int64_t span = resv_span(n, ntiles, device_sm_count());
     const size_t sms3 = sizeof(int) * (3 * (size_t)ntiles + 1);
-    static char attr;
+    static SetupFlag attr;
     if (!setup_done(&attr)) {
       const int mx = (int)(sizeof(int) * (3 * kScanFuseTiles + 1));
       CUNA_CK(cudaFuncSetAttribute(k_bin_scatter_resv<SampCompat<T, false>>,

@@ -344,7 +344,7 @@ inline int df_log_elems(int logL, int logLseq, int nslab) {
 inline int df_colpass(double2 *z, const FftDev<dfl> &f, int nslab, cudaStream_t st) {
   const int le = df_log_elems(f.logL, f.logL1, nslab), logB = le - f.logL1;
   const size_t sm = sizeof(dcx) * ((size_t)df_pitch(1 << f.logL1, 1 << logB) + 8) << logB;
-  static char attr;
+  static SetupFlag attr;
   if (!setup_done(&attr)) {
     CUNA_CK(cudaFuncSetAttribute(k_df_colpass, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUNA_CK(cudaFuncSetAttribute(k_df_rowpass_acc, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

@@ -1,10 +1,10 @@
 // runtime.cu -- see runtime.h.
 #include <math.h>
 #include <stdarg.h>
+#include <atomic>
 #include <stdio.h>
 #include <map>
 #include <mutex>
-#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -71,16 +71,15 @@ int stream_workspace(cudaStream_t stream, size_t bytes, void **ptr) {
 }
 
 int device_sm_count() {
-  static std::mutex mu;
-  static std::map<int, int> cache;
+  static std::atomic<int> cache[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 1;
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = cache.find(dev);
-  if (it != cache.end()) return it->second;
-  int sms = 1;
+  const bool known = dev >= 0 && dev < 64;
+  int sms = known ? cache[dev].load(std::memory_order_relaxed) : 0;
+  if (sms > 0) return sms;
+  sms = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cache[dev] = sms;
+  if (known) cache[dev].store(sms, std::memory_order_relaxed);
   return sms;
 }
 
@@ -236,23 +235,16 @@ int *g_timeouts_dev = nullptr;
 std::once_flag g_timeouts_once;
 }  // namespace
 
-namespace {
-std::mutex g_setup_mu;
-std::set<std::pair<int, const void *>> *g_setup = new std::set<std::pair<int, const void *>>();
-}  // namespace
-
-bool setup_done(const void *key) {
+bool setup_done(const SetupFlag *flag) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  std::lock_guard<std::mutex> lk(g_setup_mu);
-  return g_setup->count(std::make_pair(dev, key)) != 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  return (flag->devices.load(std::memory_order_acquire) >> dev) & 1;
 }
 
-void mark_setup_done(const void *key) {
+void mark_setup_done(SetupFlag *flag) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
-  std::lock_guard<std::mutex> lk(g_setup_mu);
-  g_setup->insert(std::make_pair(dev, key));
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  flag->devices.fetch_or((uint64_t)1 << dev, std::memory_order_release);
 }
 
 int *wait_timeout_counter() {

@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
+#include <atomic>
 #include <stdint.h>
 #include "../../include/cuna2.h"
 
@@ -61,12 +62,16 @@ int fft_geometry(bool is_double, int logL, FftGeom *g, bool split = false);
 // same tables as the double one, each entry a float-float complex.
 int fft_geometry_df(int logL, FftGeom *g);
 
-// One-time per-device setup (kernel attributes): setup_done(key) tells whether
-// `key` has been marked on the current device, mark_setup_done(key) marks it.
-// Thread-safe; two threads may both run an idempotent setup before it is
-// marked.
-bool setup_done(const void *key);
-void mark_setup_done(const void *key);
+// One-time per-device setup (kernel attributes): a static flag per setup,
+// setup_done(&flag) tells whether it has been marked on the current device,
+// mark_setup_done(&flag) marks it.  Thread-safe; two threads may both run an
+// idempotent setup before it is marked.  (One bit per device: several are asked
+// on every call.)
+struct SetupFlag {
+  std::atomic<uint64_t> devices{0};
+};
+bool setup_done(const SetupFlag *flag);
+void mark_setup_done(SetupFlag *flag);
 
 // Device pointer (host-mapped) of the counter of bounded waits that ran out;
 // nullptr when mapped host memory is unavailable (TMA kernels are then not

@@ -27,9 +27,9 @@ def lomb_scargle(t, y, dy=None, nfreq=None, df=None, t0=None, R=2, m=8, out=None
         raise ValueError("nfreq is required")
     if out is None:
         out = torch.empty(int(nfreq), dtype=y.dtype, device=t.device)
-    s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
+    s = _lib.stream_handle(stream, t.device)
     dt = _lib.F32 if y.dtype == torch.float32 else _lib.F64
     _lib.check(_lib.core().cuna2_lomb_scargle(dt, t.data_ptr(), y.data_ptr(), None if dy is None else dy.data_ptr(),
                                               t.numel(), int(nfreq), float(df), float(t0), int(R), int(m),
-                                              out.data_ptr(), s or None))
+                                              out.data_ptr(), s))
     return out

@@ -9,9 +9,16 @@ plans) or complex128.
 """
 import ctypes
 
+import numpy as np
 import torch
 
 from . import _lib
+
+
+def _per_series(v, n):
+    """v as n contiguous doubles (one value for all, or one each)."""
+    a = np.array(v, np.float64)
+    return a if a.shape == (n,) else np.ascontiguousarray(np.broadcast_to(a, (n,)))
 
 
 class AdjointNFFT:
@@ -27,11 +34,11 @@ class AdjointNFFT:
         t, y, t0, T = AdjointNFFT._check(self, t, y, t0, T)
         out = torch.empty(self.nf, dtype=self.cdtype, device=t.device)
         R, m = ctypes.c_int(), ctypes.c_int()
-        s = torch.cuda.current_stream(t.device).cuda_stream
+        s = _lib.stream_handle(None, t.device)
         with torch.cuda.device(self.device):
             _lib.check(_lib.core().cuna2_plan_create_auto(
                 ctypes.byref(self._h), _lib.F32 if dtype == torch.float32 else _lib.F64, self.nf, float(tol),
-                t.data_ptr(), y.data_ptr(), out.data_ptr(), t.numel(), float(t0), float(T), s or None,
+                t.data_ptr(), y.data_ptr(), out.data_ptr(), t.numel(), float(t0), float(T), s,
                 ctypes.byref(R), ctypes.byref(m)))
         self.R, self.m = R.value, m.value
         ng, tau = ctypes.c_int64(), ctypes.c_double()
@@ -86,9 +93,9 @@ class AdjointNFFT:
         n = t.numel()
         if out is None:
             out = torch.empty(self.nf, dtype=self.cdtype, device=t.device)
-        s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
+        s = _lib.stream_handle(stream, t.device)
         _lib.check(_lib.core().cuna2_adjoint(self._h, t.data_ptr(), y.data_ptr(), out.data_ptr(), n,
-                                             float(t0), float(T), s or None))
+                                             float(t0), float(T), s))
         return out
 
     def bootstrap(self, t, y, nbs, seed=0, t0=None, T=None, out=None, stream=None):
@@ -96,10 +103,10 @@ class AdjointNFFT:
         t, y, t0, T = self._check(t, y, t0, T)
         if out is None:
             out = torch.empty((nbs, self.nf), dtype=self.cdtype, device=t.device)
-        s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
+        s = _lib.stream_handle(stream, t.device)
         _lib.check(_lib.core().cuna2_adjoint_bootstrap(self._h, t.data_ptr(), y.data_ptr(), out.data_ptr(),
                                                        t.numel(), int(nbs), seed & 0xFFFFFFFF,
-                                                       float(t0), float(T), s or None))
+                                                       float(t0), float(T), s))
         return out
 
     def multi(self, t, Y, t0=None, T=None, out=None, stream=None):
@@ -111,28 +118,27 @@ class AdjointNFFT:
         Y = Y.contiguous()
         if out is None:
             out = torch.empty((Y.shape[0], self.nf), dtype=self.cdtype, device=t.device)
-        s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
+        s = _lib.stream_handle(stream, t.device)
         _lib.check(_lib.core().cuna2_adjoint_multi(self._h, t.data_ptr(), Y.data_ptr(), out.data_ptr(), t.numel(),
-                                                   Y.shape[0], float(t0), float(T), s or None))
+                                                   Y.shape[0], float(t0), float(T), s))
         return out
 
     def backward(self, t, y, grad_F, t0, T, need_y=True, need_t=True, stream=None):
         """(dL/dy, dL/dt) for grad_F = dL/dRe F + i dL/dIm F (torch's convention)."""
         gy = torch.empty_like(y) if need_y else None
         gt = torch.empty_like(t) if need_t else None
-        s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
+        s = _lib.stream_handle(stream, t.device)
         g = grad_F.contiguous()
         if g.dtype != self.cdtype:
             g = g.to(self.cdtype)
         _lib.check(_lib.core().cuna2_adjoint_backward(
             self._h, t.data_ptr(), y.data_ptr(), g.data_ptr(), None if gy is None else gy.data_ptr(),
-            None if gt is None else gt.data_ptr(), t.numel(), float(t0), float(T), s or None))
+            None if gt is None else gt.data_ptr(), t.numel(), float(t0), float(T), s))
         return gy, gt
 
     def backward_batch(self, t, y, grad_F, t0, T, need_y=True, need_t=True, stream=None):
         """(dL/dy, dL/dt) of B series at once: t, y (B, N), grad_F (B, nf),
         t0 and T B values each (cuna2_adjoint_backward_batch)."""
-        import numpy as np
         B = t.shape[0]
         t = t.contiguous()
         y = y.contiguous()
@@ -141,12 +147,11 @@ class AdjointNFFT:
         g = grad_F.contiguous()
         if g.dtype != self.cdtype:
             g = g.to(self.cdtype)
-        t0a = np.ascontiguousarray(np.broadcast_to(np.asarray(t0, np.float64), (B,)))
-        Ta = np.ascontiguousarray(np.broadcast_to(np.asarray(T, np.float64), (B,)))
-        s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
+        t0a, Ta = _per_series(t0, B), _per_series(T, B)
+        s = _lib.stream_handle(stream, t.device)
         _lib.check(_lib.core().cuna2_adjoint_backward_batch(
             self._h, t.data_ptr(), y.data_ptr(), g.data_ptr(), None if gy is None else gy.data_ptr(),
-            None if gt is None else gt.data_ptr(), t.shape[1], B, t0a.ctypes.data, Ta.ctypes.data, s or None))
+            None if gt is None else gt.data_ptr(), t.shape[1], B, t0a.ctypes.data, Ta.ctypes.data, s))
         return gy, gt
 
     def set_graph(self, enable=True):
@@ -183,10 +188,10 @@ class AdjointNFFT:
         (log_tile, grid_method, best_ms)."""
         t, y, t0, T = self._check(t, y, t0, T)
         out = torch.empty(self.nf, dtype=self.cdtype, device=t.device)
-        s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
+        s = _lib.stream_handle(stream, t.device)
         ms = ctypes.c_float()
         _lib.check(_lib.core().cuna2_plan_autotune(self._h, t.data_ptr(), y.data_ptr(), out.data_ptr(), t.numel(),
-                                                   float(t0), float(T), s or None, int(reps), ctypes.byref(ms)))
+                                                   float(t0), float(T), s, int(reps), ctypes.byref(ms)))
         return self.schedule + (ms.value,)
 
     def frequencies(self):
@@ -208,7 +213,6 @@ class BatchAdjointNFFT:
         """The batch plan (R, m, gridding schedule) that reaches relative error
         `tol` fastest on the representative batch (t, y)
         (cuna2_batch_plan_create_auto)."""
-        import numpy as np
         self = cls.__new__(cls)
         self._setup(n, nf, dtype, t.device)
         if t.dtype != torch.float64 or y.dtype != dtype or t.numel() != int(self.n.sum()) or y.numel() != t.numel():
@@ -219,21 +223,20 @@ class BatchAdjointNFFT:
         Ta = None if T is None else np.ascontiguousarray(T, dtype=np.float64)
         out = torch.empty(int(self.nf.sum()), dtype=self.cdtype, device=t.device)
         R, m = np.zeros(ns, np.int32), np.zeros(ns, np.int32)
-        s = torch.cuda.current_stream(t.device).cuda_stream
+        s = _lib.stream_handle(None, t.device)
         self._h = ctypes.c_void_p()
         with torch.cuda.device(self.device):
             _lib.check(_lib.core().cuna2_batch_plan_create_auto(
                 ctypes.byref(self._h), _lib.F32 if dtype == torch.float32 else _lib.F64, ns,
                 self.n.ctypes.data, self.nf.ctypes.data, float(tol),
                 None if t0a is None else t0a.ctypes.data, None if Ta is None else Ta.ctypes.data,
-                t.data_ptr(), y.data_ptr(), out.data_ptr(), s or None, R.ctypes.data, m.ctypes.data))
+                t.data_ptr(), y.data_ptr(), out.data_ptr(), s, R.ctypes.data, m.ctypes.data))
         self.R, self.m = R, m  # per series
         if graph:
             _lib.check(_lib.core().cuna2_batch_set_graph(self._h, 1))
         return self
 
     def _setup(self, n, nf, dtype, device):
-        import numpy as np
         self.n = np.ascontiguousarray(n, dtype=np.int64)
         self.nf = np.ascontiguousarray(nf, dtype=np.int64)
         if self.n.shape != self.nf.shape or self.n.ndim != 1:
@@ -243,10 +246,10 @@ class BatchAdjointNFFT:
         self.device = torch.device(device) if device is not None else torch.device("cuda", torch.cuda.current_device())
         self.f_off = np.concatenate([[0], np.cumsum(self.nf)])
         self.s_off = np.concatenate([[0], np.cumsum(self.n)])
+        self._n_total, self._nf_total = int(self.s_off[-1]), int(self.f_off[-1])
 
     def __init__(self, n, nf, R=2, m=8, t0=None, T=None, dtype=torch.float32, device=None, graph=False):
         """R and m: one value for every series, or one per series."""
-        import numpy as np
         self._setup(n, nf, dtype, device)
         ns = len(self.n)
         self.R = np.ascontiguousarray(np.broadcast_to(np.asarray(R), (ns,)), dtype=np.int32)
@@ -272,7 +275,6 @@ class BatchAdjointNFFT:
             self._h = ctypes.c_void_p()
 
     def set_times(self, t0, T):
-        import numpy as np
         t0a = np.ascontiguousarray(t0, dtype=np.float64)
         Ta = np.ascontiguousarray(T, dtype=np.float64)
         _lib.check(_lib.core().cuna2_batch_set_times(self._h, t0a.ctypes.data, Ta.ctypes.data))
@@ -280,14 +282,14 @@ class BatchAdjointNFFT:
     def __call__(self, t, y, out=None, stream=None):
         if t.dtype != torch.float64 or y.dtype != self.dtype or not (t.is_cuda and y.is_cuda):
             raise TypeError("t must be float64 and y %s CUDA tensors" % self.dtype)
-        if t.numel() != int(self.s_off[-1]) or y.numel() != t.numel():
+        if t.numel() != self._n_total or y.numel() != t.numel():
             raise ValueError("t and y must hold sum(n) samples")
         t = t.contiguous()
         y = y.contiguous()
         if out is None:
-            out = torch.empty(int(self.f_off[-1]), dtype=self.cdtype, device=t.device)
-        s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
-        _lib.check(_lib.core().cuna2_batch_adjoint(self._h, t.data_ptr(), y.data_ptr(), out.data_ptr(), s or None))
+            out = torch.empty(self._nf_total, dtype=self.cdtype, device=t.device)
+        s = _lib.stream_handle(stream, t.device)
+        _lib.check(_lib.core().cuna2_batch_adjoint(self._h, t.data_ptr(), y.data_ptr(), out.data_ptr(), s))
         return out
 
     def split(self, F):
@@ -307,8 +309,8 @@ class BatchAdjointNFFT:
         """Time every admissible schedule on (t, y), keep the fastest;
         returns (log_tile, grid_method, best_ms)."""
         out = torch.empty(int(self.f_off[-1]), dtype=self.cdtype, device=t.device)
-        s = (stream if stream is not None else torch.cuda.current_stream(t.device)).cuda_stream
+        s = _lib.stream_handle(stream, t.device)
         ms = ctypes.c_float()
         _lib.check(_lib.core().cuna2_batch_autotune(self._h, t.contiguous().data_ptr(), y.contiguous().data_ptr(),
-                                                    out.data_ptr(), s or None, int(reps), ctypes.byref(ms)))
+                                                    out.data_ptr(), s, int(reps), ctypes.byref(ms)))
         return self.schedule + (ms.value,)
