@@ -239,7 +239,7 @@ template <typename T>
 int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>::type *F, int64_t n,
                 double t0, double T_, cudaStream_t st, Prof *pr = nullptr, int nbs = 0, unsigned seed = 0,
                 const T *multi = nullptr, int nmulti = 0, const BinOut *bo = nullptr,
-                const GridRepeat *grep = nullptr) {
+                const GridRepeat *grep = nullptr, const MultiValues *hook = nullptr) {
   typedef typename CxOf<T>::type C;
   typedef typename RecOf<T>::type Rec;
   if (n < 0 || (n > 0 && (!t || !y)) || (!F && !bo) || !(T_ > 0) || !std::isfinite(T_) || !std::isfinite(t0))
@@ -274,8 +274,10 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     }
   }
   const bool seg = nch > 0;
+  // short series: the whole sort in one launch
+  const bool one = !small && !seg && n > 0 && n <= kBinOneN && ntiles <= kScanFuseTiles;
   // reserved two-pass binning: CTAs of rspan samples, a table of nrb x ntiles
-  const bool resv = !small && !seg && n > 0 && ntiles <= kScanFuseTiles;
+  const bool resv = !small && !seg && !one && n > 0 && ntiles <= kScanFuseTiles;
   const int64_t rspan = resv ? resv_span(n, ntiles, nsm) : 0;
   const int nrb = resv ? (int)((n + rspan - 1) / rspan) : 0;
   // workspace: counts | cursor | offsets | phases or chunk table | reservations
@@ -288,7 +290,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   const size_t o_cnt = 0, o_cur = align_up(sizeof(int) * ntiles), o_off = 2 * o_cur;
   const size_t o_hdr = o_off + align_up(sizeof(int) * (ntiles + 1));
   const size_t nrec = seg ? 2 * ((size_t)n + CH) : 2 * (size_t)(n > 0 ? n : 1);
-  const size_t phs_b = small ? 0
+  const size_t phs_b = small || one ? 0
                              : (seg ? align_up(sizeof(int) * (size_t)ntiles * nch)
                                     : align_up(sizeof(uint64_t) * (size_t)(n > 0 ? n : 1)));
   const size_t rsv_b = resv ? align_up(sizeof(int) * (size_t)nrb * ntiles) : 0;
@@ -314,6 +316,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   if (bo && (small || seg))
     return fail(CUNA2_ERROR_UNSUPPORTED, "record inspection needs a tiled plan with the global binning form");
   mark(pr, "start", st);
+  if (hook && !one) CUNA_TRY(hook->fn(hook->ctx, false));
   if (nbs > 0) {
     static SetupFlag attrw;
     if (!setup_done(&attrw)) {
@@ -345,6 +348,18 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     k_bin_local<<<nch, 512, sizeof(int) * (2 * ntiles + 1), st>>>(smp, recs, loc, ntiles, nch, CH);
     CUNA_CK(cudaGetLastError());
     mark(pr, "bin_local", st);
+  } else if (one) {
+    SampAcc<T> smp{t, y, n, pm, e};
+    static SetupFlag attr1;
+    if (!setup_done(&attr1)) {
+      CUNA_CK(cudaFuncSetAttribute(k_bin_one<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)bin_one_smem(kBinOneN, kScanFuseTiles)));
+      mark_setup_done(&attr1);
+    }
+    k_bin_one<T><<<kBinOneCtas, kBinOneThreads, bin_one_smem(n, ntiles), st>>>(smp, offsets, recs, ntiles);
+    CUNA_CK(cudaGetLastError());
+    mark(pr, "bin_one", st);
+    if (hook) CUNA_TRY(hook->fn(hook->ctx, true));
   } else {
   // counts and cursor are adjacent: one memset zeroes both
   CUNA_CK(cudaMemsetAsync(counts, 0, o_off, st));
@@ -1144,6 +1159,18 @@ extern "C" int cuna2_adjoint_multi(cuna2_plan p, const double *t, const void *y,
   return adjoint_run<double>(p, t, (const double *)y, (double2 *)F, n, t0, T, st, nullptr, 0, 0,
                              (const double *)y, nchan);
 }
+
+namespace cuna {
+int adjoint_multi_values(cuna2_plan p, const double *t, const void *y, void *F, int64_t n, int nchan, double t0, double T,
+                         const MultiValues &values, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(p->mu);
+  if (p->dtype == CUNA2_F32)
+    return adjoint_run<float>(p, t, (const float *)y, (float2 *)F, n, t0, T, st, nullptr, 0, 0, (const float *)y, nchan,
+                              nullptr, nullptr, &values);
+  return adjoint_run<double>(p, t, (const double *)y, (double2 *)F, n, t0, T, st, nullptr, 0, 0, (const double *)y, nchan,
+                             nullptr, nullptr, &values);
+}
+}  // namespace cuna
 
 // ---------------------------------------------------------------------------
 // Integer steps read back (tests and diagnostics; the transforms never call

@@ -96,4 +96,16 @@ bool fp64_passes_forced();
 bool encode_tmap_f32_3d(void *map, const void *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
                         uint64_t s2, uint32_t b0, uint32_t b1);
 
+// cuna2_adjoint_multi whose channels y (nchan x n, device memory) the caller
+// computes on the stream: values.fn launches that work, between the binning,
+// which reads the times only, and the gridding.  `after`: a binning kernel
+// precedes it in the stream; the work may run beside it (dependent launch), but
+// its last kernel must not complete before it.
+struct MultiValues {
+  int (*fn)(void *ctx, bool after);
+  void *ctx;
+};
+int adjoint_multi_values(cuna2_plan p, const double *t, const void *y, void *F, int64_t n, int nchan, double t0,
+                         double T, const MultiValues &values, cudaStream_t st);
+
 }  // namespace cuna

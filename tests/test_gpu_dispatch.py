@@ -132,3 +132,44 @@ def test_float_float_passes_lengths(mods, nf, R, m):
     ks = np.concatenate([[-nf // 2, -nf // 2 + 1, -1, 0, 1, nf // 2 - 1], rng.integers(-nf // 2, nf // 2, 194)])
     D = _sums_extended(t, y, 50.0, ks).astype(np.complex128)
     assert rel_l2(F[ks + nf // 2], D) < 1e-11 + 10 * np.exp(-np.pi * m * np.sqrt(1 - 1 / R))
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-6), (torch.float64, 1e-11)])
+@pytest.mark.parametrize("n", [1, 8, 511, 2049, 16384, 16385])
+def test_binning_in_one_launch(mods, oracle_lib, dtype, tol, n):
+    """Short series binned by one cluster launch (up to 16384 samples) and the
+    next size above it, with samples on tile edges and the grid's seam, against
+    the oracle's double restatement (float: rounding of 2m n terms; double: the
+    restatement's phase rounding, 2 pi 2^13 1e-16 per sample)."""
+    _, nfft = mods
+    rng = np.random.default_rng(n)
+    nf, R, m, T = 1 << 14, 2, 8, 5.0
+    t = np.sort(rng.uniform(0, T, n))
+    edges = np.array([0.0, 2048.0, 4096.0, 2047.99, 32767.99]) / (R * nf) * T
+    t[:min(n, 5)] = edges[:min(n, 5)]
+    y = rng.normal(0, 1, n)
+    plan = nfft.AdjointNFFT(nf, R, m, dtype)
+    F = plan(torch.as_tensor(t, device="cuda"), torch.as_tensor(y, dtype=dtype, device="cuda"), 0.0, T).cpu().numpy()
+    ys = y.astype(np.float32).astype(np.float64) if dtype == torch.float32 else y
+    assert rel_l2(F, oracle_lib.accurate_adjoint(t, ys, 0.0, T, nf, R, m)) < tol
+
+
+@pytest.mark.parametrize("scale", [1e-30, 1.0, 1e18])
+@pytest.mark.parametrize("n,nfreq", [(65, 700), (20000, 5000)])
+def test_lomb_scargle_scales(mods, scale, n, nfreq):
+    """The float periodogram does not depend on the data's scale: sums beside the
+    one-launch binning and after the two-launch one, one and many partial sums,
+    against the double plan on the same float values.  Weighted sums of the
+    float plan carry a few 1e-7, amplified where CC SS - CS^2 is small: 1e-4, the
+    bound of the float periodogram against direct sums."""
+    from cunfft_adjoint_gb300.lombscargle import lomb_scargle
+    rng = np.random.default_rng(n)
+    t = np.sort(rng.uniform(0, 100.0, n))
+    y = np.sin(2 * np.pi * t / 2.1) + rng.normal(0, 1, n)
+    dy = rng.uniform(0.2, 0.6, n)
+    td = torch.as_tensor(t, device="cuda")
+    y32 = torch.as_tensor((y * scale).astype(np.float32), device="cuda")
+    dy32 = torch.as_tensor(dy.astype(np.float32), device="cuda")
+    P = lomb_scargle(td, y32, dy32, nfreq=nfreq, df=1 / 500.0, t0=0.0)
+    D = lomb_scargle(td, y32.double() / scale, dy32.double(), nfreq=nfreq, df=1 / 500.0, t0=0.0, R=4, m=12)
+    assert rel_l2(P.cpu().numpy(), D.cpu().numpy()) < 1e-4
