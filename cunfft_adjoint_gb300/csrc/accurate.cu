@@ -428,7 +428,9 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     CUNA_CK(cudaFuncSetAttribute(k_grid_acc<T, 8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     CUNA_CK(cudaFuncSetAttribute(k_grid_acc_sg4<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     CUNA_CK(cudaFuncSetAttribute(k_grid_acc_sg4<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    CUNA_CK(cudaFuncSetAttribute(k_grid_fixed<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    CUNA_CK(cudaFuncSetAttribute(k_grid_fixed<T, kGridThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    if constexpr (sizeof(T) == 8)
+      CUNA_CK(cudaFuncSetAttribute(k_grid_fixed<T, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     CUNA_CK(cudaFuncSetAttribute(k_grid_scatter<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     CUNA_CK(cudaFuncSetAttribute(k_grid_acc_seg<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     CUNA_CK(cudaFuncSetAttribute(k_grid_acc_seg<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
@@ -442,6 +444,10 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   else smg = grid_scatter_smem_bytes<T>(p->logTL);
   smg = (smg + 15) & ~(size_t)15;
   const dim3 gb(kGridThreads);
+  // double plans: float-float passes, which the fixed-point form feeds with
+  // float-float cells
+  const bool df = sizeof(T) == 8 && p->has_df && !fp64_passes_forced();
+  const bool dfgrid = df && !seg && p->grid_method == CUNA2_GRID_FIXED;
   auto launch_grid = [&]() -> int {
     if (seg) {
       const size_t sm = smg + segb;
@@ -475,7 +481,16 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
           le = launch_pdl(k_grid_acc<T, 4, false>, ggrid, gb, smg, st, rc, oc, grid, e, wc, nv, nslab, group, sstr);
         else le = launch_pdl(k_grid_acc<T, 4>, ggrid, gb, smg, st, rc, oc, grid, e, wc, nv, nslab, group, sstr);
       } else if (p->grid_method == CUNA2_GRID_FIXED) {
-        le = launch_pdl(k_grid_fixed<T>, ggrid, gb, smg, st, rc, oc, grid, e, wc, nv, nslab, group, sstr);
+        bool few = false;
+        if constexpr (sizeof(T) == 8) {
+          few = (int64_t)ggrid.x * ggrid.y < 2 * nsm;
+          if (few)
+            le = launch_pdl(k_grid_fixed<T, 1024>, ggrid, dim3(1024), grid_fixed_smem_bytes<T, 1024>(p->logTL, p->m), st,
+                            rc, oc, grid, e, wc, nv, nslab, group, sstr, dfgrid);
+        }
+        if (!few)
+          le = launch_pdl(k_grid_fixed<T, kGridThreads>, ggrid, gb, smg, st, rc, oc, grid, e, wc, nv, nslab, group, sstr,
+                          dfgrid);
       } else {
         le = launch_pdl(k_grid_scatter<T>, ggrid, gb, smg, st, rc, oc, grid, e, wc, nv, nslab, group, sstr);
       }
@@ -500,9 +515,9 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
       // double plans compute both passes in float-float (the FP32 pipe); the
       // grid and the spectrum are double, the values between the passes
       // float-float in the grid's memory
-      if (p->has_df && !fp64_passes_forced()) {
+      if (df) {
         const FftDev<dfl> fd = to_dev<dfl>(p->geom_df);
-        CUNA_TRY(df_colpass(z, fd, nslab, st));
+        CUNA_TRY(df_colpass(z, fd, nslab, dfgrid, st));
         mark(pr, "fft_colpass", st);
         CUNA_TRY(df_rowpass(z, fd, e, F, nslab, st));
         mark(pr, "fft_rowpass", st);

@@ -970,12 +970,13 @@ __global__ void __launch_bounds__(kGridThreads, sizeof(T) == 4 ? 6 : 3) k_grid_s
 // is bit-reproducible run to run.  A non-finite value makes its tiles NaN.
 // records [c0, c0 + cnt) -> srec (values from ws when given); returns the
 // thread's max |value| (NaN once one is not finite)
-template <typename T, class Src>
+template <typename T, int NT> __host__ __device__ constexpr int fixed_cap() { return GridCfg<T>::CAP > NT ? GridCfg<T>::CAP : NT; }
+template <typename T, int NT, class Src>
 __device__ __forceinline__ float fixed_stage(const Src &recs, int c0, int cnt,
                                             int base, const T *__restrict__ ws, SRec<T> *srec) {
   float ym = 0.f;
 #pragma unroll 1
-  for (int i = threadIdx.x; i < cnt; i += kGridThreads) {
+  for (int i = threadIdx.x; i < cnt; i += NT) {
     const typename RecOf<T>::type rc = recs[c0 + i];
     SRec<T> r;
     r.f = rc.a;
@@ -990,10 +991,10 @@ __device__ __forceinline__ float fixed_stage(const Src &recs, int c0, int cnt,
 
 // clear a fixed-point tile of TL cells (TL a multiple of 4, acc 16-byte
 // aligned) with 16-byte stores
-template <typename A> __device__ __forceinline__ void fixed_clear(A *acc, int TL) {
+template <int NT, typename A> __device__ __forceinline__ void fixed_clear(A *acc, int TL) {
   int4 *v = reinterpret_cast<int4 *>(acc);
   const int nv = TL * (int)sizeof(A) / 16;
-  for (int i = threadIdx.x; i < nv; i += kGridThreads) v[i] = make_int4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < nv; i += NT) v[i] = make_int4(0, 0, 0, 0);
 }
 // cells [i, i + 4) of a fixed-point tile as values: 16-byte shared loads
 __device__ __forceinline__ void fixed_load4(const int *acc, int i, float inv, float &a, float &b, float &c,
@@ -1025,18 +1026,19 @@ __device__ __forceinline__ void fixed_load4(const long long *acc, int i, double 
 // The integer sums, hence the grid's bits, equal the int64 form's.
 constexpr int kSplitBits = 20;
 constexpr int kSplitMaxH = 2048;
-template <typename T> struct FixAdd {  // one atomic in the tile's own type
-  typename FixAcc<T>::type *acc;
-  __device__ __forceinline__ void operator()(int c, typename FixAcc<T>::type v) const {
-    FixAcc<T>::add(acc + c, v);
-  }
-};
 struct SplitAdd {
   int *hi;
   unsigned *lo;
-  __device__ __forceinline__ void operator()(int c, long long v) const {
-    atomicAdd(lo + c, (unsigned)v & ((1u << kSplitBits) - 1u));
-    atomicAdd(hi + c, (int)(v >> kSplitBits));
+  // the integer h 2^20 + l
+  __device__ __forceinline__ void operator()(int c, int h, int l) const {
+    atomicAdd(lo + c, (unsigned)l & ((1u << kSplitBits) - 1u));
+    atomicAdd(hi + c, h + (l >> kSplitBits));
+  }
+};
+struct WideAdd {  // one 64-bit atomic
+  long long *acc;
+  __device__ __forceinline__ void operator()(int c, int h, int l) const {
+    FixAcc<double>::add(acc + c, ((long long)h << kSplitBits) + l);
   }
 };
 // cells [i, i + 4) of a split tile as values: 16-byte shared loads
@@ -1051,97 +1053,121 @@ __device__ __forceinline__ void fixed_load4_split(const int *hi, const unsigned 
   d = (double)((long long)h.w * U + l.w) * inv;
 }
 
-// Tap arithmetic of the fixed-point form: float plans in float; double plans
-// in float-float on the FP32 pipe (about 48 bits, below the 2^-50 quantum's
-// reach only where a tap is far below its tile's bound), the per-record
-// factors E, Q, 1/Q and the 2m coefficients formed in double first.
-template <typename T> struct TapOf { typedef T type; };
-template <> struct TapOf<double> { typedef dfl type; };
-__device__ __forceinline__ float tap_from(float v) { return v; }
-__device__ __forceinline__ dfl tap_from(double v) { return df_from_double(v); }
-__device__ __forceinline__ int tap_fix(float w) { return FixAcc<float>::to_fix(w); }
-// round(hi + lo) for |hi + lo| <= 2^50, from the bit fields of hi: at or
-// above 2^23 hi is an integer (its 24-bit significand shifted left) and lo,
-// below half its ulp, rounds on its own; below 2^23 the float sum rounds.
-__device__ __forceinline__ long long tap_fix(dfl w) {
-  if (fabsf(w.hi) >= 8388608.0f) {
-    const int b = __float_as_int(w.hi);
-    const int sh = ((b >> 23) & 0xff) - 150;
-    const long long mag = (long long)((b & 0x7fffff) | 0x800000) << sh;
-    return (b < 0 ? -mag : mag) + (long long)__float2int_rn(w.lo);
-  }
-  return (long long)__float2int_rn(w.hi + w.lo);
-}
+// A double plan's coefficients exp2(-k1 d^2), d = 0..m, in shared memory: the
+// float-float value with each half twice (hi, hi, lo, lo), the packed operand.
+constexpr int kTapCoefBytes = 17 * 16 > 32 * 4 ? 17 * 16 : 32 * 4;
 
-// all 2m taps of the staged records srec[0, cnt) into the tile through add
-// (add(c, v): integer v into local cell c), scaled by sc; cd holds the
-// coefficients exp2(-k1 d^2) in the tap arithmetic's type
-template <typename T, class Add>
-__device__ __forceinline__ void fixed_taps(const SRec<T> *srec, int cnt, T sc, const AccParams<T> &e,
-                                           const T *cd, const Add &add, int TL, int gmask) {
-  typedef typename TapOf<T>::type W;
-  const W *cw = reinterpret_cast<const W *>(cd);
+// All 2m taps of the staged records srec[0, cnt) into the tile as integers
+// scaled by sc.  Float: float products, one conversion and one atomic per tap;
+// cd holds exp2(-k1 d^2), d = -m+1..m.
+__device__ __forceinline__ void fixed_taps(const SRec<float> *srec, int cnt, float sc, const AccParams<float> &e,
+                                           const float *cd, int *acc, int TL, int gmask, int nthr) {
   const int m = e.m;
-  W k1w, k2w;  // the exponent constants in the tap arithmetic
-  if constexpr (sizeof(T) == 8) {
-    k1w = df_from_double(e.k1);
-    k2w = df_from_double(e.k2);
-  }
 #pragma unroll 1
-  for (int i = threadIdx.x; i < cnt; i += kGridThreads) {
-    const SRec<T> q = srec[i];
-    W Ew, Qw, Qiw;
-    if constexpr (sizeof(T) == 8) {
-      // E = y sc 2^(-k1 f^2), Q = 2^(k2 f), 1/Q in float-float: only the two
-      // conversions from double use the FP64 pipe
-      const dfl fw = df_from_double(q.f);
-      Ew = df_from_double(q.y * sc) * df_exp2(-(k1w * fw * fw));
-      Qw = df_exp2(k2w * fw);
-      Qiw = df_rcp(Qw);
-    } else {
-      Ew = q.y * sc * exp2_g(-e.k1 * q.f * q.f);
-      Qw = exp2_g(e.k2 * q.f);
-      Qiw = exp2_g(-e.k2 * q.f);
-    }
+  for (int i = threadIdx.x; i < cnt; i += nthr) {
+    const SRec<float> q = srec[i];
+    const float E = q.y * sc * exp2_g(-e.k1 * q.f * q.f);
+    const float Q = exp2_g(e.k2 * q.f), Qi = exp2_g(-e.k2 * q.f);
     const int p0 = q.lc;
     if (p0 - m + 1 >= 0 && p0 + m < TL) {  // every tap inside the tile
-      W u = Ew;
+      float u = E;
 #pragma unroll 4
       for (int d = 0; d <= m; ++d) {  // taps right of the cell, Q^d
-        add(p0 + d, tap_fix(u * cw[d + m - 1]));
-        u = u * Qw;
+        FixAcc<float>::add(acc + p0 + d, FixAcc<float>::to_fix(u * cd[d + m - 1]));
+        u = u * Q;
       }
-      u = Ew * Qiw;
+      u = E * Qi;
 #pragma unroll 4
       for (int d = -1; d > -m; --d) {  // taps left of the cell
-        add(p0 + d, tap_fix(u * cw[d + m - 1]));
-        u = u * Qiw;
+        FixAcc<float>::add(acc + p0 + d, FixAcc<float>::to_fix(u * cd[d + m - 1]));
+        u = u * Qi;
       }
     } else {  // near the tile edge: wrap, keep the taps inside the tile
-      W u = Ew;
+      float u = E;
       for (int d = 0; d <= m; ++d) {
         const int lc = (p0 + d) & gmask;
-        if (lc < TL) add(lc, tap_fix(u * cw[d + m - 1]));
-        u = u * Qw;
+        if (lc < TL) FixAcc<float>::add(acc + lc, FixAcc<float>::to_fix(u * cd[d + m - 1]));
+        u = u * Q;
       }
-      u = Ew * Qiw;
+      u = E * Qi;
       for (int d = -1; d > -m; --d) {
         const int lc = (p0 + d) & gmask;
-        if (lc < TL) add(lc, tap_fix(u * cw[d + m - 1]));
-        u = u * Qiw;
+        if (lc < TL) FixAcc<float>::add(acc + lc, FixAcc<float>::to_fix(u * cd[d + m - 1]));
+        u = u * Qi;
       }
+    }
+  }
+}
+
+// a tap p + e (|p| <= 2^50, e its rounding remainder) as the integer nearest it,
+// h 2^20 + l: h from p alone (exact: p has 24 bits, so either p / 2^20 is an
+// integer or its nearest integer is below 2^24), l from what is left
+__device__ __forceinline__ void tap_fix(float p, float e, int &h, int &l) {
+  h = __float2int_rn(p * 0x1p-20f);
+  l = __float2int_rn(fmaf((float)h, -0x1p20f, p) + e);
+}
+
+// Double: the taps d = k and d = -k of a record as one packed pair in
+// float-float (about 48 bits, below the 2^-50 quantum's reach only where a tap
+// is far below its tile's bound), E Q^k and E Q^-k by running products with the
+// shared coefficient c_k; only the two conversions from double use the FP64
+// pipe.  13 packed operations per pair of taps and 9 scalar ones per tap to
+// split it into the two words, where scalar products and a 64-bit integer took
+// 60 per tap (1e6 samples on 2^22 cells: 120 -> 80 us, flushing float-float
+// cells included).
+template <class Add>
+__device__ __forceinline__ void fixed_taps_df(const SRec<double> *srec, int cnt, double sc, const AccParams<double> &e,
+                                              const ulonglong2 *cw, const Add &add, int TL, int gmask, int nthr) {
+  const int m = e.m;
+  const dfl k1w = df_from_double(e.k1), k2w = df_from_double(e.k2);  // the exponent constants
+  const f2 m1 = pk2(-1.0f, -1.0f);
+  auto tap = [&](int c, float p, float r) {
+    c &= gmask;
+    if (c < TL) {
+      int h, l;
+      tap_fix(p, r, h, l);
+      add(c, h, l);
+    }
+  };
+#pragma unroll 1
+  for (int i = threadIdx.x; i < cnt; i += nthr) {
+    const SRec<double> q = srec[i];
+    const dfl fw = df_from_double(q.f);
+    // E = y sc 2^(-k1 f^2), Q = 2^(k2 f), 1/Q
+    const dfl E = df_from_double(q.y * sc) * df_exp2(-(k1w * fw * fw));
+    const dfl Q = df_exp2(k2w * fw), Qi = df_rcp(Q);
+    const int p0 = q.lc;
+    tap(p0, E.hi, E.lo);
+    const f2 Qh = pk2(Q.hi, Qi.hi), Ql = pk2(Q.lo, Qi.lo), nQh = mul2(Qh, m1);
+    f2 Uh = pk2(E.hi, E.hi), Ul = pk2(E.lo, E.lo);
+#pragma unroll 2
+    for (int k = 1; k <= m; ++k) {
+      {  // U <- U Q: float-float product, renormalised
+        const f2 p = mul2(Uh, Qh), w = fma2(Uh, nQh, p);
+        const f2 r = sub2(fma2(Ul, Qh, mul2(Uh, Ql)), w);
+        Uh = add2(p, r);
+        Ul = sub2(r, sub2(Uh, p));
+      }
+      const ulonglong2 c = cw[k];
+      const f2 p = mul2(Uh, c.x);
+      const f2 r = fma2(Ul, c.x, fma2(Uh, c.y, fma2(Uh, c.x, mul2(p, m1))));
+      float ph, pl, rh, rl;
+      unpk2(p, ph, pl);
+      unpk2(r, rh, rl);
+      tap(p0 + k, ph, rh);
+      if (k < m) tap(p0 - k, pl, rl);
     }
   }
 }
 
 // the tile's fixed-point scale from the per-warp maxima of |value| (NaN once
 // one was not finite) and the largest bucket count hmax
-template <typename T>
+template <typename T, int NT>
 __device__ __forceinline__ T fixed_scale(const float *red, int hmax) {
   float y = 0.f;
   bool bad = false;
 #pragma unroll
-  for (int w = 0; w < kGridThreads / 32; ++w) {
+  for (int w = 0; w < NT / 32; ++w) {
     bad |= isnan(red[w]);
     y = fmaxf(y, red[w]);
   }
@@ -1153,28 +1179,79 @@ __device__ __forceinline__ T fixed_scale(const float *red, int hmax) {
 }
 
 // the taps of srec[0, cnt) into the tile, in split form when asked (double)
-template <typename T>
+template <typename T, int NT>
 __device__ __forceinline__ void tile_taps(bool split, const SRec<T> *srec, int cnt, T sc, const AccParams<T> &e,
-                                          const T *cd, typename FixAcc<T>::type *acc, int TL, int gmask) {
+                                          const void *cd, typename FixAcc<T>::type *acc, int TL, int gmask) {
   if constexpr (sizeof(T) == 8) {
-    if (split) {
-      const SplitAdd add{reinterpret_cast<int *>(acc), reinterpret_cast<unsigned *>(acc) + TL};
-      fixed_taps<T>(srec, cnt, sc, e, cd, add, TL, gmask);
-      return;
-    }
+    const ulonglong2 *cw = static_cast<const ulonglong2 *>(cd);
+    if (split)
+      fixed_taps_df(srec, cnt, sc, e, cw, SplitAdd{reinterpret_cast<int *>(acc), reinterpret_cast<unsigned *>(acc) + TL},
+                    TL, gmask, NT);
+    else fixed_taps_df(srec, cnt, sc, e, cw, WideAdd{acc}, TL, gmask, NT);
+  } else {
+    fixed_taps(srec, cnt, sc, e, static_cast<const float *>(cd), acc, TL, gmask, NT);
   }
-  fixed_taps<T>(srec, cnt, sc, e, cd, FixAdd<T>{acc}, TL, gmask);
+}
+
+// Two cells h 2^20 + l (l < 2^32) times inv as one float-float complex value:
+// each integer as three exact floats (h rounded to 24 bits; the remainder with
+// l's high half; l's low half) added up, the product renormalised.
+__device__ __forceinline__ dcx fixed_pair_df(int h0, unsigned l0, int h1, unsigned l1, dfl inv) {
+  const float f0 = (float)h0, f1 = (float)h1;
+  const int r0 = h0 - (int)f0, r1 = h1 - (int)f1;  // |r| <= 64
+  const f2 a = mul2(pk2(f0, f1), pk2(0x1p20f, 0x1p20f));
+  const f2 b = mul2(pk2((float)(r0 * 16 + (int)(l0 >> 16)), (float)(r1 * 16 + (int)(l1 >> 16))), pk2(0x1p16f, 0x1p16f));
+  const f2 c = pk2((float)(l0 & 0xffffu), (float)(l1 & 0xffffu));
+  const f2 s = add2(a, b), v = sub2(s, a);
+  const f2 e = add2(add2(sub2(a, sub2(s, v)), sub2(b, v)), c);
+  const f2 xh = add2(s, e), xl = sub2(e, sub2(xh, s));
+  const f2 ih = pk2(inv.hi, inv.hi), p = mul2(xh, ih);
+  const f2 r = sub2(fma2(xl, ih, mul2(xh, pk2(inv.lo, inv.lo))), fma2(xh, pk2(-inv.hi, -inv.hi), p));
+  dcx o;
+  o.h = add2(p, r);
+  o.l = sub2(r, sub2(o.h, p));
+  return o;
+}
+
+// the tile into the grid as float-float (pairs of cells are the complex points
+// of the FFT), for the float-float passes: integer and FP32 operations only,
+// where the double cells cost two FP64-pipe operations each here and as many
+// conversions in the column pass
+template <int NT>
+__device__ __forceinline__ void tile_flush_df(bool split, const long long *acc, int TL, double inv, double *out) {
+  const dfl iv(inv);
+  ulonglong2 *o = reinterpret_cast<ulonglong2 *>(out);
+  const int *hi = reinterpret_cast<const int *>(acc);
+  const unsigned *lo = reinterpret_cast<const unsigned *>(acc) + TL;
+  for (int i = 2 * threadIdx.x; i < TL; i += 2 * NT) {
+    int2 h;
+    uint2 l;
+    if (split) {
+      h = *reinterpret_cast<const int2 *>(hi + i);
+      l = *reinterpret_cast<const uint2 *>(lo + i);
+    } else {
+      const longlong2 v = *reinterpret_cast<const longlong2 *>(acc + i);
+      h = make_int2((int)(v.x >> kSplitBits), (int)(v.y >> kSplitBits));
+      l = make_uint2((unsigned)v.x & ((1u << kSplitBits) - 1u), (unsigned)v.y & ((1u << kSplitBits) - 1u));
+    }
+    const dcx w = fixed_pair_df(h.x, l.x, h.y, l.y, iv);
+    o[i >> 1] = make_ulonglong2(w.h, w.l);
+  }
 }
 
 // fixed-order flush of the tile: out[i] = cell i * inv (inv = 1 / scale)
-template <typename T>
-__device__ __forceinline__ void tile_flush(bool split, const typename FixAcc<T>::type *acc, int TL, T inv,
-                                           T *__restrict__ out) {
+template <typename T, int NT>
+__device__ __forceinline__ void tile_flush(bool split, const typename FixAcc<T>::type *acc, int TL, T inv, T *out,
+                                           bool dfout) {
   if constexpr (sizeof(T) == 8) {
+    if (dfout) {
+      tile_flush_df<NT>(split, acc, TL, inv, out);
+      return;
+    }
     if (split) {
       const int *hi = reinterpret_cast<const int *>(acc);
       const unsigned *lo = reinterpret_cast<const unsigned *>(acc) + TL;
-      for (int i = 4 * threadIdx.x; i < TL; i += 4 * kGridThreads) {
+      for (int i = 4 * threadIdx.x; i < TL; i += 4 * NT) {
         T a, b, c, d;
         fixed_load4_split(hi, lo, i, inv, a, b, c, d);
         store4(out + i, a, b, c, d);
@@ -1182,24 +1259,25 @@ __device__ __forceinline__ void tile_flush(bool split, const typename FixAcc<T>:
       return;
     }
   }
-  for (int i = 4 * threadIdx.x; i < TL; i += 4 * kGridThreads) {
+  for (int i = 4 * threadIdx.x; i < TL; i += 4 * NT) {
     T a, b, c, d;
     fixed_load4(acc, i, inv, a, b, c, d);
     store4(out + i, a, b, c, d);
   }
 }
 
-template <typename T, class Src>
+// NT threads; dfout (double): cells written in float-float
+template <typename T, class Src, int NT = kGridThreads>
 __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
                                                 int base, T *__restrict__ grid, const AccParams<T> &e,
                                                 const T *__restrict__ wts, int64_t nvals, int sbeg, int send,
-                                                int64_t slab_stride) {
+                                                int64_t slab_stride, bool dfout = false) {
   typedef FixAcc<T> FA;
   typedef typename FA::type A;
-  constexpr int CAP = GridCfg<T>::CAP;
+  constexpr int CAP = fixed_cap<T, NT>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ float red[kGridThreads / 32];
-  __shared__ int redi[kGridThreads / 32];
+  __shared__ float red[NT / 32];
+  __shared__ int redi[NT / 32];
   __shared__ T scale_s;
   const int TL = 1 << e.logTL, m = e.m;
   const int gmask = (int)e.ng - 1;
@@ -1208,35 +1286,43 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
   const int NB = ((TL + 2 * m) >> logBS) + 1;
   A *acc = reinterpret_cast<A *>(smem_raw);                                  // TL cells
   SRec<T> *srec = reinterpret_cast<SRec<T> *>(smem_raw + sizeof(A) * TL);    // CAP staged records
-  T *cd = reinterpret_cast<T *>(srec + CAP);                                 // exp2(-k1 d^2), d = -m+1..m
-  int *hist = reinterpret_cast<int *>(cd + 32);                              // NB buckets
+  // coefficients exp2(-k1 d^2): float d = -m+1..m; double d = 0..m, packed float-float
+  void *cd = srec + CAP;
+  int *hist = reinterpret_cast<int *>(static_cast<char *>(cd) + kTapCoefBytes);  // NB buckets
   const int nchunks = (r1 - r0 + CAP - 1) / CAP;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int d = threadIdx.x; d < 2 * m; d += kGridThreads) {
-    const T dd = (T)(d - m + 1);
-    reinterpret_cast<typename TapOf<T>::type *>(cd)[d] = tap_from(exp2_g(-e.k1 * dd * dd));
+  if constexpr (sizeof(T) == 8) {
+    for (int d = threadIdx.x; d <= m; d += NT) {
+      const dfl c = df_from_double(exp2_g(-e.k1 * (T)(d * d)));
+      static_cast<ulonglong2 *>(cd)[d] = make_ulonglong2(pk2(c.hi, c.hi), pk2(c.lo, c.lo));
+    }
+  } else {
+    for (int d = threadIdx.x; d < 2 * m; d += NT) {
+      const T dd = (T)(d - m + 1);
+      static_cast<T *>(cd)[d] = exp2_g(-e.k1 * dd * dd);
+    }
   }
   // bucket histogram of the tile's records (slab independent); a record of
   // this tile lies in [base - m, base + TL + m) modulo ng
-  for (int b = threadIdx.x; b < NB; b += kGridThreads) hist[b] = 0;
+  for (int b = threadIdx.x; b < NB; b += NT) hist[b] = 0;
   if (!wts && sbeg + 1 == send && nchunks <= 1) {
     // One slab of the records' own values, one staging chunk: a single read
     // of the records stages them, builds the histogram and bounds |value|;
     // the largest bucket count is the largest count an atomic returned.
     // Three barriers per tile instead of six; same scale, same bits.
-    constexpr int PER = CAP / kGridThreads;
+    constexpr int PER = CAP / NT;
     const int cnt = r1 - r0;
-    fixed_clear(acc, TL);
+    fixed_clear<NT>(acc, TL);
     __syncthreads();
     typename RecOf<T>::type rc[PER];
 #pragma unroll
     for (int k = 0; k < PER; ++k)
-      if (threadIdx.x + k * kGridThreads < cnt) rc[k] = recs[r0 + threadIdx.x + k * kGridThreads];
+      if (threadIdx.x + k * NT < cnt) rc[k] = recs[r0 + threadIdx.x + k * NT];
     float ym = 0.f;
     int hm = 0;
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
-      const int i = threadIdx.x + k * kGridThreads;
+      const int i = threadIdx.x + k * NT;
       if (i >= cnt) continue;
       SRec<T> r;
       r.f = rc[k].a;
@@ -1259,38 +1345,38 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
     __syncthreads();
     int hmax = 0;
 #pragma unroll
-    for (int w = 0; w < kGridThreads / 32; ++w) hmax = max(hmax, redi[w]);
-    const T sc = fixed_scale<T>(red, hmax);
+    for (int w = 0; w < NT / 32; ++w) hmax = max(hmax, redi[w]);
+    const T sc = fixed_scale<T, NT>(red, hmax);
     const bool split = sizeof(T) == 8 && hmax <= kSplitMaxH;
-    if (sc > (T)0) tile_taps<T>(split, srec, cnt, sc, e, cd, acc, TL, gmask);
+    if (sc > (T)0) tile_taps<T, NT>(split, srec, cnt, sc, e, cd, acc, TL, gmask);
     __syncthreads();
     const T inv = sc > (T)0 ? (T)1 / sc : (sc == sc ? (T)0 : sc);
-    tile_flush<T>(split, acc, TL, inv, grid + (int64_t)sbeg * slab_stride + base);
+    tile_flush<T, NT>(split, acc, TL, inv, grid + (int64_t)sbeg * slab_stride + base, dfout);
     return;
   }
   __syncthreads();
 #pragma unroll 1
-  for (int i = r0 + threadIdx.x; i < r1; i += kGridThreads)
+  for (int i = r0 + threadIdx.x; i < r1; i += NT)
     atomicAdd(&hist[((recs[i].cell - base + m) & gmask) >> logBS], 1);
   __syncthreads();
   int hmax = 0;
-  for (int b = threadIdx.x; b < NB; b += kGridThreads) hmax = max(hmax, hist[b]);
+  for (int b = threadIdx.x; b < NB; b += NT) hmax = max(hmax, hist[b]);
   for (int o = 16; o > 0; o >>= 1) hmax = max(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
   if (lane == 0) redi[warp] = hmax;
   __syncthreads();
   hmax = 0;
 #pragma unroll
-  for (int w = 0; w < kGridThreads / 32; ++w) hmax = max(hmax, redi[w]);
+  for (int w = 0; w < NT / 32; ++w) hmax = max(hmax, redi[w]);
   const bool split = sizeof(T) == 8 && hmax <= kSplitMaxH;
   for (int slab = sbeg; slab < send; ++slab) {
     const T *ws = wts ? wts + (int64_t)slab * nvals : nullptr;
     float ym = 0.f;
     if (slab > sbeg) __syncthreads();  // the previous slab's flush is done with acc and srec
     if (nchunks == 1) {
-      ym = fixed_stage<T>(recs, r0, r1 - r0, base, ws, srec);
+      ym = fixed_stage<T, NT>(recs, r0, r1 - r0, base, ws, srec);
     } else {  // bound pass over all of the tile's records
 #pragma unroll 1
-      for (int i = r0 + threadIdx.x; i < r1; i += kGridThreads) {
+      for (int i = r0 + threadIdx.x; i < r1; i += NT) {
         const T v = ws ? ws[recs[i].p] : recs[i].b;
         ym = isfinite(v) && !isnan(ym) ? fmaxf(ym, (float)fabs(v)) : __int_as_float(0x7fffffff);
       }
@@ -1300,9 +1386,9 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
       ym = (isnan(u) || isnan(ym)) ? __int_as_float(0x7fffffff) : fmaxf(ym, u);
     }
     if (lane == 0) red[warp] = ym;
-    fixed_clear(acc, TL);
+    fixed_clear<NT>(acc, TL);
     __syncthreads();
-    if (threadIdx.x == 0) scale_s = fixed_scale<T>(red, hmax);
+    if (threadIdx.x == 0) scale_s = fixed_scale<T, NT>(red, hmax);
     __syncthreads();
     const T sc = scale_s;
     for (int ck = 0; ck < nchunks; ++ck) {
@@ -1310,37 +1396,40 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
       const int cnt = min(CAP, r1 - c0);
       if (nchunks > 1) {
         if (ck > 0) __syncthreads();
-        fixed_stage<T>(recs, c0, cnt, base, ws, srec);
+        fixed_stage<T, NT>(recs, c0, cnt, base, ws, srec);
         __syncthreads();
       }
-      if (sc > (T)0) tile_taps<T>(split, srec, cnt, sc, e, cd, acc, TL, gmask);
+      if (sc > (T)0) tile_taps<T, NT>(split, srec, cnt, sc, e, cd, acc, TL, gmask);
     }
     __syncthreads();
     // fixed-order flush: cell = integer / scale
     const T inv = sc > (T)0 ? (T)1 / sc : (sc == sc ? (T)0 : sc);
-    tile_flush<T>(split, acc, TL, inv, grid + (int64_t)slab * slab_stride + base);
+    tile_flush<T, NT>(split, acc, TL, inv, grid + (int64_t)slab * slab_stride + base, dfout);
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kGridThreads, sizeof(T) == 4 ? 6 : 4) k_grid_fixed(
+// NT = 256, or 1024 for double launches that do not give every SM two tiles
+// (one transform of 2^19 cells is 128 tiles of 4096: 54 us with eight warps per
+// SM and scalar taps, 28 us here).
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, NT > 256 ? 1 : (sizeof(T) == 4 ? 6 : 4)) k_grid_fixed(
     const typename RecOf<T>::type *recs, const int *off, T *grid, AccParams<T> e, const T *wts, int64_t nvals,
-    int nslab, int group, int64_t slab_stride) {
+    int nslab, int group, int64_t slab_stride, bool dfout) {
   pdl_trigger();
   pdl_wait();  // records and offsets come from the binning
   const int tile = blockIdx.x;
   const int sbeg = blockIdx.y * group, send = min(nslab, sbeg + group);
   const CgSrc<typename RecOf<T>::type> rp{recs};
-  grid_tile_fixed<T>(rp, __ldcg(off + tile), __ldcg(off + tile + 1), tile << e.logTL, grid, e, wts, nvals, sbeg, send,
-                     slab_stride);
+  grid_tile_fixed<T, CgSrc<typename RecOf<T>::type>, NT>(rp, __ldcg(off + tile), __ldcg(off + tile + 1), tile << e.logTL,
+                                                         grid, e, wts, nvals, sbeg, send, slab_stride, dfout);
 }
 
-template <typename T> size_t grid_fixed_smem_bytes(int logTL, int m) {
+template <typename T, int NT = kGridThreads> size_t grid_fixed_smem_bytes(int logTL, int m) {
   int logBS = 4;
   while ((1 << logBS) < 2 * m) ++logBS;
   const size_t NB = ((((size_t)1 << logTL) + 2 * m) >> logBS) + 1;
-  return sizeof(typename FixAcc<T>::type) * ((size_t)1 << logTL) + sizeof(SRec<T>) * (size_t)GridCfg<T>::CAP +
-         sizeof(T) * 32 + sizeof(int) * NB;
+  return sizeof(typename FixAcc<T>::type) * ((size_t)1 << logTL) + sizeof(SRec<T>) * (size_t)fixed_cap<T, NT>() +
+         kTapCoefBytes + sizeof(int) * NB;
 }
 
 // ---------------------------------------------------------------------------

@@ -111,6 +111,34 @@ __device__ __forceinline__ dfl df_rcp(dfl a) {
   const dfl e = dfl(1.0f, 0.f) - a * r0;
   return r0 + r0 * e;
 }
+// Packed pairs of floats: one .f32x2 instruction computes on both halves, each
+// rounded as the scalar operation.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk2(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpk2(f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// a - b = fma(b, -1, a), one rounding
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, pk2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ f2 neg2(f2 a) { return a ^ 0x8000000080000000ull; }
+
 // A float-float complex value: the two parts' high floats packed in one
 // 64-bit register pair, their low floats in another (re in the low half).
 struct __align__(16) dcx {

@@ -25,33 +25,6 @@
 
 namespace cuna {
 
-// packed pairs of floats
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pk2(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpk2(f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-// a - b = fma(b, -1, a), one rounding
-__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, pk2(-1.0f, -1.0f), a); }
-__device__ __forceinline__ f2 neg2(f2 a) { return a ^ 0x8000000080000000ull; }
-
 __device__ __forceinline__ dcx dc_fast(f2 s, f2 e) {  // s + e renormalised, |s| >= |e|
   dcx r;
   r.h = add2(s, e);
@@ -241,13 +214,15 @@ __device__ __forceinline__ void df_fft(dcx *s, int pitch, int logL, int logB, co
 struct DfColSrc {
   const double2 *p;  // slab + c0
   int logL2;
+  bool df;  // the gridding wrote float-float (tile_flush_df), else double
   __device__ __forceinline__ dcx load(int seq, int i) const {
     // through L2: the gridding may still have been writing when this kernel started
-    return dc_load(__ldcg(p + ((int64_t)i << logL2) + seq));
+    const double2 *q = p + ((int64_t)i << logL2) + seq;
+    return df ? dc_ldcg(reinterpret_cast<const dcx *>(q)) : dc_load(__ldcg(q));
   }
 };
 
-__global__ void __launch_bounds__(1024, 1) k_df_colpass(double2 *grid, FftDev<dfl> f, int logB) {
+__global__ void __launch_bounds__(1024, 1) k_df_colpass(double2 *grid, FftDev<dfl> f, int logB, bool df_in) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   dcx *s = reinterpret_cast<dcx *>(smem_raw);
   const int L1 = 1 << f.logL1, B = 1 << logB, pitch = df_pitch(L1, B);
@@ -259,7 +234,7 @@ __global__ void __launch_bounds__(1024, 1) k_df_colpass(double2 *grid, FftDev<df
     steps[i] = twiddle_L(f, (c0 + (i >> 3)) * ((i & 7) << (f.logL1 - 3)));
   pdl_wait();  // the grid comes from the gridding
   // every read precedes the first barrier, every write follows it: in place is safe
-  df_fft<true>(s, pitch, f.logL1, logB, f.tw1, DfColSrc{z, f.logL2});
+  df_fft<true>(s, pitch, f.logL1, logB, f.tw1, DfColSrc{z, f.logL2, df_in});
   const int seq = threadIdx.x & (B - 1), k0 = threadIdx.x >> logB;
   const dcx w0 = twiddle_L(f, (c0 + seq) * k0);
   ulonglong2 *out = reinterpret_cast<ulonglong2 *>(z) + seq;
@@ -341,7 +316,7 @@ inline int df_log_elems(int logL, int logLseq, int nslab) {
 }
 
 // Both passes of nslab packed grids of 2^f.logL points at z; 0 on success
-inline int df_colpass(double2 *z, const FftDev<dfl> &f, int nslab, cudaStream_t st) {
+inline int df_colpass(double2 *z, const FftDev<dfl> &f, int nslab, bool df_in, cudaStream_t st) {
   const int le = df_log_elems(f.logL, f.logL1, nslab), logB = le - f.logL1;
   const size_t sm = sizeof(dcx) * ((size_t)df_pitch(1 << f.logL1, 1 << logB) + 8) << logB;
   static SetupFlag attr;
@@ -350,7 +325,7 @@ inline int df_colpass(double2 *z, const FftDev<dfl> &f, int nslab, cudaStream_t 
     CUNA_CK(cudaFuncSetAttribute(k_df_rowpass_acc, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     mark_setup_done(&attr);
   }
-  CUNA_CK(launch_pdl(k_df_colpass, dim3(1 << (f.logL2 - logB), nslab), dim3(1 << (le - 3)), sm, st, z, f, logB));
+  CUNA_CK(launch_pdl(k_df_colpass, dim3(1 << (f.logL2 - logB), nslab), dim3(1 << (le - 3)), sm, st, z, f, logB, df_in));
   return CUNA2_SUCCESS;
 }
 inline int df_rowpass(const double2 *z, const FftDev<dfl> &f, const AccParams<double> &e, double2 *F, int nslab,
