@@ -5,7 +5,8 @@
 // the same hardware approximations and the per-tap weights agree with the
 // reference's GPU build bit for bit; only the summation order differs.
 //
-// Pipeline per call (all on the caller's stream, no host synchronisation):
+// Pipeline per call (all on the caller's stream, no host synchronisation;
+// dependent launches from the scatter pass on):
 //   k_bin_count / k_scan_tiles / k_bin_scatter  samples -> tile-sorted records
 //   k_grid_compat     one CTA per (tile, resample): taps accumulated in shared
 //                     memory in fixed point, flushed once with f_hat[c].x += acc[c]
@@ -47,21 +48,41 @@ constexpr int kCompatMaxRf = 64;  // shared E3 table size
 __device__ __forceinline__ int compat_origin(float x, int ng, int rf) { return (int)(ng * x - rf); }
 __device__ __forceinline__ int compat_origin(double x, int ng, int rf) { return (int)(ng * x - rf); }
 
-__global__ void k_compat_filter_f32(cuna2_filter_properties_f32 *f, const float *x, int ng, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    int u = compat_origin(x[i], ng, f->filter_radius);
-    float eps = ng * x[i] - u;
-    float eps2 = eps / f->b;
-    f->E1[i] = expf(-eps * eps2) / sqrtf(CUNA_PI * f->b);
-    f->E2[i] = expf(2 * eps2);
-  } else if (i < n + f->filter_radius) {
-    int m = i - n;
-    f->E3[m] = expf(-m * m / f->b);
+// kFilterItems samples per thread, their loads in flight together (the kernel
+// streams 12 bytes per float sample through short dependent chains: 1e6 samples
+// 9.8 us with one per thread)
+constexpr int kFilterItems = 4, kFilterThreads = 256;
+
+__global__ void __launch_bounds__(kFilterThreads) k_compat_filter_f32(cuna2_filter_properties_f32 *f, const float *x,
+                                                                      int ng, int n) {
+  const int i0 = blockIdx.x * (kFilterThreads * kFilterItems) + threadIdx.x;
+  float xv[kFilterItems];
+#pragma unroll
+  for (int k = 0; k < kFilterItems; ++k) {
+    const int i = i0 + k * kFilterThreads;
+    xv[k] = i < n ? x[i] : 0.f;
+  }
+  const float b = f->b;
+  const int rf = f->filter_radius;
+  float *E1 = f->E1, *E2 = f->E2;
+#pragma unroll
+  for (int k = 0; k < kFilterItems; ++k) {
+    const int i = i0 + k * kFilterThreads;
+    if (i < n) {
+      int u = compat_origin(xv[k], ng, rf);
+      float eps = ng * xv[k] - u;
+      float eps2 = eps / b;
+      E1[i] = expf(-eps * eps2) / sqrtf(CUNA_PI * b);
+      E2[i] = expf(2 * eps2);
+    } else if (i < n + rf) {
+      int m = i - n;
+      f->E3[m] = expf(-m * m / b);
+    }
   }
 }
 
-__global__ void k_compat_filter_f64(cuna2_filter_properties_f64 *f, const double *x, int ng, int n) {
+__global__ void __launch_bounds__(kFilterThreads) k_compat_filter_f64(cuna2_filter_properties_f64 *f, const double *x,
+                                                                      int ng, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     int u = compat_origin(x[i], ng, f->filter_radius);
@@ -136,13 +157,32 @@ __device__ __forceinline__ void compat_facs(int k0, int stride, int ng, double b
 
 __device__ __forceinline__ float cpow(float a, int m) { return powf(a, m); }
 
-// Reference cell j = (int)((x + 0.5) * (ng - 1)) (double arithmetic,
-// src/gridding.cu:43,93) and the tap bounds of :53-58.  Returns false when the
+// Reference cell j = (int)((x + 0.5) * (ng - 1)), in double arithmetic
+// (src/gridding.cu:43,93).
+__device__ __forceinline__ int compat_cell(double x, int ng) { return (int)((x + 0.5) * (ng - 1)); }
+// The same for a float sample without the FP64 pipe (four operations of it per
+// sample in each binning pass; 1e6 samples, ng = 2^22: with the dependent
+// launches and the filter pass 118 -> 97 us per call): in units of 2^-40, x is an integer
+// when 2^-16 <= |x| <= 1/2 (or 0), x + 1/2 and its product with ng - 1 < 2^23
+// are exact in 64 bits, and the double product, rounded to 53 of its at most 63
+// bits, truncates to another integer only if the fraction is within 2^-31 of 1.
+// Everything else takes the double expression.
+__device__ __forceinline__ int compat_cell(float x, int ng) {
+  const unsigned u = __float_as_uint(x), ex = (u >> 23) & 0xff;
+  if (ex >= 111 && fabsf(x) <= 0.5f && ng <= (1 << 23)) {
+    const long long m = (long long)((u & 0x7fffffu) | 0x800000u) << (ex - 110);
+    const unsigned long long p = (unsigned long long)((1ll << 39) + ((int)u < 0 ? -m : m)) * (unsigned)(ng - 1);
+    if ((p & ((1ull << 40) - 1)) < (1ull << 40) - 1024) return (int)(p >> 40);
+  }
+  return compat_cell((double)x, ng);
+}
+
+// The cell and the tap bounds of src/gridding.cu:53-58.  Returns false when the
 // tap range is empty.  |j| beyond 2^30 is treated as empty: the reference's
 // int arithmetic overflows there and writes out of bounds.
-__device__ __forceinline__ bool compat_taps(double xd, int ng, int rf, bool clamp, int &j, int &ms,
-                                            int &me) {
-  j = (int)((xd + 0.5) * (ng - 1));
+template <typename T>
+__device__ __forceinline__ bool compat_taps(T x, int ng, int rf, bool clamp, int &j, int &ms, int &me) {
+  j = compat_cell(x, ng);
   if (clamp) {
     if (j >= ng) j = ng - 1;
     if (j < 0) j = 0;
@@ -185,7 +225,7 @@ template <typename T, bool BOOT> struct SampCompat {
   __device__ __forceinline__ void prep(int64_t i, const Raw &r, Prep<Rec> &p) const {
     int j, ms, me;
     p.nt = 0;
-    if (!compat_taps((double)r.x, ng, fp->filter_radius, !BOOT, j, ms, me)) return;
+    if (!compat_taps(r.x, ng, fp->filter_radius, !BOOT, j, ms, me)) return;
     const int t0 = (j + ms) >> kCompatLogTL, t1 = (j + me - 1) >> kCompatLogTL;
     p.t[0] = t0;
     p.t[1] = t1;
@@ -286,12 +326,12 @@ constexpr int kCompatThreads = 256;
 constexpr int kCompatThreadsFew = 1024;
 
 template <typename T, bool BOOT, int NT>
-__global__ void __launch_bounds__(NT) k_grid_compat(const typename RecOf<T>::type *__restrict__ recs,
-                                                                const int *__restrict__ off,
-                                                                typename CxOf<T>::type *f_hat, int ng,
-                                                                const typename FpOf<T>::type *fp,
-                                                                const T *__restrict__ y, int n, unsigned seed) {
+__global__ void __launch_bounds__(NT) k_grid_compat(const typename RecOf<T>::type *rec_ptr, const int *off,
+                                                    typename CxOf<T>::type *f_hat, int ng,
+                                                    const typename FpOf<T>::type *fp, const T *__restrict__ y, int n,
+                                                    unsigned seed) {
   typedef typename RecOf<T>::type Rec;
+  const CgSrc<Rec> recs{rec_ptr};
   typedef FixAccWide<T> FA;
   typedef typename FA::type A;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -301,6 +341,7 @@ __global__ void __launch_bounds__(NT) k_grid_compat(const typename RecOf<T>::typ
   __shared__ float red[NT / 32];
   __shared__ int redi[NT / 32];
   __shared__ T scale_s;
+  pdl_trigger();
   const int tile = blockIdx.x, slab = blockIdx.y;
   const int base = tile << kCompatLogTL;
   const int tl = min(1 << kCompatLogTL, ng - base);
@@ -314,7 +355,8 @@ __global__ void __launch_bounds__(NT) k_grid_compat(const typename RecOf<T>::typ
   for (int m = threadIdx.x; m < rf && m < kCompatMaxRf; m += NT) e3[m] = E3g[m];
   for (int q = threadIdx.x; q < NB; q += NT) hist[q] = 0;
   __syncthreads();
-  const int r0 = off[tile], r1 = off[tile + 1];
+  pdl_wait();  // records and offsets come from the binning
+  const int r0 = __ldcg(off + tile), r1 = __ldcg(off + tile + 1);
   // bound pass: records per bucket and the largest |value| (NaN if any is not finite)
   float ym = 0.f;
   for (int r = r0 + threadIdx.x; r < r1; r += NT) {
@@ -453,7 +495,7 @@ __global__ void __launch_bounds__(1 << (LOGE - 4)) k_ct_colpass_oop(const typena
 template <typename T, int LOG2> struct CtRowSrc {
   const typename CxOf<T>::type *p;  // first row of the block
   __device__ __forceinline__ typename CxOf<T>::type load(int seq, int j, int dr) const {
-    return p[(seq << LOG2) + j + dr];
+    return __ldcg(p + (seq << LOG2) + j + dr);  // through L2: the column pass may still be writing
   }
 };
 
@@ -487,10 +529,22 @@ __global__ void __launch_bounds__(1 << (LOGE - 4)) k_ct_rowpass_compat(const typ
   CtRowSrc<T, LOG2> src{in + blockIdx.y * slab_stride + ((int64_t)r0 << LOG2)};
   __shared__ T hs[4];  // read by the storing stage, after at least one barrier
   static_assert(LOG2 > 4, "the row transform has more than one stage");
+  pdl_trigger();
   compat_fac_steps(1 << (last_logns<LOG2>() + LOG1), 1 << LOGL, fp->b, hs);
+  pdl_wait();  // the rows come from the column pass
   CtFacDst<T, LOG1> dst{out + blockIdx.y * slab_stride, 1 << LOGL, r0, norm, fp->b, fp->normfac, hs};
   // rows are read point-fastest (contiguous), outputs written row-fastest
   ct_fft<T, LOG2, LOGB, true, false, true>(s, f.tw2, src, dst);
+}
+
+// Dependent launch for the float kernels only.  The double ones are bound by
+// the FP64 pipe: CTAs that become resident early crowd the SMs that happen to
+// have room and then share their pipes (1e5 samples, ng = 2^19: 193 -> 276 us).
+template <typename T, typename... KArgs, typename... Args>
+cudaError_t launch_compat(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  if (sizeof(T) == 4) return launch_pdl(k, grid, block, smem, st, args...);
+  k<<<grid, block, smem, st>>>(static_cast<KArgs>(args)...);
+  return cudaGetLastError();
 }
 
 template <typename T, int LOGL, int LOGE>
@@ -509,11 +563,13 @@ int compat_ct_sized(typename CxOf<T>::type *f_hat, typename CxOf<T>::type *scrat
     mark_setup_done(&attr);
   }
   const int64_t L = (int64_t)1 << LOGL;
-  k_ct_colpass_oop<T, LOGL, LOGE><<<dim3((1 << LOG2) / BA, nbs), TH, smA, st>>>(f_hat, scratch, f, L);
-  if (cudaPeekAtLastError() != cudaSuccess) return -1;
-  k_ct_rowpass_compat<T, LOGL, LOGE><<<dim3((1 << LOG1) / BB, nbs), TH, smB, st>>>(scratch, f_hat, f, dfp, L,
-                                                                                   norm ? 1 : 0);
-  if (cudaPeekAtLastError() != cudaSuccess) return -1;
+  typedef typename CxOf<T>::type C;
+  if (launch_compat<T>(k_ct_colpass_oop<T, LOGL, LOGE>, dim3((1 << LOG2) / BA, nbs), dim3(TH), smA, st, (const C *)f_hat,
+                 scratch, f, L) != cudaSuccess)
+    return -1;
+  if (launch_compat<T>(k_ct_rowpass_compat<T, LOGL, LOGE>, dim3((1 << LOG1) / BB, nbs), dim3(TH), smB, st, (const C *)scratch,
+                 f_hat, f, dfp, L, norm ? 1 : 0) != cudaSuccess)
+    return -1;
   return 1;
 }
 template <typename T, int LOGL>
@@ -749,11 +805,13 @@ int compat_bin(const T *x, const T *y, int n, int ng, const typename FpOf<T>::ty
     if (boot) {
       k_bin_count_resv<<<nrb, 512, sizeof(int) * ntiles, st>>>(sb, cw.counts, cw.resv, ntiles, span);
       CUNA_CK(cudaGetLastError());
-      k_bin_scatter_resv<<<nrb, 512, sms3, st>>>(sb, cw.counts, cw.resv, cw.offsets, recs, ntiles, span);
+      CUNA_CK(launch_pdl(k_bin_scatter_resv<SampCompat<T, true>>, dim3(nrb), dim3(512), sms3, st, sb,
+                         (const int *)cw.counts, (const int *)cw.resv, cw.offsets, recs, ntiles, span));
     } else {
       k_bin_count_resv<<<nrb, 512, sizeof(int) * ntiles, st>>>(sp, cw.counts, cw.resv, ntiles, span);
       CUNA_CK(cudaGetLastError());
-      k_bin_scatter_resv<<<nrb, 512, sms3, st>>>(sp, cw.counts, cw.resv, cw.offsets, recs, ntiles, span);
+      CUNA_CK(launch_pdl(k_bin_scatter_resv<SampCompat<T, false>>, dim3(nrb), dim3(512), sms3, st, sp,
+                         (const int *)cw.counts, (const int *)cw.resv, cw.offsets, recs, ntiles, span));
     }
     CUNA_CK(cudaGetLastError());
   } else {
@@ -783,11 +841,10 @@ int compat_grid(const T *x, const T *y, typename CxOf<T>::type *f_hat, int n, in
   const dim3 gg(ntiles, boot ? nbs : 1);
   constexpr int NF = kCompatThreadsFew, NM = kCompatThreads;
   const bool few = (int64_t)gg.x * gg.y < 2 * (int64_t)device_sm_count();
-  if (boot && few) k_grid_compat<T, true, NF><<<gg, NF, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
-  else if (boot) k_grid_compat<T, true, NM><<<gg, NM, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
-  else if (few) k_grid_compat<T, false, NF><<<gg, NF, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
-  else k_grid_compat<T, false, NM><<<gg, NM, smg, st>>>(recs, cw.offsets, f_hat, ng, dfp, y, n, seed);
-  CUNA_CK(cudaGetLastError());
+  auto k = boot ? (few ? k_grid_compat<T, true, NF> : k_grid_compat<T, true, NM>)
+                : (few ? k_grid_compat<T, false, NF> : k_grid_compat<T, false, NM>);
+  CUNA_CK(launch_compat<T>(k, gg, dim3(few ? NF : NM), smg, st, (const Rec *)recs, (const int *)cw.offsets, f_hat, ng, dfp, y,
+                     n, seed));
   return CUNA2_SUCCESS;
 }
 
@@ -816,11 +873,11 @@ int compat_filter(const T *x, int n, int ng, FP *h, FP *d, cudaStream_t st) {
   h->filter_radius = rf;
   h->normfac = sqrt(2 * CUNA_PI);
   CUNA_CK(cudaMemcpyAsync(d, h, sizeof(FP), cudaMemcpyHostToDevice, st));
-  const int nb = (n + rf + 255) / 256;
+  const int per = kFilterThreads * (sizeof(T) == 4 ? kFilterItems : 1), nb = (int)(((int64_t)n + rf + per - 1) / per);
   if (sizeof(T) == 4)
-    k_compat_filter_f32<<<nb, 256, 0, st>>>((cuna2_filter_properties_f32 *)d, (const float *)x, ng, n);
+    k_compat_filter_f32<<<nb, kFilterThreads, 0, st>>>((cuna2_filter_properties_f32 *)d, (const float *)x, ng, n);
   else
-    k_compat_filter_f64<<<nb, 256, 0, st>>>((cuna2_filter_properties_f64 *)d, (const double *)x, ng, n);
+    k_compat_filter_f64<<<nb, kFilterThreads, 0, st>>>((cuna2_filter_properties_f64 *)d, (const double *)x, ng, n);
   CUNA_CK(cudaGetLastError());
   return CUNA2_SUCCESS;
 }
@@ -921,7 +978,7 @@ __global__ void k_inspect_compat_taps(const T *x, int n, int ng, int rf, int cla
   if (i >= n) return;
   const T xi = x[i];
   int j = 0, ms = 0, me = 0;
-  const bool any = compat_taps((double)xi, ng, rf, clamp != 0, j, ms, me);
+  const bool any = compat_taps(xi, ng, rf, clamp != 0, j, ms, me);
   if (cell) cell[i] = j;
   if (origin) origin[i] = compat_origin(xi, ng, rf);
   if (tlo) tlo[i] = any ? ms : 0;

@@ -134,24 +134,32 @@ def test_float_float_passes_lengths(mods, nf, R, m):
     assert rel_l2(F[ks + nf // 2], D) < 1e-11 + 10 * np.exp(-np.pi * m * np.sqrt(1 - 1 / R))
 
 
-@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-6), (torch.float64, 1e-11)])
-@pytest.mark.parametrize("n", [1, 8, 511, 2049, 16384, 16385])
-def test_binning_in_one_launch(mods, oracle_lib, dtype, tol, n):
-    """Short series binned by one cluster launch (up to 16384 samples) and the
-    next size above it, with samples on tile edges and the grid's seam, against
-    the oracle's double restatement (float: rounding of 2m n terms; double: the
-    restatement's phase rounding, 2 pi 2^13 1e-16 per sample)."""
-    _, nfft = mods
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n,nf", [(1, 1 << 15), (8, 1 << 15), (511, 1 << 20), (2049, 1 << 18), (16384, 1 << 16), (16385, 1 << 16)])
+def test_binning_in_one_launch(mods, oracle_lib, dt, n, nf):
+    """Short series binned by one cluster launch (up to 16384 samples; the next
+    size takes the two-launch sort), few and many tiles, samples on tile edges
+    and the grid's seam: every tile's records equal the oracle's integer steps,
+    as sets."""
+    import test_gpu_integer_steps as steps
+    from cunfft_adjoint_gb300 import _lib, nfft
     rng = np.random.default_rng(n)
-    nf, R, m, T = 1 << 14, 2, 8, 5.0
+    R, m, T = 2, 8, 5.0
     t = np.sort(rng.uniform(0, T, n))
-    edges = np.array([0.0, 2048.0, 4096.0, 2047.99, 32767.99]) / (R * nf) * T
+    edges = np.array([0.0, 2048.0, 4096.0, 2047.99, R * nf - 0.01]) / (R * nf) * T
     t[:min(n, 5)] = edges[:min(n, 5)]
-    y = rng.normal(0, 1, n)
-    plan = nfft.AdjointNFFT(nf, R, m, dtype)
-    F = plan(torch.as_tensor(t, device="cuda"), torch.as_tensor(y, dtype=dtype, device="cuda"), 0.0, T).cpu().numpy()
-    ys = y.astype(np.float32).astype(np.float64) if dtype == torch.float32 else y
-    assert rel_l2(F, oracle_lib.accurate_adjoint(t, ys, 0.0, T, nf, R, m)) < tol
+    y = rng.normal(0, 1, n).astype(dt)
+    plan = nfft.AdjointNFFT(nf, R, m, torch.float32 if dt == np.float32 else torch.float64)
+
+    class Lib:
+        check, core = staticmethod(_lib.check), staticmethod(_lib.core)
+    log_tile, offs, recs = steps._plan_bins_device(Lib, plan, t, y, 0.0, T)
+    _, cell, _, _ = oracle_lib.phases(t, 0.0, T, plan.ng)
+    ta, tb = oracle_lib.accurate_tiles(cell, plan.ng, m, log_tile)
+    want = sorted([(int(a), int(cell[i]), i) for i, a in enumerate(ta)]
+                  + [(int(b), int(cell[i]), i) for i, b in enumerate(tb) if b != ta[i] and b >= 0])
+    tile = np.repeat(np.arange(len(offs) - 1), np.diff(offs))
+    assert sorted(zip(tile.tolist(), recs["cell"].tolist(), recs["p"].tolist())) == want
 
 
 @pytest.mark.parametrize("scale", [1e-30, 1.0, 1e18])
