@@ -79,7 +79,9 @@ template <typename T> struct BwdCoef {
 // 0..V-1 of them): W/V vector loads instead of 2M scalar ones.  Only the first
 // and the last groups hold cells outside the window; they are set to zero.
 //  - float: exp2 per tap (the hardware's, whose bits exp2f returns for the
-//    exponents above -126 that taps have) and the sums in tap order.
+//    exponents above -126 that taps have) and the sums in tap order; what is
+//    not a sum runs on two taps at a time in the packed instructions, which
+//    round each half as the scalar ones do.
 //  - double: with h the centre cell, x0 = b0 + h - s and the factorisation
 //    exp2(-k1 (j + x0)^2) = E Q^j c_j (E = exp2(-k1 x0^2), Q = exp2(-2 k1 x0),
 //    c_j = exp2(-k1 j^2)), the sums run as two Horner chains outwards-in:
@@ -112,12 +114,17 @@ __device__ __forceinline__ void bwd_window(const T *R, int ng, int cell, T fr, c
   const int lo = cell - M + 1;
   const int b0 = lo & ~(V - 1), a = lo - b0;
   T v[W];
+  if ((unsigned)b0 <= (unsigned)(ng - W)) {
 #pragma unroll
-  for (int g = 0; g < X::NG; ++g) {
-    int b = b0 + g * V;
-    if (b < 0) b += ng;
-    else if (b >= ng) b -= ng;
-    BwdVec<T, V>::load(R + b, v + g * V);
+    for (int g = 0; g < X::NG; ++g) BwdVec<T, V>::load(R + b0 + g * V, v + g * V);
+  } else {  // wraps around the period
+#pragma unroll
+    for (int g = 0; g < X::NG; ++g) {
+      int b = b0 + g * V;
+      if (b < 0) b += ng;
+      else if (b >= ng) b -= ng;
+      BwdVec<T, V>::load(R + b, v + g * V);
+    }
   }
   // cells before the window (i < a <= V - 1) and after it (i >= a + 2M)
 #pragma unroll
@@ -126,15 +133,24 @@ __device__ __forceinline__ void bwd_window(const T *R, int ng, int cell, T fr, c
     if (i >= 2 * M) v[i] = i < a + 2 * M ? v[i] : (T)0;
   }
   if constexpr (sizeof(T) == 4) {
-    const T d0 = (T)(b0 - cell);
-    sy = (T)0;
-    st = (T)0;
+    const float d0 = (float)(b0 - cell);
+    const f2 nk = pk2(-cf.k1, -cf.k1), nf = pk2(-fr, -fr), two = pk2(2.f, 2.f);
+    f2 D = pk2(d0, d0 + 1.f);  // the cells' whole distances, exact
+    sy = 0.f;
+    st = 0.f;
 #pragma unroll
-    for (int i = 0; i < W; ++i) {
-      const T dd = (d0 + (T)i) - fr;
-      const T w = v[i] * exp2_g(-cf.k1 * dd * dd);
-      sy += w;
-      st += w * dd * cf.inv2tau;
+    for (int i = 0; i < W; i += 2) {
+      const f2 dd = add2(D, nf);
+      float x0, x1, w0, w1, u0, u1;
+      unpk2(mul2(mul2(nk, dd), dd), x0, x1);
+      const f2 w = mul2(pk2(v[i], v[i + 1]), pk2(exp2_g(x0), exp2_g(x1)));
+      unpk2(w, w0, w1);
+      unpk2(mul2(w, dd), u0, u1);
+      sy += w0;
+      st = fmaf(u0, cf.inv2tau, st);
+      sy += w1;
+      st = fmaf(u1, cf.inv2tau, st);
+      D = add2(D, two);
     }
   } else {
     const T x0 = (T)(b0 + H - cell) - fr;
@@ -168,7 +184,8 @@ __device__ __forceinline__ double to_double(float v) {
 // Interpolation at every sample of the series blockIdx.y from its real field.
 // Bound by the instruction issue (float, 64 series of 2e5 sorted samples, m =
 // 10: 276 us with 2m scalar loads, wraps and a 64-bit division per sample, 191
-// us here) and, for double, by the FP64 pipe (2e5 samples: 217 us with an exp2
+// us with scalar arithmetic and a wrap test per group, 170 us here) and, for
+// double, by the FP64 pipe (2e5 samples: 217 us with an exp2
 // per tap, 65 us here).
 template <typename T, int M>
 __global__ void __launch_bounds__(256) k_bwd_interp(const double *__restrict__ t, const T *__restrict__ y, int64_t n,
