@@ -80,16 +80,38 @@ __global__ void __launch_bounds__(512) k_bin_count(S smp, int *__restrict__ coun
 }
 
 // Single CTA (1024 threads): offsets[t] = sum_{u<t} counts[u], offsets[ntiles]
-// = total, cursor[t] = 0.
+// = total, cursor[t] = 0 (where given).  A thread owns whole groups of four
+// counts, moved as 16-byte words where the arrays are aligned to them: single
+// words at a stride of a thread's share make one SM write a sector per word
+// (8192 tiles: 12.4 us, 6.0 us here).
+__device__ __forceinline__ int4 scan_load4(const int *p, int n, bool vec) {
+  if (vec && n >= 4) return *reinterpret_cast<const int4 *>(p);
+  return make_int4(n > 0 ? p[0] : 0, n > 1 ? p[1] : 0, n > 2 ? p[2] : 0, n > 3 ? p[3] : 0);
+}
+__device__ __forceinline__ void scan_store4(int *p, int4 v, int n, bool vec) {
+  if (vec && n >= 4) {
+    *reinterpret_cast<int4 *>(p) = v;
+    return;
+  }
+  if (n > 0) p[0] = v.x;
+  if (n > 1) p[1] = v.y;
+  if (n > 2) p[2] = v.z;
+  if (n > 3) p[3] = v.w;
+}
 __global__ void __launch_bounds__(1024) k_scan_tiles(const int *__restrict__ counts,
                                                      int *__restrict__ offsets,
                                                      int *__restrict__ cursor, int ntiles) {
   __shared__ int wsum[32];
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int per = (ntiles + nt - 1) / nt;
+  const int per = ((ntiles + nt - 1) / nt + 3) & ~3;
   const int beg = min(tid * per, ntiles), end = min(beg + per, ntiles);
+  const bool vec = (((uintptr_t)counts | (uintptr_t)offsets | (uintptr_t)cursor) & 15) == 0;
   int sum = 0;
-  for (int i = beg; i < end; ++i) sum += counts[i];
+#pragma unroll 2
+  for (int i = beg; i < end; i += 4) {
+    const int4 c = scan_load4(counts + i, end - i, vec);
+    sum += c.x + c.y + c.z + c.w;
+  }
   const int lane = tid & 31, w = tid >> 5;
   int v = sum;
 #pragma unroll
@@ -110,10 +132,12 @@ __global__ void __launch_bounds__(1024) k_scan_tiles(const int *__restrict__ cou
   }
   __syncthreads();
   int run = v - sum + (w > 0 ? wsum[w - 1] : 0);
-  for (int i = beg; i < end; ++i) {
-    offsets[i] = run;
-    run += counts[i];
-    cursor[i] = 0;
+#pragma unroll 2
+  for (int i = beg; i < end; i += 4) {
+    const int4 c = scan_load4(counts + i, end - i, vec);
+    scan_store4(offsets + i, make_int4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z), end - i, vec);
+    run += c.x + c.y + c.z + c.w;
+    if (cursor) scan_store4(cursor + i, make_int4(0, 0, 0, 0), end - i, vec);
   }
   if (tid == nt - 1) offsets[ntiles] = wsum[(nt >> 5) - 1];
 }
