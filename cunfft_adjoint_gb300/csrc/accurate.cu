@@ -440,7 +440,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   }
   size_t smg;
   if (p->grid_method == CUNA2_GRID_GATHER) smg = grid_smem_bytes<T>(p->logTL, p->m);
-  else if (p->grid_method == CUNA2_GRID_FIXED) smg = grid_fixed_smem_bytes<T>(p->logTL, p->m);
+  else if (p->grid_method == CUNA2_GRID_FIXED) smg = grid_fixed_smem_bytes<T>(p->logTL, p->m, !seg && !wts);
   else smg = grid_scatter_smem_bytes<T>(p->logTL);
   smg = (smg + 15) & ~(size_t)15;
   const dim3 gb(kGridThreads);

@@ -526,7 +526,7 @@ int batch_run(cuna2_batch_plan_st *p, const double *t, const T *y, typename CxOf
       // the bucket table's length depends on m, not monotonically: the
       // largest over the batch's filter widths
       size_t smg = 0;
-      for (int mw : p->m_set) smg = std::max(smg, grid_fixed_smem_bytes<T>(p->log_tile, mw));
+      for (int mw : p->m_set) smg = std::max(smg, grid_fixed_smem_bytes<T>(p->log_tile, mw, true));
       k_bgrid<T><<<ntl, kGridThreads, smg, st>>>(rc, p->offsets, (T *)p->grid, D, ts);
     }
     CUNA_CK(cudaGetLastError());

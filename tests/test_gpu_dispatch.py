@@ -181,3 +181,49 @@ def test_lomb_scargle_scales(mods, scale, n, nfreq):
     P = lomb_scargle(td, y32, dy32, nfreq=nfreq, df=1 / 500.0, t0=0.0)
     D = lomb_scargle(td, y32.double() / scale, dy32.double(), nfreq=nfreq, df=1 / 500.0, t0=0.0, R=4, m=12)
     assert rel_l2(P.cpu().numpy(), D.cpu().numpy()) < 1e-4
+
+
+@pytest.mark.parametrize("R,m", [(8, 1), (4, 4), (2, 5), (2, 8), (2, 16)])
+@pytest.mark.parametrize("cnt", [0, 1, 256, 257, 512, 513, 1024, 1025, 2600])
+def test_fixed_point_own_values(mods, cnt, R, m):
+    """Float fixed-point tiles of one transform, which read their records twice
+    (the first two of a thread kept in registers), against the same records
+    staged in shared memory, as a channel of a multi-channel transform runs:
+    equal bits.  cnt samples fall into one tile, some at its edges, few into
+    the others.  Against the double plan of the same filter: 2e-6 (2^-22 of
+    each weight's exp2 and 2^-30 of a tile's bound per tap)."""
+    from cunfft_adjoint_gb300 import _lib
+    _, nfft = mods
+    rng = np.random.default_rng(cnt + m)
+    nf, T = (1 << 17) // R, 3.0
+    ng = R * nf
+    pos = np.concatenate([4096 * 5 + rng.uniform(m, 4096 - m, cnt), rng.uniform(0, ng, 50),
+                          4096 * 5 + rng.uniform(-m, m, min(cnt, 4)), rng.uniform(0, m, 3), ng - rng.uniform(0, m, 3)])
+    t = torch.as_tensor(pos / ng * T, device="cuda")
+    y = torch.as_tensor(rng.normal(0, 1, pos.size), device="cuda")
+    plan = nfft.AdjointNFFT(nf, R, m)
+    plan.set_schedule(12, _lib.GRID_FIXED)
+    F = plan(t, y.float(), 0.0, T).clone()
+    assert torch.equal(plan.multi(t, torch.stack([y.float(), -y.float()]), 0.0, T)[0], F)
+    D = nfft.AdjointNFFT(nf, R, m, torch.float64)(t, y.float().double(), 0.0, T)
+    assert rel_l2(F.cpu().numpy(), D.cpu().numpy()) < 2e-6
+
+
+@pytest.mark.parametrize("n,log_tile", [(0, 9), (1, 9), (5000, 9), (5000, 11)])
+def test_scan_of_many_tiles(mods, n, log_tile):
+    """8192 and 2048 tiles: one CTA's scan of the counts (above 4096 tiles) and
+    the scatter pass's own, against the double plan (float rounding, 2e-6)."""
+    from cunfft_adjoint_gb300 import _lib
+    _, nfft = mods
+    rng = np.random.default_rng(n)
+    nf, T = 1 << 21, 2.0
+    t = torch.as_tensor(rng.uniform(0, T, n), device="cuda")
+    y = torch.as_tensor(rng.normal(0, 1, n), device="cuda")
+    plan = nfft.AdjointNFFT(nf, 2, 8)
+    plan.set_schedule(log_tile, _lib.GRID_GATHER)
+    F = plan(t, y.float(), 0.0, T)
+    if n == 0:
+        assert not F.abs().any()
+        return
+    D = nfft.AdjointNFFT(nf, 2, 8, torch.float64)(t, y.float().double(), 0.0, T)
+    assert rel_l2(F.cpu().numpy(), D.cpu().numpy()) < 2e-6
