@@ -336,9 +336,10 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
       CUNA_CK(cudaFuncSetAttribute(k_nfft_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
       mark_setup_done(&attr);
     }
-    const bool alone = nslab <= nsm, gather = small_gather(L, alone, sizeof(T) == 4);
-    k_nfft_small<T><<<nslab, small_threads<T>(L, alone, gather), small_smem<T>(L, p->m, gather), st>>>(
-        t, y, n, pm, e, f, F, wts, gather);
+    const bool alone = nslab <= nsm;
+    const int cap = small_cap(L, alone, sizeof(T) == 4);
+    k_nfft_small<T><<<nslab, small_threads<T>(L, alone, cap), small_smem<T>(L, p->m, cap), st>>>(
+        t, y, n, pm, e, f, F, wts, cap);
     CUNA_CK(cudaGetLastError());
     mark(pr, "nfft_small", st);
     return CUNA2_SUCCESS;

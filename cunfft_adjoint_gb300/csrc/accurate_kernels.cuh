@@ -420,7 +420,7 @@ __device__ __forceinline__ void gauss_acc(T y, T x, T k1, const GaussCW<T, CW> &
 //
 // Two griddings.  Scatter: a thread per sample adds its 2m taps with shared
 // atomics (float: compare-and-swap loops, 3 adds per clock and SM).  Gather
-// (float): the samples go in chunks of up to small_cap(ng) records; a chunk is
+// (float): the samples go in chunks of up to small_cap records; a chunk is
 // counting-sorted in shared memory by group of four cells (one atomic per
 // record ranks it, the gather reads it through an index), then every thread
 // sums its groups of four cells over the records in reach, as the tiled gather
@@ -432,24 +432,28 @@ __device__ __forceinline__ void gauss_acc(T y, T x, T k1, const GaussCW<T, CW> &
 // R = 2, m = 8: 28.7 us per call with L / 16 threads and the scatter, 14.1 us
 // here.
 inline bool small_gather(int L, bool alone, bool is_float) { return is_float && L <= (alone ? 8192 : 2048); }
+// records of a chunk (0: scatter).  With an SM to itself a transform takes the
+// most, fewer chunks of five barriers each; in a batch the shared memory of
+// CTAs that share an SM counts.  On the device, with a group's records shared
+// out to its idle threads: 2000 samples on 64 cells 160 us in chunks of 32,
+// 10.9 in one; 500 samples on 2^11 cells 6.1 either way.
 constexpr int kSmallCapMax = 2048;
-__host__ __device__ __forceinline__ int small_cap(int64_t ng) {
-  const int64_t c = ng / 4;
-  return (int)(c < 32 ? 32 : (c > kSmallCapMax ? kSmallCapMax : c));
+inline int small_cap(int L, bool alone, bool is_float) {
+  if (!small_gather(L, alone, is_float)) return 0;
+  return alone ? kSmallCapMax : std::max(32, std::min(kSmallCapMax, L / 2));
 }
 // shared bytes: FFT buffer | gather: records, index, group starts; scatter: E3
-template <typename T> size_t small_smem(int L, int m, bool gather) {
+template <typename T> size_t small_smem(int L, int m, int cap) {
   const size_t fft = sizeof(typename CxOf<T>::type) * (size_t)fft_pitch(L, 1);
-  if (!gather) return fft + sizeof(T) * (2 * m + 2);
-  const int cap = small_cap(2 * (int64_t)L);
+  if (cap == 0) return fft + sizeof(T) * (2 * m + 2);
   return ((fft + 15) & ~(size_t)15) + (size_t)cap * (sizeof(SRec<float>) + sizeof(int)) +
          sizeof(int) * ((size_t)(2 * L) / 4 + 1);
 }
 // threads of a small transform: the FFT keeps L / 16 busy, the samples, groups
 // and outputs more; `alone`: the launch has an SM per transform
-template <typename T> int small_threads(int L, bool alone, bool gather) {
+template <typename T> int small_threads(int L, bool alone, int cap) {
   const int most = sizeof(T) == 4 ? 1024 : 512;
-  const int want = gather ? (alone ? L / 2 : L / 8) : (alone ? most : L / kFftE);
+  const int want = cap ? (alone ? std::max(L / 2, 256) : L / 8) : (alone ? most : L / kFftE);
   return std::max(std::max(32, std::min(most, L / kFftE)), std::min(most, want));
 }
 
@@ -458,7 +462,8 @@ template <typename T> int small_threads(int L, bool alone, bool gather) {
 // indices wrap around the periodic grid (images o = -1, 0, 1)
 template <bool MASKED>
 __device__ __forceinline__ void small_gather4(const SRec<float> *srec, const int *order, const int *start, int g, int NG,
-                                              int ng, int m, float k1, const GaussCW<float, 4> &gw, float *a) {
+                                              int ng, int m, float k1, const GaussCW<float, 4> &gw, int part, int step,
+                                              float *a) {
   const int c0 = 4 * g;
   const int glo = (c0 - m) >> 2, ghi = (c0 + m + 2) >> 2;
 #pragma unroll 1
@@ -467,7 +472,7 @@ __device__ __forceinline__ void small_gather4(const SRec<float> *srec, const int
     if (lo > hi) continue;
     const int c = c0 - o * ng;  // the group's first cell as this image sees it
     const int re = start[hi + 1];
-    for (int r = start[lo]; r < re; ++r) {
+    for (int r = start[lo] + part; r < re; r += step) {
       const SRec<float> q = srec[order[r]];
       const int dc = c - q.lc;
       gauss_acc<float, 4, MASKED>(q.y, (float)dc - q.f, k1, gw, m - dc, 2 * m, a);
@@ -477,11 +482,17 @@ __device__ __forceinline__ void small_gather4(const SRec<float> *srec, const int
 
 __device__ __forceinline__ void small_grid_gather(const double *__restrict__ t, const float *__restrict__ y, int64_t n,
                                                   const PhaseMul &pm, const AccParams<float> &e, float *sr,
-                                                  SRec<float> *srec, int *order, int *start) {
-  const int ng = (int)e.ng, NG = ng / 4, m = e.m, cap = small_cap(ng);
+                                                  SRec<float> *srec, int *order, int *start, int cap) {
+  const int ng = (int)e.ng, NG = ng / 4, m = e.m;
   const GaussCW<float, 4> gw(e.k1);
   // as tail_free_gather: exp(-m^2 / (4 tau)) < 1e-8
   const bool masked = e.k1 * (float)(m * m) < 26.6f;
+  // Where there are fewer groups than threads, 2^LP threads share a group's
+  // records (NG is a power of two: with LP > 0 either all threads have a group
+  // or, at LP = 5, whole warps have none).
+  int LP = 0;
+  while (LP < 5 && (NG << LP) < (int)blockDim.x) ++LP;
+  const int part = threadIdx.x & ((1 << LP) - 1), step = 1 << LP;
   int64_t c0 = 0;
   do {
     const int cnt = (int)min((int64_t)cap, n - c0);
@@ -499,14 +510,20 @@ __device__ __forceinline__ void small_grid_gather(const double *__restrict__ t, 
     cta_scan_in_place(start, NG);
     for (int i = threadIdx.x; i < cnt; i += blockDim.x) order[start[srec[i].lc >> 2] + srec[i].pad] = i;
     __syncthreads();
-    for (int g = threadIdx.x; g < NG; g += blockDim.x) {
+    for (int g = threadIdx.x >> LP; g < NG; g += blockDim.x >> LP) {
       float a[4] = {0.f, 0.f, 0.f, 0.f};
-      if (masked) small_gather4<true>(srec, order, start, g, NG, ng, m, e.k1, gw, a);
-      else small_gather4<false>(srec, order, start, g, NG, ng, m, e.k1, gw, a);
+      if (masked) small_gather4<true>(srec, order, start, g, NG, ng, m, e.k1, gw, part, step, a);
+      else small_gather4<false>(srec, order, start, g, NG, ng, m, e.k1, gw, part, step, a);
+      for (int o = 1; o < step; o <<= 1) {  // whole warps: see LP
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float &d = sr[real_slot(4 * g + i)];
-        d = c0 == 0 ? a[i] : d + a[i];
+        for (int i = 0; i < 4; ++i) a[i] += __shfl_xor_sync(0xffffffffu, a[i], o);
+      }
+      if (part == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float &d = sr[real_slot(4 * g + i)];
+          d = c0 == 0 ? a[i] : d + a[i];
+        }
       }
     }
     c0 += cap;
@@ -516,19 +533,18 @@ __device__ __forceinline__ void small_grid_gather(const double *__restrict__ t, 
 template <typename T>
 __device__ __forceinline__ void nfft_small_body(const double *__restrict__ t, const T *__restrict__ y,
                                                 int64_t n, const PhaseMul &pm, const AccParams<T> &e,
-                                                const FftDev<T> &f, typename CxOf<T>::type *F, bool gather) {
+                                                const FftDev<T> &f, typename CxOf<T>::type *F, int cap) {
   typedef typename CxOf<T>::type C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int L = 1 << f.logL;
   const int pitch = fft_pitch(L, 1);
   C *s = reinterpret_cast<C *>(smem_raw);
   T *sr = reinterpret_cast<T *>(smem_raw);
-  if (sizeof(T) == 4 && gather) {
+  if (sizeof(T) == 4 && cap) {
     if constexpr (sizeof(T) == 4) {
-      const int cap = small_cap(e.ng);
       SRec<float> *srec = reinterpret_cast<SRec<float> *>(smem_raw + ((sizeof(C) * pitch + 15) & ~(size_t)15));
       int *order = reinterpret_cast<int *>(srec + cap);
-      small_grid_gather(t, y, n, pm, e, sr, srec, order, order + cap);
+      small_grid_gather(t, y, n, pm, e, sr, srec, order, order + cap, cap);
     }
   } else {
     T *e3 = reinterpret_cast<T *>(s + pitch);
@@ -572,14 +588,14 @@ template <typename T>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_nfft_small(const double *__restrict__ t, const T *__restrict__ y,
                                                      int64_t n, PhaseMul pm, AccParams<T> e, FftDev<T> f,
                                                      typename CxOf<T>::type *F, const T *__restrict__ wts,
-                                                     bool gather) {
+                                                     int cap) {
   // one CTA per output slab: slab b grids wts[b*n + j] when wts is given
   // (bootstrap resample b), else y[j]
   if (wts) {
     y = wts + (int64_t)blockIdx.x * n;
     F += (int64_t)blockIdx.x * e.nf;
   }
-  nfft_small_body<T>(t, y, n, pm, e, f, F, gather);
+  nfft_small_body<T>(t, y, n, pm, e, f, F, cap);
 }
 
 __device__ __forceinline__ void store4(float *p, float a, float b, float c, float d) {

@@ -227,9 +227,9 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 1024 : 512) k_bsmall(const do
                                                                         const T *__restrict__ y,
                                                                         const BDesc<T> *__restrict__ D,
                                                                         const int *__restrict__ list,
-                                                                        typename CxOf<T>::type *F, bool gather) {
+                                                                        typename CxOf<T>::type *F, int cap) {
   const BDesc<T> d = D[list[blockIdx.x]];
-  nfft_small_body<T>(t + d.s_off, y + d.s_off, d.n, d.pm, d.e, d.f, F + d.f_off, gather);
+  nfft_small_body<T>(t + d.s_off, y + d.s_off, d.n, d.pm, d.e, d.f, F + d.f_off, cap);
 }
 
 template <typename T> AccParams<T> series_params(int64_t nf, int R, int m, double tau, int logTL) {
@@ -480,9 +480,10 @@ int batch_run(cuna2_batch_plan_st *p, const double *t, const T *y, typename CxOf
     for (size_t c = 0; c < p->small_classes.size(); ++c) {
       const int logL = p->small_classes[c].first, cnt = p->small_classes[c].second;
       const int L = 1 << logL;
-      const bool alone = cnt <= device_sm_count(), gather = small_gather(L, alone, sizeof(T) == 4);
-      k_bsmall<T><<<cnt, small_threads<T>(L, alone, gather), small_smem<T>(L, p->m_max, gather), ss>>>(
-          t, y, D, (const int *)p->d_small_list + p->small_class_off[c], F, gather);
+      const bool alone = cnt <= device_sm_count();
+      const int cap = small_cap(L, alone, sizeof(T) == 4);
+      k_bsmall<T><<<cnt, small_threads<T>(L, alone, cap), small_smem<T>(L, p->m_max, cap), ss>>>(
+          t, y, D, (const int *)p->d_small_list + p->small_class_off[c], F, cap);
       CUNA_CK(cudaGetLastError());
     }
     if (fork) CUNA_CK(cudaEventRecord(p->ev_join, p->side));
