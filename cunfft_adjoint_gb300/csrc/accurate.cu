@@ -32,6 +32,7 @@
 #include <vector>
 #include "accurate_kernels.cuh"
 #include "backward.h"
+#include "cluster.cuh"
 #include "fftpass.cuh"
 #include "fftpass_df.cuh"
 
@@ -48,6 +49,10 @@ struct cuna2_plan_st {
   // run tiled (binning, tiled gridding, two FFT passes) instead
   bool has_split = false;
   bool tiled_single = true;
+  // float plans of middling length: a short single transform in one cluster
+  // launch (cluster.cuh), until the caller chooses a schedule
+  bool cluster = false;
+  cuna::FftGeom geom_cl;
   cuna::FftGeom geom4;
   // double plans with four-step passes: the float-float geometry the passes
   // compute in (fft_geometry_df)
@@ -255,7 +260,10 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   const AccParams<T> e = make_params<T>(p);
   // a few slabs of a small plan (one transform, a few channels) run tiled
   // over many CTAs when they can; many slabs take one CTA each
-  const bool small = p->small && !(p->has_split && p->tiled_single && 2 * nslab <= device_sm_count());
+  bool clus = false;
+  if constexpr (sizeof(T) == 4)
+    clus = p->cluster && cluster_takes(p->geom.logL, n, nslab) && p->binning == CUNA2_BIN_GLOBAL && !bo && !grep;
+  const bool small = !clus && p->small && !(p->has_split && p->tiled_single && 2 * nslab <= device_sm_count());
   const FftDev<T> f = to_dev<T>(small || !p->small ? p->geom : p->geom4);
   const int L = 1 << p->geom.logL;
   const int ntiles = p->ntiles;
@@ -264,7 +272,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   // Chunks of CH samples: at least two per SM, at most kSegMaxChunks.
   const int nsm = device_sm_count();
   int CH = 0, nch = 0;
-  if (p->binning == CUNA2_BIN_LOCAL && !small && n > 0 && ntiles <= kScanFuseTiles) {
+  if (p->binning == CUNA2_BIN_LOCAL && !small && !clus && n > 0 && ntiles <= kScanFuseTiles) {
     int64_t want = std::max<int64_t>(std::max<int64_t>((n + 2 * nsm - 1) / (2 * nsm),
                                                        (n + kSegMaxChunks - 1) / kSegMaxChunks), 1024);
     want = (want + 511) / 512 * 512;
@@ -275,9 +283,9 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   }
   const bool seg = nch > 0;
   // short series: the whole sort in one launch
-  const bool one = !small && !seg && n > 0 && n <= kBinOneN && ntiles <= kScanFuseTiles;
+  const bool one = !small && !seg && !clus && n > 0 && n <= kBinOneN && ntiles <= kScanFuseTiles;
   // reserved two-pass binning: CTAs of rspan samples, a table of nrb x ntiles
-  const bool resv = !small && !seg && !one && n > 0 && ntiles <= kScanFuseTiles;
+  const bool resv = !small && !seg && !one && !clus && n > 0 && ntiles <= kScanFuseTiles;
   const int64_t rspan = resv ? resv_span(n, ntiles, nsm) : 0;
   const int nrb = resv ? (int)((n + rspan - 1) / rspan) : 0;
   // workspace: counts | cursor | offsets | phases or chunk table | reservations
@@ -290,12 +298,12 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   const size_t o_cnt = 0, o_cur = align_up(sizeof(int) * ntiles), o_off = 2 * o_cur;
   const size_t o_hdr = o_off + align_up(sizeof(int) * (ntiles + 1));
   const size_t nrec = seg ? 2 * ((size_t)n + CH) : 2 * (size_t)(n > 0 ? n : 1);
-  const size_t phs_b = small || one ? 0
+  const size_t phs_b = small || one || clus ? 0
                              : (seg ? align_up(sizeof(int) * (size_t)ntiles * nch)
                                     : align_up(sizeof(uint64_t) * (size_t)(n > 0 ? n : 1)));
   const size_t rsv_b = resv ? align_up(sizeof(int) * (size_t)nrb * ntiles) : 0;
-  const size_t rec_b = small ? 0 : align_up(sizeof(Rec) * nrec);
-  const size_t grid_b = small ? 0 : align_up(sizeof(T) * (size_t)p->ng * nslab);
+  const size_t rec_b = small || clus ? 0 : align_up(sizeof(Rec) * nrec);
+  const size_t grid_b = small || clus ? 0 : align_up(sizeof(T) * (size_t)p->ng * nslab);
   const bool share = resv && phs_b + rsv_b <= grid_b;
   const size_t o_phs = share ? o_hdr + rec_b : o_hdr;
   const size_t o_rsv = o_phs + phs_b;
@@ -329,6 +337,23 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     k_boot_weights<T><<<nbs, 1024, sm ? sizeof(int) * (size_t)n : 0, st>>>(y, (int)n, seed, wts);
     CUNA_CK(cudaGetLastError());
     mark(pr, "boot_weights", st);
+  }
+  if constexpr (sizeof(T) == 4) {
+    if (clus) {
+      const bool masked = !tail_free_gather(true, p->m, p->tau) || masked_gather_forced();
+      const float *v = wts ? wts : y;
+      const int logL = p->geom.logL;
+      if (logL < kClusterLo) {
+        if (masked) CUNA_TRY(nfft_cluster_small<true>(logL, t, v, (int)n, pm, e, to_dev<T>(p->geom), F, nslab, st));
+        else CUNA_TRY(nfft_cluster_small<false>(logL, t, v, (int)n, pm, e, to_dev<T>(p->geom), F, nslab, st));
+      } else {
+        const FftDev<T> fc = to_dev<T>(p->geom_cl);
+        if (masked) CUNA_TRY(nfft_cluster<true>(logL, t, v, (int)n, pm, e, fc, F, nslab, st));
+        else CUNA_TRY(nfft_cluster<false>(logL, t, v, (int)n, pm, e, fc, F, nslab, st));
+      }
+      mark(pr, "nfft_cluster", st);
+      return CUNA2_SUCCESS;
+    }
   }
   if (small) {
     static SetupFlag attr;
@@ -598,6 +623,11 @@ extern "C" int cuna2_plan_create(cuna2_plan *plan, int dtype, int64_t nf, int R,
   }
   p->has_df = dtype == CUNA2_F64 && !p->small && logL <= 23;
   if (p->has_df && (st = fft_geometry_df(logL, &p->geom_df))) {
+    delete p;
+    return st;
+  }
+  p->cluster = dtype == CUNA2_F32 && cluster_fits(logL, m);
+  if (p->cluster && logL >= kClusterLo && (st = fft_geometry(false, logL, &p->geom_cl, logL <= kSingleLogF32))) {
     delete p;
     return st;
   }
@@ -893,7 +923,8 @@ extern "C" int cuna2_plan_set_schedule(cuna2_plan p, int log_tile, int grid_meth
   if (!schedule_ok(p, log_tile, grid_method))
     return fail(CUNA2_ERROR_INVALID_VALUE, "schedule (log_tile=%d, grid_method=%d) not admissible for ng=%lld m=%d",
                 log_tile, grid_method, (long long)p->ng, p->m);
-  if (log_tile != p->logTL || grid_method != p->grid_method) drop_graphs(p);
+  if (log_tile != p->logTL || grid_method != p->grid_method || p->cluster) drop_graphs(p);
+  p->cluster = false;  // the caller's schedule runs from here on
   p->logTL = log_tile;
   p->ntiles = (int)(p->ng >> log_tile);
   p->grid_method = grid_method;
@@ -958,12 +989,22 @@ extern "C" int cuna2_plan_autotune(cuna2_plan p, const double *t, const void *y,
     flush = nullptr;
   }
   int s = CUNA2_SUCCESS;
-  if (p->small) {  // the single-CTA path: no tiles to choose
+  bool best_cluster = false;
+  if (p->cluster && cluster_takes(p->geom.logL, n, 1)) {
+    s = time_schedule(p, t, y, F, n, t0, T, st, reps, flush, flush_bytes, &best);
+    best_cluster = !s;
+  }
+  p->cluster = false;
+  if (!s && p->small) {  // the single-CTA path: no tiles to choose
     const bool keep = p->tiled_single;
     p->tiled_single = false;
-    s = time_schedule(p, t, y, F, n, t0, T, st, reps, flush, flush_bytes, &best);
+    float ms = 0;
+    s = time_schedule(p, t, y, F, n, t0, T, st, reps, flush, flush_bytes, &ms);
     p->tiled_single = keep;
-    best_tiled = false;
+    if (!s && ms < best) {
+      best = ms;
+      best_tiled = best_cluster = false;
+    }
   }
   if (!s && (!p->small || p->has_split)) {  // tiled schedules
     p->tiled_single = true;
@@ -984,6 +1025,7 @@ extern "C" int cuna2_plan_autotune(cuna2_plan p, const double *t, const void *y,
             best_method = method;
             best_bin = bin;
             best_tiled = true;
+            best_cluster = false;
           }
         }
   }
@@ -993,6 +1035,7 @@ extern "C" int cuna2_plan_autotune(cuna2_plan p, const double *t, const void *y,
   p->grid_method = best_method;
   p->binning = best_bin;
   p->tiled_single = best_tiled;
+  p->cluster = best_cluster;
   if (flush) {
     cudaStreamSynchronize(st);
     cudaFree(flush);

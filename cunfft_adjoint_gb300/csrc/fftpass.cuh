@@ -37,6 +37,43 @@ struct CtNoDst {
   template <int R, int LOGNS, typename C> __device__ void store(int, int, C *) const {}
 };
 
+// Outputs of the CTA's transformed rows in s: the real unpack, deconvolution and
+// centring of every k = k1 + L1 k2 <= K, to Fs[0 .. nf).
+// A thread keeps one row (the CTA's threads are a multiple of its 2P = B
+// rows) and steps through its outputs k = k1 + L1 k2 <= K: the row's indices,
+// twiddle and partner are formed once, and the columns beyond K cost nothing
+// (the pass is near its instruction issue, 94 per point; with half the outputs
+// skipped in a 16-step loop the bootstrap of 1024 x 2^15 points took 332 us,
+// 325 here).
+template <typename T, int LOG1, int LOG2, int LOGB, int THREADS>
+__device__ __forceinline__ void rowpass_outputs(const typename CxOf<T>::type *s, const typename CxOf<T>::type *twr,
+                                                const typename CxOf<T>::type *twc, int p0, const AccParams<T> &e,
+                                                typename CxOf<T>::type *Fs) {
+  typedef typename CxOf<T>::type C;
+  constexpr int L2 = 1 << LOG2, LOGP = LOGB - 1, P = 1 << LOGP, PITCH = fft_pitch(L2, 1 << LOGB);
+  const int i = threadIdx.x & (P - 1), half = (threadIdx.x >> LOGP) & 1;
+  const int p = p0 + i, k1 = ct_pair_row<LOG1>(p, half);
+  // Z[L - k] is in row (L1 - k1) mod L1: the slot's other row, or the same row
+  // for the self-paired rows 0 and L1/2 of slot 0
+  const C *zk = s + (half * P + i) * PITCH, *zm = s + (p == 0 ? half * P + i : (1 - half) * P + i) * PITCH;
+  const C tw1 = twr[2 * i + half];
+  const int mlast = k1 == 0 ? L2 : L2 - 1, K = (int)e.K;
+  const T c0 = e.c0, c1 = e.c1 * (T)1.4426950408889634;
+  C *Fp = Fs + K, *Fn = Fs + K;
+#pragma unroll 4
+  for (int k2 = threadIdx.x >> LOGB; k2 <= (K - k1) >> LOG1; k2 += THREADS >> LOGB) {
+    const int k = k1 + (k2 << LOG1), k2m = (mlast - k2) & (L2 - 1);
+    const C Zk = zk[cpad16(k2)], Zm = cconj(zm[cpad16(k2m)]);
+    // real unpack, deconvolution c0 exp2(c1 k^2) with the (-1)^k of the origin
+    const C G2 = cadd(cadd(Zk, Zm), cmul(cmul(tw1, twc[k2]), cmuli(csub(Zm, Zk))));
+    const T kf = (T)k;
+    const T sc = c0 * exp2_g(c1 * kf * kf);
+    const C Fk = cscale(G2, (k & 1) ? -sc : sc);
+    if (k < K) Fp[k] = Fk;
+    if (k >= 1) Fn[-k] = cconj(Fk);
+  }
+}
+
 // row-pair block `pblock` of one packed grid z; outputs Fs[0 .. nf)
 template <typename T, int LOGL, int LOGE = PassCfg<T>::LOGE>
 __device__ __forceinline__ void ct_rowpass_body(const typename CxOf<T>::type *slab, const FftDev<T> &f,
@@ -65,33 +102,7 @@ __device__ __forceinline__ void ct_rowpass_body(const typename CxOf<T>::type *sl
   pdl_wait();  // the rows come from the column pass
   CtPairSrc<T, LOG1, LOG2, LOGP> src{slab, p0};
   ct_fft<T, LOG2, LOGB, false, false, false>(s, f.tw2, src, CtNoDst());
-  // A thread keeps one row (the CTA's threads are a multiple of its 2P = B
-  // rows) and steps through its outputs k = k1 + L1 k2 <= K: the row's indices,
-  // twiddle and partner are formed once, and the columns beyond K cost nothing
-  // (the pass is near its instruction issue, 94 per point; with half the outputs
-  // skipped in a 16-step loop the bootstrap of 1024 x 2^15 points took 332 us,
-  // 325 here).
-  const int i = threadIdx.x & (P - 1), half = (threadIdx.x >> LOGP) & 1;
-  const int p = p0 + i, k1 = ct_pair_row<LOG1>(p, half);
-  // Z[L - k] is in row (L1 - k1) mod L1: the slot's other row, or the same row
-  // for the self-paired rows 0 and L1/2 of slot 0
-  const C *zk = s + (half * P + i) * PITCH, *zm = s + (p == 0 ? half * P + i : (1 - half) * P + i) * PITCH;
-  const C tw1 = twr[2 * i + half];
-  const int mlast = k1 == 0 ? L2 : L2 - 1, K = (int)e.K;
-  const T c0 = e.c0, c1 = e.c1 * (T)1.4426950408889634;
-  C *Fp = Fs + K, *Fn = Fs + K;
-#pragma unroll 4
-  for (int k2 = threadIdx.x >> LOGB; k2 <= (K - k1) >> LOG1; k2 += THREADS >> LOGB) {
-    const int k = k1 + (k2 << LOG1), k2m = (mlast - k2) & (L2 - 1);
-    const C Zk = zk[cpad16(k2)], Zm = cconj(zm[cpad16(k2m)]);
-    // real unpack, deconvolution c0 exp2(c1 k^2) with the (-1)^k of the origin
-    const C G2 = cadd(cadd(Zk, Zm), cmul(cmul(tw1, twc[k2]), cmuli(csub(Zm, Zk))));
-    const T kf = (T)k;
-    const T sc = c0 * exp2_g(c1 * kf * kf);
-    const C Fk = cscale(G2, (k & 1) ? -sc : sc);
-    if (k < K) Fp[k] = Fk;
-    if (k >= 1) Fn[-k] = cconj(Fk);
-  }
+  rowpass_outputs<T, LOG1, LOG2, LOGB, THREADS>(s, twr, twc, p0, e, Fs);
 }
 
 // three CTAs per SM for the short rows of many small grids (bootstrap), where

@@ -60,9 +60,14 @@ template <typename T> inline bool pass_few(int logL, int nslab, int part) {
 // CTA holds; 2^LOGNS points already transformed.  IN_G / OUT_G: the stage
 // reads from src / writes to dst instead of shared memory.  SEQ_FAST: thread
 // g takes sequence g mod 2^LOGS (else point-fastest).  FTW: every twiddle is
-// read from the table (see below).
-template <typename T, int R, int LOGN, int LOGNS, int LOGS, bool IN_G, bool OUT_G, bool SEQ_FAST, bool FTW, class Src,
-          class Dst>
+// read from the table (see below).  PART: the block has more threads than the
+// FFT, whose first THREADS call this and meet at a barrier of their own.
+template <int THREADS, bool PART> __device__ __forceinline__ void ct_barrier() {
+  if constexpr (PART) asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+  else __syncthreads();
+}
+template <typename T, int R, int LOGN, int LOGNS, int LOGS, bool IN_G, bool OUT_G, bool SEQ_FAST, bool FTW, bool PART,
+          class Src, class Dst>
 __device__ __forceinline__ void ct_stage(typename CxOf<T>::type *s, const typename CxOf<T>::type *__restrict__ tw,
                                          const Src &src, const Dst &dst) {
   typedef typename CxOf<T>::type C;
@@ -116,7 +121,7 @@ __device__ __forceinline__ void ct_stage(typename CxOf<T>::type *s, const typena
     }
     dftR<R>(v[u]);
   }
-  if ((!IN_G || in_smem<Src>::value) && (!OUT_G || in_smem<Dst>::value)) __syncthreads();
+  if ((!IN_G || in_smem<Src>::value) && (!OUT_G || in_smem<Dst>::value)) ct_barrier<THREADS, PART>();
 #pragma unroll
   for (int u = 0; u < NB; ++u) {
     const int g = threadIdx.x + u * THREADS;
@@ -131,35 +136,35 @@ __device__ __forceinline__ void ct_stage(typename CxOf<T>::type *s, const typena
       for (int r = 0; r < R; ++r) b[cpad16(r << LOGNS)] = v[u][r];
     }
   }
-  if (!OUT_G) __syncthreads();
+  if (!OUT_G) ct_barrier<THREADS, PART>();
 }
 
 // radix-16 stages from LOGNS on; the last one writes to dst when TO_GLOBAL
-template <typename T, int LOGN, int LOGS, int LOGNS, bool TO_GLOBAL, bool FSF, bool LSF, bool FTW, class Src,
+template <typename T, int LOGN, int LOGS, int LOGNS, bool TO_GLOBAL, bool FSF, bool LSF, bool FTW, bool PART, class Src,
           class Dst>
 __device__ __forceinline__ void ct_rest(typename CxOf<T>::type *s, const typename CxOf<T>::type *__restrict__ tw,
                                         const Src &src, const Dst &dst) {
   if constexpr (LOGNS + 4 >= LOGN) {
-    ct_stage<T, 16, LOGN, LOGNS, LOGS, false, TO_GLOBAL, TO_GLOBAL ? LSF : FSF, FTW>(s, tw, src, dst);
+    ct_stage<T, 16, LOGN, LOGNS, LOGS, false, TO_GLOBAL, TO_GLOBAL ? LSF : FSF, FTW, PART>(s, tw, src, dst);
   } else {
-    ct_stage<T, 16, LOGN, LOGNS, LOGS, false, false, FSF, FTW>(s, tw, src, dst);
-    ct_rest<T, LOGN, LOGS, LOGNS + 4, TO_GLOBAL, FSF, LSF, FTW>(s, tw, src, dst);
+    ct_stage<T, 16, LOGN, LOGNS, LOGS, false, false, FSF, FTW, PART>(s, tw, src, dst);
+    ct_rest<T, LOGN, LOGS, LOGNS + 4, TO_GLOBAL, FSF, LSF, FTW, PART>(s, tw, src, dst);
   }
 }
 
 // Src -> stages -> Dst (TO_GLOBAL) or -> shared memory s[seq*PITCH + pad16(k)]
 // followed by a barrier.  FSF / LSF: thread mapping of the loading stages /
 // of the storing stage.
-template <typename T, int LOGN, int LOGS, bool TO_GLOBAL, bool FSF, bool LSF, bool FTW = (sizeof(T) == 8), class Src,
-          class Dst>
+template <typename T, int LOGN, int LOGS, bool TO_GLOBAL, bool FSF, bool LSF, bool FTW = (sizeof(T) == 8),
+          bool PART = false, class Src, class Dst>
 __device__ __forceinline__ void ct_fft(typename CxOf<T>::type *s, const typename CxOf<T>::type *__restrict__ tw,
                                        const Src &src, const Dst &dst) {
   constexpr int R0L = (LOGN & 3) == 0 ? 4 : (LOGN & 3);
   if constexpr (R0L == LOGN) {
-    ct_stage<T, (1 << R0L), LOGN, 0, LOGS, true, TO_GLOBAL, TO_GLOBAL ? LSF : FSF, FTW>(s, tw, src, dst);
+    ct_stage<T, (1 << R0L), LOGN, 0, LOGS, true, TO_GLOBAL, TO_GLOBAL ? LSF : FSF, FTW, PART>(s, tw, src, dst);
   } else {
-    ct_stage<T, (1 << R0L), LOGN, 0, LOGS, true, false, FSF, FTW>(s, tw, src, dst);
-    ct_rest<T, LOGN, LOGS, R0L, TO_GLOBAL, FSF, LSF, FTW>(s, tw, src, dst);
+    ct_stage<T, (1 << R0L), LOGN, 0, LOGS, true, false, FSF, FTW, PART>(s, tw, src, dst);
+    ct_rest<T, LOGN, LOGS, R0L, TO_GLOBAL, FSF, LSF, FTW, PART>(s, tw, src, dst);
   }
 }
 

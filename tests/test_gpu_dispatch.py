@@ -227,3 +227,49 @@ def test_scan_of_many_tiles(mods, n, log_tile):
         return
     D = nfft.AdjointNFFT(nf, 2, 8, torch.float64)(t, y.float().double(), 0.0, T)
     assert rel_l2(F.cpu().numpy(), D.cpu().numpy()) < 2e-6
+
+
+@pytest.mark.parametrize("kind", ["uniform", "runs", "burst"])
+@pytest.mark.parametrize("n,nf,R,m", [(0, 1 << 12, 2, 8), (1, 1 << 12, 2, 1), (9, 1 << 13, 2, 16), (3001, 1 << 12, 4, 12),
+                                      (4097, 1 << 12, 8, 8), (9999, 1 << 14, 4, 5), (16384, 1 << 16, 2, 8),
+                                      (16384, 1 << 12, 2, 8), (16385, 1 << 14, 2, 8), (2049, 16, 4, 8), (2049, 1 << 11, 2, 16),
+                                      (16384, 1 << 9, 2, 3), (9000, 1 << 8, 8, 8), (8192, 1 << 14, 4, 8),
+                                      (8193, 1 << 14, 4, 8)])
+def test_short_series_in_one_cluster(mods, kind, n, nf, R, m):
+    """The whole short transform in one cluster launch, the grid's FFT spread
+    over its CTAs or, where it is small, in one (and one sample more, which
+    takes the tiled path): samples uniform, at the edges of the eight
+    CTAs' runs of cells and the period's seam, and all inside one run, whose
+    list then overflows for n > 4096 (grids of fewer than 16 cells per run: the
+    single-CTA path).  Against the double plan of the same
+    filter, one and three channels, and against the tiled path, which a chosen
+    schedule takes.  Tolerances: float rounding with 2^-22 per weight, 2e-6; a
+    burst adds up to n random terms per cell in sequence, eps sqrt(n), 2e-5."""
+    from cunfft_adjoint_gb300 import _lib
+    _, nfft = mods
+    rng = np.random.default_rng(n + m)
+    T, ng = 5.0, R * nf
+    if kind == "uniform":
+        pos = rng.uniform(0, ng, n)
+    elif kind == "runs":
+        pos = (ng // 8 * rng.integers(0, 8, n) + rng.uniform(-m - 1, m + 1, n)) % ng
+    else:
+        pos = 3 * ng // 8 + rng.uniform(0, 60, n)
+    tol = 2e-6 if kind == "uniform" else 2e-5
+    t = torch.as_tensor(pos / ng * T, device="cuda")
+    Y = torch.as_tensor(rng.normal(0, 1, (3, n)), device="cuda").float()
+    plan = nfft.AdjointNFFT(nf, R, m)
+    F = plan(t, Y[0].contiguous(), 0.0, T).clone()
+    if n == 0:
+        assert not F.abs().any()
+        return
+    M = plan.multi(t, Y, 0.0, T).clone()
+    plan.set_schedule(min(11, ng.bit_length() - 1), _lib.GRID_GATHER)
+    G = plan(t, Y[0].contiguous(), 0.0, T)
+    ref = nfft.AdjointNFFT(nf, R, m, torch.float64)
+    for c in range(3):
+        D = ref(t, Y[c].double(), 0.0, T).cpu().numpy()
+        assert rel_l2(M[c].cpu().numpy(), D) < tol
+        if c == 0:
+            assert rel_l2(F.cpu().numpy(), D) < tol
+            assert rel_l2(G.cpu().numpy(), D) < tol
