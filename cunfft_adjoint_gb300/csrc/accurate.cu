@@ -438,7 +438,11 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     return CUNA2_SUCCESS;
   }
   // bootstrap / channels: each CTA grids a group of slabs of one tile, reusing its staged records
-  const int group = wts ? std::min(8, nslab) : 1;
+  int group = wts ? std::min(8, nslab) : 1;
+  // slabs four at a time, their values fetched ahead: as many per CTA as leave
+  // each SM a dozen (a CTA sorts its tile's records once)
+  if (sizeof(T) == 4 && wts && p->grid_method == CUNA2_GRID_GATHER && p->logTL == 11 && !seg)
+    group = std::min(nslab, (int)std::min<int64_t>(32, std::max<int64_t>(8, (int64_t)ntiles * nslab / (12 * nsm) / 4 * 4)));
   const dim3 ggrid(ntiles, (nslab + group - 1) / group);
   // the chunk runs of a tile sit behind the form's own shared memory
   const size_t segb = seg ? sizeof(int) * (2 * (size_t)nch + 1) : 0;

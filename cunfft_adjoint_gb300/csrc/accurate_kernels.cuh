@@ -618,13 +618,31 @@ __device__ __forceinline__ void grid_slots(int p0, int ng, int TL, int m, int &s
   s1 = a >= 0 ? (b >= 0 ? b : c) : (b >= 0 ? c : -1);
 }
 
+// eight cells, 32-byte aligned, as one sector (two 16-byte stores of a thread
+// reach the L2 as half sectors)
+__device__ __forceinline__ void store8(float *p, const float *v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+// asynchronous copy of a 4-byte value to shared memory (zero unless `in`)
+__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // One grid tile [base, base + 2^logTL) from records [r0, r1), for slabs
 // [sbeg, send): slab s grids value wts[s*nvals + p] of sample p when wts is
 // given (bootstrap), else the record's own value.
 // CW consecutive cells per thread in the gather (4 or 8)
 // SG > 1 (slab weights given, CW = 8 on 2048-cell tiles): SG slabs share each
 // record's Gaussian, computed once per record visit and scaled by each slab's
-// value from shared memory.
+// value from shared memory.  Bound by the grid's writes and the latency of the
+// values' loads (1024 slabs of 2^16 cells, 5000 records, 268 MB: 117 us with
+// eight slabs per CTA and the values loaded between two barriers, 93 with 16
+// and copies one group ahead, 80 with 32-byte stores).
 template <typename T, int CW, class Src, int SG = 1, bool MASKED = true>
 __device__ __forceinline__ void grid_tile_body(const Src &recs, int r0, int r1,
                                                int base, T *__restrict__ grid, const AccParams<T> &e,
@@ -645,7 +663,8 @@ __device__ __forceinline__ void grid_tile_body(const Src &recs, int r0, int r1,
   int *start = reinterpret_cast<int *>(smem_raw);                                       // NG + 1 groups
   SRec<T> *srec = reinterpret_cast<SRec<T> *>(smem_raw + sizeof(int) * ((W + 2 + 3) & ~3));  // placed records
   int *sp = reinterpret_cast<int *>(srec + CAP);                                         // sample index
-  T *yv = reinterpret_cast<T *>(sp + CAP);  // SG > 1: yv[s * CAP + r], value of slab s for placed record r
+  // SG > 1: yv[s * CAP + r], value of slab s for placed record r, two buffers
+  T *yv = reinterpret_cast<T *>(sp + CAP);
   static_assert(SG == 1 || CW == 8, "slab groups run with 8-cell groups on 2048-cell tiles");
   __shared__ int wsum[kGridThreads / 32];
   // a single tile spanning the whole grid maps a record to up to two slots;
@@ -748,15 +767,31 @@ __device__ __forceinline__ void grid_tile_body(const Src &recs, int r0, int r1,
         for (int i = threadIdx.x; i < placed; i += kGridThreads) srec[i].y = ws[sp[i]];
         __syncthreads();
       }
-      if constexpr (SG > 1) {  // the group's values (0 past the last slab)
+      const T *yb = yv;
+      if constexpr (SG > 1) {
+        // the group's values (0 past the last slab): asynchronous copies, the
+        // next group's while this one's are gathered where the records stay
         const int placed = start[(W - 1) / CW];
+        auto fetch = [&](int first, T *dst) {
 #pragma unroll
-        for (int g = 0; g < SG; ++g) {
-          const T *ws = wts + (int64_t)(slab + g) * nvals;
-          for (int i = threadIdx.x; i < placed; i += kGridThreads)
-            yv[g * CAP + i] = slab + g < send ? ws[sp[i]] : (T)0;
+          for (int g = 0; g < SG; ++g) {
+            const bool in = first + g < send;
+            const T *ws = wts + (int64_t)(in ? first + g : sbeg) * nvals;
+            for (int i = threadIdx.x; i < placed; i += kGridThreads) cp_async4(dst + g * CAP + i, ws + sp[i], in);
+          }
+        };
+        if (nchunks > 1) {
+          fetch(slab, yv);
+          cp_async_wait();
+          __syncthreads();
+        } else {
+          const int odd = ((slab - sbeg) / SG) & 1;
+          if (slab == sbeg) fetch(slab, yv);
+          cp_async_wait();
+          __syncthreads();  // and the last group's gather is done with the other buffer
+          yb = yv + odd * SG * CAP;
+          if (slab + SG < send) fetch(slab + SG, yv + (1 - odd) * SG * CAP);
         }
-        __syncthreads();
       }
       // gather: the thread's cells cl0 .. cl0+CW-1 (local) take the records in
       // slots cl0 .. cl0 + CW - 1 + 2m - 1; record slot lc reaches cell c iff
@@ -797,7 +832,7 @@ __device__ __forceinline__ void grid_tile_body(const Src &recs, int r0, int r1,
             }
 #pragma unroll
             for (int g = 0; g < SG; ++g) {
-              const T yg = yv[g * CAP + r];
+              const T yg = yb[g * CAP + r];
 #pragma unroll
               for (int i = 0; i < CW; ++i) acc[g][i] = fma(yg, w[i], acc[g][i]);
             }
@@ -808,7 +843,7 @@ __device__ __forceinline__ void grid_tile_body(const Src &recs, int r0, int r1,
           for (int i = 0; i < CW; ++i) acc[0][CW * q + i] += a[0][i];
         }
       }
-      __syncthreads();
+      if (SG == 1 || nchunks > 1) __syncthreads();
     }
 #pragma unroll
     for (int g = 0; g < SG; ++g) {
@@ -820,10 +855,12 @@ __device__ __forceinline__ void grid_tile_body(const Src &recs, int r0, int r1,
         // TL is a power of two >= CW (gather tiles have >= 512 cells or span
         // the grid, ng >= 4m >= 4 and CW = 4 there), so groups are whole
         if (q < npass && cl0 < TL) {
+          if constexpr (CW == 8 && sizeof(T) == 4) store8(out + cl0, acc[g]);
+          else
 #pragma unroll
-          for (int i = 0; i < CW; i += 4)
-            store4(out + cl0 + i, acc[g][CW * q + i], acc[g][CW * q + i + 1], acc[g][CW * q + i + 2],
-                   acc[g][CW * q + i + 3]);
+            for (int i = 0; i < CW; i += 4)
+              store4(out + cl0 + i, acc[g][CW * q + i], acc[g][CW * q + i + 1], acc[g][CW * q + i + 2],
+                     acc[g][CW * q + i + 3]);
         }
       }
     }
@@ -1581,7 +1618,7 @@ template <typename T> size_t grid_smem_bytes(int logTL, int m, int sg = 1) {
   const int W = (1 << logTL) + 2 * m;
   const size_t CAP = GridCfg<T>::CAP;
   return sizeof(int) * ((W + 2 + 3) & ~3) + sizeof(SRec<T>) * CAP + sizeof(int) * CAP +
-         (sg > 1 ? sizeof(T) * sg * CAP : 0);
+         (sg > 1 ? 2 * sizeof(T) * sg * CAP : 0);
 }
 
 // Last four-step pass of the packed real transform: CTA owns row pairs
