@@ -325,7 +325,9 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     return fail(CUNA2_ERROR_UNSUPPORTED, "record inspection needs a tiled plan with the global binning form");
   mark(pr, "start", st);
   if (hook && !one) CUNA_TRY(hook->fn(hook->ctx, false));
-  if (nbs > 0) {
+  // the resamples' weights: before everything, or, where the series is sorted
+  // in one launch of eight CTAs, beside that launch
+  auto boot_weights = [&](bool beside) {
     static SetupFlag attrw;
     if (!setup_done(&attrw)) {
       CUNA_CK(cudaFuncSetAttribute(k_boot_weights<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -333,11 +335,15 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
       mark_setup_done(&attrw);
     }
     const bool sm = n <= kBootSmemN;
+    const size_t smb = sm ? sizeof(int) * (size_t)n : 0;
     if (!sm) CUNA_CK(cudaMemsetAsync(wts, 0, sizeof(T) * (size_t)n * nbs, st));
-    k_boot_weights<T><<<nbs, 1024, sm ? sizeof(int) * (size_t)n : 0, st>>>(y, (int)n, seed, wts);
+    if (beside) CUNA_CK(launch_pdl(k_boot_weights<T>, dim3(nbs), dim3(1024), smb, st, y, (int)n, seed, wts));
+    else k_boot_weights<T><<<nbs, 1024, smb, st>>>(y, (int)n, seed, wts);
     CUNA_CK(cudaGetLastError());
     mark(pr, "boot_weights", st);
-  }
+    return (int)CUNA2_SUCCESS;
+  };
+  if (nbs > 0 && !one) CUNA_TRY(boot_weights(false));
   if constexpr (sizeof(T) == 4) {
     if (clus) {
       const bool masked = !tail_free_gather(true, p->m, p->tau) || masked_gather_forced();
@@ -386,6 +392,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     CUNA_CK(cudaGetLastError());
     mark(pr, "bin_one", st);
     if (hook) CUNA_TRY(hook->fn(hook->ctx, true));
+    if (nbs > 0) CUNA_TRY(boot_weights(true));
   } else {
   // counts and cursor are adjacent: one memset zeroes both
   CUNA_CK(cudaMemsetAsync(counts, 0, o_off, st));

@@ -1685,6 +1685,7 @@ template <typename T>
 __global__ void __launch_bounds__(1024) k_boot_weights(const T *__restrict__ y, int n, unsigned seed,
                                                        T *__restrict__ wts) {
   extern __shared__ int cnt[];
+  pdl_trigger();
   const int b = blockIdx.x;
   T *w = wts + (int64_t)b * n;
   const unsigned s0 = seed + (unsigned)b * (unsigned)n;
@@ -1702,6 +1703,7 @@ __global__ void __launch_bounds__(1024) k_boot_weights(const T *__restrict__ y, 
       atomicAdd(&w[d], y[d]);
     }
   }
+  pdl_wait();  // a sort launched before runs beside this; who waits for this waits for both
 }
 
 // ---------------------------------------------------------------------------
