@@ -273,3 +273,27 @@ def test_short_series_in_one_cluster(mods, kind, n, nf, R, m):
         if c == 0:
             assert rel_l2(F.cpu().numpy(), D) < tol
             assert rel_l2(G.cpu().numpy(), D) < tol
+
+
+@pytest.mark.parametrize("m", [2, 8])
+@pytest.mark.parametrize("n,dense", [(1, False), (20_000, False), (20_000, True)])
+@pytest.mark.parametrize("chan", [2, 4, 5, 9, 33])
+def test_channels_in_groups(mods, chan, n, dense, m):
+    """Channels gridded four at a time, their values fetched a group ahead
+    (tiles of at most 1024 records) or per chunk of records (one dense tile):
+    full and partial groups, one and several per CTA, with and without tap
+    masks, against the double plan (float rounding, 2e-6; a dense tile adds up
+    to some 40 terms per cell, 4e-6)."""
+    _, nfft = mods
+    rng = np.random.default_rng(chan)
+    nf, T = 1 << 17, 2.0
+    pos = rng.uniform(0, 1, n)
+    if dense:
+        pos[: n // 2] = 0.4 + pos[: n // 2] * 0.004
+    t = torch.as_tensor(pos * T, device="cuda")
+    Y = torch.as_tensor(rng.normal(0, 1, (chan, n)), device="cuda").float()
+    M = nfft.AdjointNFFT(nf, 2, m).multi(t, Y, 0.0, T)
+    ref = nfft.AdjointNFFT(nf, 2, m, torch.float64)
+    for c in {0, 1, chan // 2, chan - 1}:
+        D = ref(t, Y[c].double(), 0.0, T)
+        assert rel_l2(M[c].cpu().numpy(), D.cpu().numpy()) < (4e-6 if dense else 2e-6)
