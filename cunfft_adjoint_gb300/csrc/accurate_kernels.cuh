@@ -299,7 +299,7 @@ __global__ void __cluster_dims__(kBinOneCtas, 1, 1) __launch_bounds__(kBinOneThr
     const int nt = sample_tiles(cell, smp.e, t);
     typename RecOf<T>::type r;
     rec_set(r, cell, fr, smp.y[i], i);
-    for (int q = 0; q < nt; ++q) recs[atomicAdd(&cur[t[q]], 1)] = r;
+    for (int q = 0; q < nt; ++q) rec_store(recs + atomicAdd(&cur[t[q]], 1), r);
   }
   cluster_barrier();  // no CTA leaves while another may read its histogram
 }

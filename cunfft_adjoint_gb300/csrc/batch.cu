@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(512) k_bscatter(const double *__restrict__ t, 
     smp.prep(i, raw[k], p);
     for (int q = 0; q < p.nt; ++q) {
       const int u = p.t[q];
-      recs[lbase[u] + atomicAdd(&lc[u], 1)] = p.rec;
+      rec_store(recs + lbase[u] + atomicAdd(&lc[u], 1), p.rec);
     }
   }
 }

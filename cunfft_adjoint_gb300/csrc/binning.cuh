@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(512) k_bin_scatter(S smp, const int *__restric
   for (int it = 0; it < kScatterItems; ++it)
     for (int q = 0; q < p[it].nt; ++q) {
       const int pos = sm ? lbase[p[it].t[q]] + rk[it][q] : rk[it][q];
-      recs[pos] = p[it].rec;
+      rec_store(recs + pos, p[it].rec);
     }
 }
 
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(512) k_bin_scatter_resv(S smp, const int *coun
       smp.prep(i, raw[it], p);
       for (int q = 0; q < p.nt; ++q) {
         const int t = p.t[q];
-        recs[base[t] + atomicAdd(&lc[t], 1)] = p.rec;
+        rec_store(recs + base[t] + atomicAdd(&lc[t], 1), p.rec);
       }
     }
   }
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(512) k_bin_local(S smp, typename S::Rec *__res
   for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
     Prep<Rec> p;
     smp.prep(i, smp.load(i, true), p);
-    for (int q = 0; q < p.nt; ++q) out[atomicAdd(&cur[p.t[q]], 1)] = p.rec;
+    for (int q = 0; q < p.nt; ++q) rec_store(out + atomicAdd(&cur[p.t[q]], 1), p.rec);
   }
 }
 
