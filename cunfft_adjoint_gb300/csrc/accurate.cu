@@ -522,7 +522,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
         if constexpr (sizeof(T) == 8) {
           few = (int64_t)ggrid.x * ggrid.y < 2 * nsm;
           if (few)
-            le = launch_pdl(k_grid_fixed<T, 1024>, ggrid, dim3(1024), grid_fixed_smem_bytes<T, 1024>(p->logTL, p->m), st,
+            le = launch_pdl(k_grid_fixed<T, 1024>, ggrid, dim3(1024), grid_fixed_smem_bytes<T, 1024>(p->logTL, p->m, !wts), st,
                             rc, oc, grid, e, wc, nv, nslab, group, sstr, dfgrid);
         }
         if (!few)

@@ -1005,6 +1005,15 @@ __global__ void __launch_bounds__(kGridThreads, sizeof(T) == 4 ? 6 : 3) k_grid_s
 // is bit-reproducible run to run.  A non-finite value makes its tiles NaN.
 // records [c0, c0 + cnt) -> srec (values from ws when given); returns the
 // thread's max |value| (NaN once one is not finite)
+// max(ym, |v|), NaN once a value was not finite (double: |v| to 2^-23 below,
+// without the conversions of the FP64 pipe; the tile's range has room for it)
+__device__ __forceinline__ float value_bound(float ym, float v) {
+  return isfinite(v) && !isnan(ym) ? fmaxf(ym, fabsf(v)) : __int_as_float(0x7fffffff);
+}
+__device__ __forceinline__ float value_bound(float ym, double v) {
+  const bool finite = (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
+  return finite && !isnan(ym) ? fmaxf(ym, fabsf(df_from_double(v).hi)) : __int_as_float(0x7fffffff);
+}
 template <typename T, int NT> __host__ __device__ constexpr int fixed_cap() { return GridCfg<T>::CAP > NT ? GridCfg<T>::CAP : NT; }
 template <typename T, int NT, class Src>
 __device__ __forceinline__ float fixed_stage(const Src &recs, int c0, int cnt,
@@ -1019,7 +1028,7 @@ __device__ __forceinline__ float fixed_stage(const Src &recs, int c0, int cnt,
     r.lc = rc.cell - base;
     r.pad = rc.p;
     srec[i] = r;
-    ym = isfinite(r.y) && !isnan(ym) ? fmaxf(ym, (float)fabs(r.y)) : __int_as_float(0x7fffffff);
+    ym = value_bound(ym, r.y);
   }
   return ym;
 }
@@ -1147,6 +1156,10 @@ __device__ __forceinline__ void tap_fix(float p, float e, int &h, int &l) {
   l = __float2int_rn(fmaf((float)h, -0x1p20f, p) + e);
 }
 
+struct TapConst {  // the exponent constants in float-float
+  dfl k1, k2;
+  __device__ explicit TapConst(const AccParams<double> &e) : k1(df_from_double(e.k1)), k2(df_from_double(e.k2)) {}
+};
 // Double: the taps d = k and d = -k of a record as one packed pair in
 // float-float (about 48 bits, below the 2^-50 quantum's reach only where a tap
 // is far below its tile's bound), E Q^k and E Q^-k by running products with the
@@ -1154,32 +1167,20 @@ __device__ __forceinline__ void tap_fix(float p, float e, int &h, int &l) {
 // pipe.  13 packed operations per pair of taps and 9 scalar ones per tap to
 // split it into the two words, where scalar products and a 64-bit integer took
 // 60 per tap (1e6 samples on 2^22 cells: 120 -> 80 us, flushing float-float
-// cells included).
+// cells included; 71 with unstaged records and the scale's divisions by one
+// warp).
 template <class Add>
-__device__ __forceinline__ void fixed_taps_df(const SRec<double> *srec, int cnt, double sc, const AccParams<double> &e,
-                                              const ulonglong2 *cw, const Add &add, int TL, int gmask, int nthr) {
-  const int m = e.m;
-  const dfl k1w = df_from_double(e.k1), k2w = df_from_double(e.k2);  // the exponent constants
+__device__ __forceinline__ void fixed_taps_df(double y, double f, int p0, double sc, const TapConst &tc, int m,
+                                              const ulonglong2 *cw, const Add &add, int TL, int gmask) {
   const f2 m1 = pk2(-1.0f, -1.0f);
-  auto tap = [&](int c, float p, float r) {
-    c &= gmask;
-    if (c < TL) {
-      int h, l;
-      tap_fix(p, r, h, l);
-      add(c, h, l);
-    }
-  };
-#pragma unroll 1
-  for (int i = threadIdx.x; i < cnt; i += nthr) {
-    const SRec<double> q = srec[i];
-    const dfl fw = df_from_double(q.f);
-    // E = y sc 2^(-k1 f^2), Q = 2^(k2 f), 1/Q
-    const dfl E = df_from_double(q.y * sc) * df_exp2(-(k1w * fw * fw));
-    const dfl Q = df_exp2(k2w * fw), Qi = df_rcp(Q);
-    const int p0 = q.lc;
+  const dfl fw = df_from_double(f);
+  // E = y sc 2^(-k1 f^2), Q = 2^(k2 f), 1/Q
+  const dfl E = df_from_double(y * sc) * df_exp2(-(tc.k1 * fw * fw));
+  const dfl Q = df_exp2(tc.k2 * fw), Qi = df_rcp(Q);
+  const f2 Qh = pk2(Q.hi, Qi.hi), Ql = pk2(Q.lo, Qi.lo), nQh = mul2(Qh, m1);
+  f2 Uh = pk2(E.hi, E.hi), Ul = pk2(E.lo, E.lo);
+  auto taps = [&](auto tap) {
     tap(p0, E.hi, E.lo);
-    const f2 Qh = pk2(Q.hi, Qi.hi), Ql = pk2(Q.lo, Qi.lo), nQh = mul2(Qh, m1);
-    f2 Uh = pk2(E.hi, E.hi), Ul = pk2(E.lo, E.lo);
 #pragma unroll 2
     for (int k = 1; k <= m; ++k) {
       {  // U <- U Q: float-float product, renormalised
@@ -1197,6 +1198,22 @@ __device__ __forceinline__ void fixed_taps_df(const SRec<double> *srec, int cnt,
       tap(p0 + k, ph, rh);
       if (k < m) tap(p0 - k, pl, rl);
     }
+  };
+  if (p0 - m + 1 >= 0 && p0 + m < TL) {  // every tap inside the tile
+    taps([&](int c, float p, float r) {
+      int h, l;
+      tap_fix(p, r, h, l);
+      add(c, h, l);
+    });
+  } else {  // near the tile edge: wrap, keep the taps inside the tile
+    taps([&](int c, float p, float r) {
+      c &= gmask;
+      if (c < TL) {
+        int h, l;
+        tap_fix(p, r, h, l);
+        add(c, h, l);
+      }
+    });
   }
 }
 
@@ -1224,10 +1241,14 @@ __device__ __forceinline__ void tile_taps(bool split, const SRec<T> *srec, int c
                                           const void *cd, typename FixAcc<T>::type *acc, int TL, int gmask) {
   if constexpr (sizeof(T) == 8) {
     const ulonglong2 *cw = static_cast<const ulonglong2 *>(cd);
-    if (split)
-      fixed_taps_df(srec, cnt, sc, e, cw, SplitAdd{reinterpret_cast<int *>(acc), reinterpret_cast<unsigned *>(acc) + TL},
-                    TL, gmask, NT);
-    else fixed_taps_df(srec, cnt, sc, e, cw, WideAdd{acc}, TL, gmask, NT);
+    const TapConst tc(e);
+    const SplitAdd sa{reinterpret_cast<int *>(acc), reinterpret_cast<unsigned *>(acc) + TL};
+#pragma unroll 1
+    for (int i = threadIdx.x; i < cnt; i += NT) {
+      const SRec<double> q = srec[i];
+      if (split) fixed_taps_df(q.y, q.f, q.lc, sc, tc, e.m, cw, sa, TL, gmask);
+      else fixed_taps_df(q.y, q.f, q.lc, sc, tc, e.m, cw, WideAdd{acc}, TL, gmask);
+    }
   } else {
 #pragma unroll 1
     for (int i = threadIdx.x; i < cnt; i += NT)
@@ -1331,8 +1352,8 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
   A *acc = reinterpret_cast<A *>(smem_raw);                                  // TL cells
   SRec<T> *srec = reinterpret_cast<SRec<T> *>(smem_raw + sizeof(A) * TL);    // CAP staged records
   // coefficients exp2(-k1 d^2): float d = 1..m; double d = 0..m, packed float-float
-  // (float tiles of one slab of the records' own values stage none)
-  constexpr bool kOwn = sizeof(T) == 4 && !std::is_same<Src, SegSrc<T>>::value;
+  // (tiles of one slab of the records' own values stage none)
+  constexpr bool kOwn = !std::is_same<Src, SegSrc<T>>::value;
   const bool own = kOwn && !wts && sbeg + 1 == send;
   void *cd = own ? srec : srec + CAP;
   int *hist = reinterpret_cast<int *>(static_cast<char *>(cd) + kTapCoefBytes);  // NB buckets
@@ -1357,6 +1378,7 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
       // staging (bound by the shared-memory pipe, of which the staging and a
       // coefficient read per tap were a quarter: 64 series of 2e5 samples, m =
       // 10: 224 -> 166 us; 5.4e8 cells, 5.8e7 samples, m = 8: 1107 -> 1044 us).
+      typedef typename RecOf<T>::type Rec;
       constexpr int KEEP = 2;
       const int cnt = r1 - r0;
       fixed_clear<NT>(acc, TL);
@@ -1367,13 +1389,13 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
       // returned; many: the buckets are read back (an atomic that returns
       // nothing is cheaper where a warp's samples share a bucket)
       const bool few = cnt <= 4 * NT;
-      auto see = [&](const RecF &r) {
+      auto see = [&](const Rec &r) {
         int *h = &hist[((r.cell - base + m) & gmask) >> logBS];
         if (few) hm = max(hm, atomicAdd(h, 1) + 1);
         else atomicAdd(h, 1);
-        ym = isfinite(r.b) && !isnan(ym) ? fmaxf(ym, fabsf(r.b)) : __int_as_float(0x7fffffff);
+        ym = value_bound(ym, r.b);
       };
-      RecF rc[KEEP], nx[KEEP];
+      Rec rc[KEEP], nx[KEEP];
 #pragma unroll
       for (int k = 0; k < KEEP; ++k)
         if (threadIdx.x + k * NT < cnt) rc[k] = recs[r0 + threadIdx.x + k * NT];
@@ -1406,25 +1428,55 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
       int hmax = 0;
 #pragma unroll
       for (int w = 0; w < NT / 32; ++w) hmax = max(hmax, redi[w]);
-      const float sc = fixed_scale<float, NT>(red, hmax);
-      if (sc > 0.f) {
-        const float *c = static_cast<const float *>(cd);
-        RecF r = rc[0];
+      T sc, inv;
+      auto scale = [&] {
+        sc = fixed_scale<T, NT>(red, hmax);
+        inv = sc > (T)0 ? (T)1 / sc : (sc == sc ? (T)0 : sc);
+      };
+      if constexpr (sizeof(T) == 4) {
+        scale();
+      } else {  // two FP64 divisions, by one warp: all of them would fill the FP64 pipe
+        __shared__ T scale_i;
+        if (warp == 0) {
+          scale();
+          if (lane == 0) {
+            scale_s = sc;
+            scale_i = inv;
+          }
+        }
+        __syncthreads();
+        sc = scale_s;
+        inv = scale_i;
+      }
+      const bool split = sizeof(T) == 8 && hmax <= kSplitMaxH;
+      auto each = [&](auto taps) {
+        Rec r = rc[0];
 #pragma unroll 1
         for (int i = threadIdx.x; i < cnt; i += NT) {
-          RecF n = rc[1];  // the next one, on its way
+          Rec n = rc[1];  // the next one, on its way
           if (i >= NT && i + NT < cnt) n = recs[r0 + i + NT];
-          fixed_taps(r.b, r.a, r.cell - base, sc, e, c, acc, TL, gmask);
+          taps(r);
           r = n;
+        }
+      };
+      if (sc > (T)0) {
+        if constexpr (sizeof(T) == 4) {
+          const float *c = static_cast<const float *>(cd);
+          each([&](const Rec &r) { fixed_taps(r.b, r.a, r.cell - base, sc, e, c, acc, TL, gmask); });
+        } else {
+          const ulonglong2 *cw = static_cast<const ulonglong2 *>(cd);
+          const TapConst tc(e);
+          const SplitAdd sa{reinterpret_cast<int *>(acc), reinterpret_cast<unsigned *>(acc) + TL};
+          if (split) each([&](const Rec &r) { fixed_taps_df(r.b, r.a, r.cell - base, sc, tc, m, cw, sa, TL, gmask); });
+          else each([&](const Rec &r) { fixed_taps_df(r.b, r.a, r.cell - base, sc, tc, m, cw, WideAdd{acc}, TL, gmask); });
         }
       }
       __syncthreads();
-      const float inv = sc > 0.f ? 1.f / sc : (sc == sc ? 0.f : sc);
-      tile_flush<T, NT>(false, acc, TL, inv, grid + (int64_t)sbeg * slab_stride + base, false);
+      tile_flush<T, NT>(split, acc, TL, inv, grid + (int64_t)sbeg * slab_stride + base, dfout);
       return;
     }
   }
-  if (!wts && sbeg + 1 == send && nchunks <= 1) {
+  if (!kOwn && !wts && sbeg + 1 == send && nchunks <= 1) {
     // One slab of the records' own values, one staging chunk: a single read
     // of the records stages them, builds the histogram and bounds |value|;
     // the largest bucket count is the largest count an atomic returned.
@@ -1450,7 +1502,7 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
       r.pad = rc[k].p;
       srec[i] = r;
       hm = max(hm, atomicAdd(&hist[((rc[k].cell - base + m) & gmask) >> logBS], 1) + 1);
-      ym = isfinite(r.y) && !isnan(ym) ? fmaxf(ym, (float)fabs(r.y)) : __int_as_float(0x7fffffff);
+      ym = value_bound(ym, r.y);
     }
     for (int o = 16; o > 0; o >>= 1) {
       const float u = __shfl_xor_sync(0xffffffffu, ym, o);
@@ -1497,7 +1549,7 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
 #pragma unroll 1
       for (int i = r0 + threadIdx.x; i < r1; i += NT) {
         const T v = ws ? ws[recs[i].p] : recs[i].b;
-        ym = isfinite(v) && !isnan(ym) ? fmaxf(ym, (float)fabs(v)) : __int_as_float(0x7fffffff);
+        ym = value_bound(ym, v);
       }
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -1529,7 +1581,7 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
 
 // NT = 256, or 1024 for double launches that do not give every SM two tiles
 // (one transform of 2^19 cells is 128 tiles of 4096: 54 us with eight warps per
-// SM and scalar taps, 28 us here).
+// SM and scalar taps, 23 us here).
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT, NT > 256 ? 1 : (sizeof(T) == 4 ? 6 : 4)) k_grid_fixed(
     const typename RecOf<T>::type *recs, const int *off, T *grid, AccParams<T> e, const T *wts, int64_t nvals,
@@ -1543,12 +1595,12 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : (sizeof(T) == 4 ? 6 : 4)) k
                                                          grid, e, wts, nvals, sbeg, send, slab_stride, dfout);
 }
 
-// own: float tiles of one slab of the records' own values, which stage no records
+// own: tiles of one slab of the records' own values, which stage no records
 template <typename T, int NT = kGridThreads> size_t grid_fixed_smem_bytes(int logTL, int m, bool own = false) {
   int logBS = 4;
   while ((1 << logBS) < 2 * m) ++logBS;
   const size_t NB = ((((size_t)1 << logTL) + 2 * m) >> logBS) + 1;
-  const size_t staged = own && sizeof(T) == 4 ? 0 : (size_t)fixed_cap<T, NT>();
+  const size_t staged = own ? 0 : (size_t)fixed_cap<T, NT>();
   return sizeof(typename FixAcc<T>::type) * ((size_t)1 << logTL) + sizeof(SRec<T>) * staged +
          kTapCoefBytes + sizeof(int) * NB;
 }
