@@ -12,15 +12,19 @@
 // are fused in.
 //
 // Precision: s_j is reduced in 64-bit fixed point (phase.cuh); gridding, FFT
-// and epilogue run in the plan's type.  The single-CTA path uses the fast
-// Gaussian gridding factorisation y E1 E2^d E3[d] (E2^d by repeated
-// multiplication); the tiled path evaluates each tap (float) or factorises
-// per four taps (double).
+// and epilogue run in the plan's type, double plans' tiled gridding and
+// four-step passes in float-float.  Taps come from the fast Gaussian gridding
+// factorisation (Greengard & Lee 2004): running products about a record's own
+// cell (fixed point, single-CTA double) or about a group of four or eight
+// cells (gather).
 //
 // Kernels:
 //   k_nfft_small<T>      ng <= 2^15 (f32) / 2^14 (f64): one CTA per transform,
-//                        gridding straight into shared memory (no sort), FFT,
-//                        epilogue -- a single launch.
+//                        gridding in shared memory (float: sorted there and
+//                        gathered), FFT, epilogue -- a single launch.
+//   k_nfft_cluster       a short float transform in one launch of an eight-CTA
+//                        cluster (cluster.cuh).
+//   k_bin_one            the sort of a short series in one cluster launch.
 //   binning (binning.cuh) + k_grid_scatter / k_grid_acc (the plan's schedule)
 //                        + k_ct_colpass + k_ct_rowpass_acc (fftpass.cuh,
 //                        compile-time geometry per length) for larger grids;

@@ -285,8 +285,10 @@ int cuna2_plan_time_grid(cuna2_plan plan, const double *t, const void *y, void *
  * All compute the same sums to rounding.  With more than one tile,
  * 2^log_tile >= 2m.
  * New plans start at (11, CUNA2_GRID_GATHER) for float and (12,
- * CUNA2_GRID_FIXED) for double (a grid of at most 8192 cells is one tile).  Changing the
- * schedule drops the plan's cached graphs.  No counterpart in the reference
+ * CUNA2_GRID_FIXED) for double (a grid of at most 8192 cells is one tile).
+ * Short float transforms (n <= 16384, R nf <= 2^16 cells; see cluster.cuh) run
+ * in one launch without tiles until a schedule is set or autotuned.  Changing
+ * the schedule drops the plan's cached graphs.  No counterpart in the reference
  * (its gridding kernel, src/gridding.cu:36-65, has a fixed launch shape). */
 enum { CUNA2_GRID_GATHER = 0, CUNA2_GRID_SCATTER = 1, CUNA2_GRID_FIXED = 2 };
 int cuna2_plan_set_schedule(cuna2_plan plan, int log_tile, int grid_method);
