@@ -399,7 +399,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
     if (nbs > 0) CUNA_TRY(boot_weights(true));
   } else {
   // counts and cursor are adjacent: one memset zeroes both
-  CUNA_CK(cudaMemsetAsync(counts, 0, o_off, st));
+  if (!resv) CUNA_CK(cudaMemsetAsync(counts, 0, o_off, st));
   if (resv) {
     // count (caching each sample's phase) and reserve, then scan + scatter
     SampAcc<T> smp{t, y, n, pm, e, phases};
@@ -410,8 +410,9 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
                                    (int)(sizeof(int) * (3 * kScanFuseTiles + 1))));
       mark_setup_done(&attrs);
     }
-    k_bin_count_resv<<<nrb, 512, sizeof(int) * ntiles, st>>>(smp, counts, rsv, ntiles, rspan);
-    CUNA_CK(cudaGetLastError());
+    k_zero_counts<<<(ntiles + 255) / 256, 256, 0, st>>>(counts, ntiles);
+    CUNA_CK(launch_pdl(k_bin_count_resv<SampAcc<T>>, dim3(nrb), dim3(512), sizeof(int) * ntiles, st, smp, counts, rsv,
+                       ntiles, rspan));
     mark(pr, "bin_count", st);
     CUNA_CK(launch_pdl(k_bin_scatter_resv<SampAccS<T>>, dim3(nrb), dim3(512), sizeof(int) * (3 * ntiles + 1), st, sms,
                        (const int *)counts, (const int *)rsv, offsets, recs, ntiles, rspan));

@@ -243,6 +243,16 @@ __device__ __forceinline__ void cta_exclusive_scan(const int *in, int *out, int 
 constexpr int kScanFuseTiles = 4096;  // 3 shared arrays of ntiles ints: 48 KB
 constexpr int kResvEntries = 1 << 22; // reservation table limit (ints)
 
+// counts[0, n) = 0 in front of k_bin_count_resv, which is launched as its
+// dependent and waits for it only before the reservations: after a memset and
+// its gap the counting starts 3 us later (1e6 samples, Nf = 2^20, float: 61.3 us
+// per call, 58.0 here).
+__global__ void k_zero_counts(int *counts, int n) {
+  pdl_trigger();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) counts[i] = 0;
+}
+
 template <class S>
 __global__ void __launch_bounds__(512) k_bin_count_resv(S smp, int *__restrict__ counts, int *__restrict__ resv,
                                                         int ntiles, int64_t span) {
@@ -273,6 +283,7 @@ __global__ void __launch_bounds__(512) k_bin_count_resv(S smp, int *__restrict__
     }
   }
   __syncthreads();
+  pdl_wait();  // counts are zero
   int res[TPT];
 #pragma unroll
   for (int k = 0; k < TPT; ++k) {

@@ -848,8 +848,8 @@ int compat_bin(const T *x, const T *y, int n, int ng, const typename FpOf<T>::ty
   const size_t smc = ntiles <= kBinSmemTiles ? sizeof(int) * ntiles : 0;
   const int gcount = (int)std::min<int64_t>((n + 4095) / 4096, 4 * sms);
   const int gscat = (int)((n + 512 * kScatterItems - 1) / (512 * kScatterItems));
-  CUNA_CK(cudaMemsetAsync(cw.counts, 0, sizeof(int) * ntiles, st));
   const int nrb = compat_resv_blocks(n, ntiles);
+  if (nrb <= 0) CUNA_CK(cudaMemsetAsync(cw.counts, 0, sizeof(int) * ntiles, st));
   if (nrb > 0) {
     // count + reserve, then scan + scatter without global atomics (binning.cuh)
     const int64_t span = resv_span(n, ntiles, device_sm_count());
@@ -863,14 +863,17 @@ int compat_bin(const T *x, const T *y, int n, int ng, const typename FpOf<T>::ty
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
       mark_setup_done(&attr);
     }
+    if (sizeof(T) == 4) k_zero_counts<<<(ntiles + 255) / 256, 256, 0, st>>>(cw.counts, ntiles);
+    else CUNA_CK(cudaMemsetAsync(cw.counts, 0, sizeof(int) * ntiles, st));  // plain launches follow
+    CUNA_CK(cudaGetLastError());
     if (boot) {
-      k_bin_count_resv<<<nrb, 512, sizeof(int) * ntiles, st>>>(sb, cw.counts, cw.resv, ntiles, span);
-      CUNA_CK(cudaGetLastError());
+      CUNA_CK(launch_compat<T>(k_bin_count_resv<SampCompat<T, true>>, dim3(nrb), dim3(512), sizeof(int) * ntiles, st, sb,
+                               cw.counts, cw.resv, ntiles, span));
       CUNA_CK(launch_pdl(k_bin_scatter_resv<SampCompat<T, true>>, dim3(nrb), dim3(512), sms3, st, sb,
                          (const int *)cw.counts, (const int *)cw.resv, cw.offsets, recs, ntiles, span));
     } else {
-      k_bin_count_resv<<<nrb, 512, sizeof(int) * ntiles, st>>>(sp, cw.counts, cw.resv, ntiles, span);
-      CUNA_CK(cudaGetLastError());
+      CUNA_CK(launch_compat<T>(k_bin_count_resv<SampCompat<T, false>>, dim3(nrb), dim3(512), sizeof(int) * ntiles, st, sp,
+                               cw.counts, cw.resv, ntiles, span));
       CUNA_CK(launch_pdl(k_bin_scatter_resv<SampCompat<T, false>>, dim3(nrb), dim3(512), sms3, st, sp,
                          (const int *)cw.counts, (const int *)cw.resv, cw.offsets, recs, ntiles, span));
     }
