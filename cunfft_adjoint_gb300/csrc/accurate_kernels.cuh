@@ -1256,23 +1256,44 @@ __device__ __forceinline__ void tile_taps(bool split, const SRec<T> *srec, int c
   }
 }
 
+// The flush's factor inv = 1 / scale as f 2^-50 p: 2^50 inv, the tile's bound, is
+// near the values themselves, where inv alone is 2^-50 of them and would leave
+// the float range long before they do.  p is a power of two, f a float-float in
+// [1, 2) (outside only where the bound is beyond the float range; 0 for an empty
+// tile, NaN for a non-finite value), so products with f lose nothing to
+// underflow and those with p round only where a cell leaves the float range.
+// (inv itself as a float-float: 9e-6 relative at values of 1e-26, all zero at
+// 1e-31.  One warp forms it for the CTA: 1e6 samples on 2^22 cells, the whole
+// transform 189.0 us as one float-float per thread, 188.2 here.)
+struct FlushScale {
+  dfl f;
+  float p;
+  FlushScale() = default;
+  __device__ explicit FlushScale(double inv) {
+    const int e = ((__double2hiint(inv) >> 20) & 0x7ff) - 1023 + 50, pe = min(max(e, -126), 127);
+    f = dfl(inv * __hiloint2double((1023 + 50 - pe) << 20, 0));
+    p = __int_as_float((127 + pe) << 23);
+  }
+};
 // Two cells h 2^20 + l (l < 2^32) times inv as one float-float complex value:
-// each integer as three exact floats (h rounded to 24 bits; the remainder with
-// l's high half; l's low half) added up, the product renormalised.
-__device__ __forceinline__ dcx fixed_pair_df(int h0, unsigned l0, int h1, unsigned l1, dfl inv) {
+// each integer, in units of 2^50, as three exact floats (h rounded to 24 bits;
+// the remainder with l's high half; l's low half) added up, the product
+// renormalised.
+__device__ __forceinline__ dcx fixed_pair_df(int h0, unsigned l0, int h1, unsigned l1, const FlushScale &inv) {
   const float f0 = (float)h0, f1 = (float)h1;
   const int r0 = h0 - (int)f0, r1 = h1 - (int)f1;  // |r| <= 64
-  const f2 a = mul2(pk2(f0, f1), pk2(0x1p20f, 0x1p20f));
-  const f2 b = mul2(pk2((float)(r0 * 16 + (int)(l0 >> 16)), (float)(r1 * 16 + (int)(l1 >> 16))), pk2(0x1p16f, 0x1p16f));
-  const f2 c = pk2((float)(l0 & 0xffffu), (float)(l1 & 0xffffu));
+  const f2 a = mul2(pk2(f0, f1), pk2(0x1p-30f, 0x1p-30f));
+  const f2 b = mul2(pk2((float)(r0 * 16 + (int)(l0 >> 16)), (float)(r1 * 16 + (int)(l1 >> 16))), pk2(0x1p-34f, 0x1p-34f));
+  const f2 c = mul2(pk2((float)(l0 & 0xffffu), (float)(l1 & 0xffffu)), pk2(0x1p-50f, 0x1p-50f));
   const f2 s = add2(a, b), v = sub2(s, a);
   const f2 e = add2(add2(sub2(a, sub2(s, v)), sub2(b, v)), c);
   const f2 xh = add2(s, e), xl = sub2(e, sub2(xh, s));
-  const f2 ih = pk2(inv.hi, inv.hi), p = mul2(xh, ih);
-  const f2 r = sub2(fma2(xl, ih, mul2(xh, pk2(inv.lo, inv.lo))), fma2(xh, pk2(-inv.hi, -inv.hi), p));
+  const f2 ih = pk2(inv.f.hi, inv.f.hi), p = mul2(xh, ih);
+  const f2 r = sub2(fma2(xl, ih, mul2(xh, pk2(inv.f.lo, inv.f.lo))), fma2(xh, pk2(-inv.f.hi, -inv.f.hi), p));
+  const f2 oh = add2(p, r), ol = sub2(r, sub2(oh, p)), pw = pk2(inv.p, inv.p);
   dcx o;
-  o.h = add2(p, r);
-  o.l = sub2(r, sub2(o.h, p));
+  o.h = mul2(oh, pw);
+  o.l = mul2(ol, pw);
   return o;
 }
 
@@ -1281,8 +1302,7 @@ __device__ __forceinline__ dcx fixed_pair_df(int h0, unsigned l0, int h1, unsign
 // where the double cells cost two FP64-pipe operations each here and as many
 // conversions in the column pass
 template <int NT>
-__device__ __forceinline__ void tile_flush_df(bool split, const long long *acc, int TL, double inv, double *out) {
-  const dfl iv(inv);
+__device__ __forceinline__ void tile_flush_df(bool split, const long long *acc, int TL, const FlushScale &iv, double *out) {
   ulonglong2 *o = reinterpret_cast<ulonglong2 *>(out);
   const int *hi = reinterpret_cast<const int *>(acc);
   const unsigned *lo = reinterpret_cast<const unsigned *>(acc) + TL;
@@ -1304,13 +1324,8 @@ __device__ __forceinline__ void tile_flush_df(bool split, const long long *acc, 
 
 // fixed-order flush of the tile: out[i] = cell i * inv (inv = 1 / scale)
 template <typename T, int NT>
-__device__ __forceinline__ void tile_flush(bool split, const typename FixAcc<T>::type *acc, int TL, T inv, T *out,
-                                           bool dfout) {
+__device__ __forceinline__ void tile_flush(bool split, const typename FixAcc<T>::type *acc, int TL, T inv, T *out) {
   if constexpr (sizeof(T) == 8) {
-    if (dfout) {
-      tile_flush_df<NT>(split, acc, TL, inv, out);
-      return;
-    }
     if (split) {
       const int *hi = reinterpret_cast<const int *>(acc);
       const unsigned *lo = reinterpret_cast<const unsigned *>(acc) + TL;
@@ -1344,6 +1359,7 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
   __shared__ float red[NT / 32];
   __shared__ int redi[NT / 32];
   __shared__ T scale_s;
+  __shared__ FlushScale flush_s;
   const int TL = 1 << e.logTL, m = e.m;
   const int gmask = (int)e.ng - 1;
   int logBS = 4;
@@ -1442,6 +1458,7 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
           if (lane == 0) {
             scale_s = sc;
             scale_i = inv;
+            if (dfout) flush_s = FlushScale(inv);
           }
         }
         __syncthreads();
@@ -1472,7 +1489,13 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
         }
       }
       __syncthreads();
-      tile_flush<T, NT>(split, acc, TL, inv, grid + (int64_t)sbeg * slab_stride + base, dfout);
+      T *out = grid + (int64_t)sbeg * slab_stride + base;
+      if constexpr (sizeof(T) == 8)
+        if (dfout) {
+          tile_flush_df<NT>(split, acc, TL, flush_s, out);
+          return;
+        }
+      tile_flush<T, NT>(split, acc, TL, inv, out);
       return;
     }
   }
@@ -1522,7 +1545,7 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
     if (sc > (T)0) tile_taps<T, NT>(split, srec, cnt, sc, e, cd, acc, TL, gmask);
     __syncthreads();
     const T inv = sc > (T)0 ? (T)1 / sc : (sc == sc ? (T)0 : sc);
-    tile_flush<T, NT>(split, acc, TL, inv, grid + (int64_t)sbeg * slab_stride + base, dfout);
+    tile_flush<T, NT>(split, acc, TL, inv, grid + (int64_t)sbeg * slab_stride + base);
     return;
   }
   __syncthreads();
@@ -1575,18 +1598,28 @@ __device__ __forceinline__ void grid_tile_fixed(const Src &recs, int r0, int r1,
     __syncthreads();
     // fixed-order flush: cell = integer / scale
     const T inv = sc > (T)0 ? (T)1 / sc : (sc == sc ? (T)0 : sc);
-    tile_flush<T, NT>(split, acc, TL, inv, grid + (int64_t)slab * slab_stride + base, dfout);
+    T *out = grid + (int64_t)slab * slab_stride + base;
+    if constexpr (sizeof(T) == 8)
+      if (dfout) {
+        tile_flush_df<NT>(split, acc, TL, FlushScale(inv), out);
+        continue;
+      }
+    tile_flush<T, NT>(split, acc, TL, inv, out);
   }
 }
 
 // NT = 256, or 1024 for double launches that do not give every SM two tiles
 // (one transform of 2^19 cells is 128 tiles of 4096: 54 us with eight warps per
 // SM and scalar taps, 23 us here).
+// These do not let the column pass launch before they end: its CTAs would all
+// start on the few SMs that have no tile, and how many do depends on the
+// cycle (2e5 samples, Nf = 2^18, forward: 67 us with an early launch, 71 with
+// the bound's exponent apart as above, 50 without).
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT, NT > 256 ? 1 : (sizeof(T) == 4 ? 6 : 4)) k_grid_fixed(
     const typename RecOf<T>::type *recs, const int *off, T *grid, AccParams<T> e, const T *wts, int64_t nvals,
     int nslab, int group, int64_t slab_stride, bool dfout) {
-  pdl_trigger();
+  if (NT == kGridThreads) pdl_trigger();
   pdl_wait();  // records and offsets come from the binning
   const int tile = blockIdx.x;
   const int sbeg = blockIdx.y * group, send = min(nslab, sbeg + group);

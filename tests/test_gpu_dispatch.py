@@ -297,3 +297,45 @@ def test_channels_in_groups(mods, chan, n, dense, m):
     for c in {0, 1, chan // 2, chan - 1}:
         D = ref(t, Y[c].double(), 0.0, T)
         assert rel_l2(M[c].cpu().numpy(), D.cpu().numpy()) < (4e-6 if dense else 2e-6)
+
+
+@pytest.mark.parametrize("e", [-86, -60, 60, 100])
+@pytest.mark.parametrize("n,nf,R,dense", [(300, 1 << 14, 2, False), (20_000, 1 << 17, 2, False), (60_000, 1 << 20, 4, False),
+                                          (20_000, 1 << 17, 2, True), (60_000, 1 << 20, 4, True)])
+def test_double_scales(mods, e, n, nf, R, dense):
+    """Double transforms do not depend on the scale of their values: F(2^e y) /
+    2^e against F(y), single, two channels and bootstrap; tiles of 1024 and of
+    256 threads, split sums and (dense: 5000 samples in one cell) 64-bit ones.
+    A power of two changes no rounding until a float-float pair's low part
+    falls below the float range: 2^-150 per operation, 2^-64 of values near
+    2^-86; its random sum over 2^22 cells and some 220 operations each,
+    deconvolved (7), is 1e-14 of one value, of spectra of sqrt(n) values 1e-15.
+    Bound: 1e-14."""
+    _, nfft = mods
+    rng = np.random.default_rng(n)
+    T, s = 3.0, 2.0 ** e
+    pos = rng.uniform(0, 1, n)
+    if dense:
+        pos[:5000] = (12345.0 + rng.uniform(0.1, 0.9, 5000)) / (R * nf)
+    t = torch.as_tensor(pos * T, device="cuda")
+    Y = torch.as_tensor(rng.normal(0, 1, (2, n)), device="cuda")
+    plan = nfft.AdjointNFFT(nf, R, 12, torch.float64)
+    for call in (lambda v: plan(t, v[0].contiguous(), 0.0, T), lambda v: plan.multi(t, v, 0.0, T),
+                 lambda v: plan.bootstrap(t, v[0].contiguous(), 2, 5, 0.0, T)):
+        F, G = call(Y).clone(), call(Y * s) / s
+        assert float((G - F).abs().square().sum().sqrt() / F.abs().square().sum().sqrt()) < 1e-14
+
+
+@pytest.mark.parametrize("e", [-86, -60, 60, 100])
+def test_double_lomb_scargle_scales(mods, e):
+    """The double periodogram of 2^e y is that of y: as above, but the weighted
+    values are 1 / n of the data, 2^-50 per operation at 2^-86 and n = 20000
+    (5000 frequencies, 2^16 cells): 2e-13.  Bound: 1e-12."""
+    from cunfft_adjoint_gb300.lombscargle import lomb_scargle
+    rng = np.random.default_rng(7)
+    n = 20_000
+    t = torch.as_tensor(np.sort(rng.uniform(0, 100.0, n)), device="cuda")
+    y = torch.as_tensor(np.sin(2 * np.pi * t.cpu().numpy() / 2.1) + rng.normal(0, 1, n), device="cuda")
+    dy = torch.as_tensor(rng.uniform(0.2, 0.6, n), device="cuda")
+    P, Q = (lomb_scargle(t, v, dy, nfreq=5000, df=1 / 500.0, t0=0.0, R=4, m=12) for v in (y, y * 2.0 ** e))
+    assert rel_l2(Q.cpu().numpy(), P.cpu().numpy()) < 1e-12
