@@ -354,8 +354,9 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
       const float *v = wts ? wts : y;
       const int logL = p->geom.logL;
       if (logL < kClusterLo) {
-        if (masked) CUNA_TRY(nfft_cluster_small<true>(logL, t, v, (int)n, pm, e, to_dev<T>(p->geom), F, nslab, st));
-        else CUNA_TRY(nfft_cluster_small<false>(logL, t, v, (int)n, pm, e, to_dev<T>(p->geom), F, nslab, st));
+        auto k = p->R >= 4 ? nfft_cluster_small<kGatherPoly>
+                           : (masked ? nfft_cluster_small<kGatherMasked> : nfft_cluster_small<kGatherFree>);
+        CUNA_TRY(k(logL, t, v, (int)n, pm, e, to_dev<T>(p->geom), F, nslab, st));
       } else {
         const FftDev<T> fc = to_dev<T>(p->geom_cl);
         if (masked) CUNA_TRY(nfft_cluster<true>(logL, t, v, (int)n, pm, e, fc, F, nslab, st));

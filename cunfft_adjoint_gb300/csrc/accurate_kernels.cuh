@@ -412,6 +412,57 @@ __device__ __forceinline__ void gauss_acc(T y, T x, T k1, const GaussCW<T, CW> &
   }
 }
 
+// 2^x of two values, -126 <= x <= 1, on the FP32 pipe: 2^n p(r), n the integer
+// nearest x, p the polynomial of degree 6 with the least maximal relative error
+// on [-1/2, 1/2] (weighted least squares, Lawson's iteration; 2e-9).  In floats
+// 8e-8 at most and 2.7e-8 rms, where ex2.approx has 2^-22.
+__device__ __forceinline__ void exp2_pair(f2 x, float &a, float &b) {
+  const f2 M = pk2(12582912.f, 12582912.f), t = add2(x, M), r = sub2(x, sub2(t, M));  // n in the low bits of t
+  f2 p = pk2(0x1.41d332p-13f, 0x1.41d332p-13f);
+  p = fma2(p, r, pk2(0x1.5f456ap-10f, 0x1.5f456ap-10f));
+  p = fma2(p, r, pk2(0x1.3b2dbcp-7f, 0x1.3b2dbcp-7f));
+  p = fma2(p, r, pk2(0x1.c6aed4p-5f, 0x1.c6aed4p-5f));
+  p = fma2(p, r, pk2(0x1.ebfbdap-3f, 0x1.ebfbdap-3f));
+  p = fma2(p, r, pk2(0x1.62e43p-1f, 0x1.62e43p-1f));
+  p = fma2(p, r, pk2(1.f, 1.f));
+  float t0, t1;
+  unpk2(t, t0, t1);
+  unpk2(p, a, b);
+  a = __int_as_float(__float_as_int(a) + (__float_as_int(t0) << 23));
+  b = __int_as_float(__float_as_int(b) + (__float_as_int(t1) << 23));
+}
+
+// a[i] += y exp2(-k1 (j + i - f)^2), i = 0..3, the weights one by one: j the
+// distance in cells of the first one from the record's own, f its fraction.
+// The transforms whose FFT one CTA holds gather with it: gauss_acc's powers of Q
+// carry the rounding of the middle cell's exponents, which beside their short
+// FFTs would show.  From R = 4 on, where three quarters of the FFT's error fall
+// outside the band, so would ex2.approx's, hence the polynomial there.
+// Relative error of the spectrum, mean of 32 series, by the scatter / gauss_acc
+// / ex2.approx per tap / polynomial: n = 1000, Nf = 2048, R = 2: 2.13 / 2.27 /
+// 1.97 / 1.93e-7; n = 300, Nf = 2048, R = 4, m = 12: 1.38 / 1.56 / 1.40 /
+// 1.24e-7; n = 700, Nf = 1024, R = 4, m = 6: 1.43 / 1.53 / 1.47 / 1.28e-7.
+enum GatherForm { kGatherMasked, kGatherFree, kGatherPoly };  // Poly: masked too (x < -126 outside the window)
+template <int FORM> __device__ __forceinline__ void gauss_acc4(float y, int j, float f, float k1, int m, float *a) {
+  const float fj = (float)j;
+  const f2 nf = pk2(-f, -f), nk = pk2(-k1, -k1);
+#pragma unroll
+  for (int i = 0; i < 4; i += 2) {
+    const f2 d = add2(pk2(fj + (float)i, fj + (float)(i + 1)), nf), x = mul2(mul2(nk, d), d);
+    float w0, w1;
+    if constexpr (FORM == kGatherPoly) {
+      exp2_pair(x, w0, w1);
+    } else {
+      float x0, x1;
+      unpk2(x, x0, x1);
+      w0 = exp2_g(x0);
+      w1 = exp2_g(x1);
+    }
+    a[i] = fmaf(FORM == kGatherFree || (unsigned)(m - j - i) < (unsigned)(2 * m) ? w0 : 0.f, y, a[i]);
+    a[i + 1] = fmaf(FORM == kGatherFree || (unsigned)(m - j - i - 1) < (unsigned)(2 * m) ? w1 : 0.f, y, a[i + 1]);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // single-CTA transform for small grids
 // ---------------------------------------------------------------------------
@@ -429,8 +480,8 @@ __device__ __forceinline__ void gauss_acc(T y, T x, T k1, const GaussCW<T, CW> &
 // 16 to 32 cells) 21 -> 11 us for 2^10-cell grids and 20 -> 18 us at 2^12
 // cells, but 29 -> 34 us at 2^13 and 114 -> 171 us at 2^15; a transform with an
 // SM to itself takes it to 2^14 cells.  One transform of n = 1000, Nf = 2048,
-// R = 2, m = 8: 28.7 us per call with L / 16 threads and the scatter, 14.1 us
-// here.
+// R = 2, m = 8: 28.7 us per call with L / 16 threads and the scatter, 10.3 us
+// here (by one cluster, cluster.cuh).
 inline bool small_gather(int L, bool alone, bool is_float) { return is_float && L <= (alone ? 8192 : 2048); }
 // records of a chunk (0: scatter).  With an SM to itself a transform takes the
 // most, fewer chunks of five barriers each; in a batch the shared memory of
@@ -438,6 +489,14 @@ inline bool small_gather(int L, bool alone, bool is_float) { return is_float && 
 // out to its idle threads: 2000 samples on 64 cells 160 us in chunks of 32,
 // 10.9 in one; 500 samples on 2^11 cells 6.1 either way.
 constexpr int kSmallCapMax = 2048;
+// Whether a series of n samples is gathered, where the launch has room for it:
+// from R = 4 on, whose weights are polynomials, in a batch only with as many
+// samples as packed points (1024 resamples of 200 samples, Nf = 1024, R = 4, m =
+// 12: 30 us by the scatter, 37 gathered; 4000 series of 300, Nf = 512: 67 and 73;
+// 1024 of 2000, Nf = 512: 127 and 104).
+__host__ __device__ inline bool small_gathers(int cap, int64_t n, int L, int64_t R) {
+  return cap > 0 && (cap == kSmallCapMax || R < 4 || n >= L);
+}
 inline int small_cap(int L, bool alone, bool is_float) {
   if (!small_gather(L, alone, is_float)) return 0;
   return alone ? kSmallCapMax : std::max(32, std::min(kSmallCapMax, L / 2));
@@ -460,10 +519,9 @@ template <typename T> int small_threads(int L, bool alone, int cap) {
 // the four cells of group g from the sorted records of one chunk, added to
 // a[]: records of the groups that hold cells 4g - m .. 4g + m + 2, whose
 // indices wrap around the periodic grid (images o = -1, 0, 1)
-template <bool MASKED>
+template <int FORM>
 __device__ __forceinline__ void small_gather4(const SRec<float> *srec, const int *order, const int *start, int g, int NG,
-                                              int ng, int m, float k1, const GaussCW<float, 4> &gw, int part, int step,
-                                              float *a) {
+                                              int ng, int m, float k1, int part, int step, float *a) {
   const int c0 = 4 * g;
   const int glo = (c0 - m) >> 2, ghi = (c0 + m + 2) >> 2;
 #pragma unroll 1
@@ -474,8 +532,7 @@ __device__ __forceinline__ void small_gather4(const SRec<float> *srec, const int
     const int re = start[hi + 1];
     for (int r = start[lo] + part; r < re; r += step) {
       const SRec<float> q = srec[order[r]];
-      const int dc = c - q.lc;
-      gauss_acc<float, 4, MASKED>(q.y, (float)dc - q.f, k1, gw, m - dc, 2 * m, a);
+      gauss_acc4<FORM>(q.y, c - q.lc, q.f, k1, m, a);
     }
   }
 }
@@ -484,9 +541,8 @@ __device__ __forceinline__ void small_grid_gather(const double *__restrict__ t, 
                                                   const PhaseMul &pm, const AccParams<float> &e, float *sr,
                                                   SRec<float> *srec, int *order, int *start, int cap) {
   const int ng = (int)e.ng, NG = ng / 4, m = e.m;
-  const GaussCW<float, 4> gw(e.k1);
   // as tail_free_gather: exp(-m^2 / (4 tau)) < 1e-8
-  const bool masked = e.k1 * (float)(m * m) < 26.6f;
+  const bool masked = e.k1 * (float)(m * m) < 26.6f, poly = e.ng >= 4 * e.nf;
   // Where there are fewer groups than threads, 2^LP threads share a group's
   // records (NG is a power of two: with LP > 0 either all threads have a group
   // or, at LP = 5, whole warps have none).
@@ -512,8 +568,9 @@ __device__ __forceinline__ void small_grid_gather(const double *__restrict__ t, 
     __syncthreads();
     for (int g = threadIdx.x >> LP; g < NG; g += blockDim.x >> LP) {
       float a[4] = {0.f, 0.f, 0.f, 0.f};
-      if (masked) small_gather4<true>(srec, order, start, g, NG, ng, m, e.k1, gw, part, step, a);
-      else small_gather4<false>(srec, order, start, g, NG, ng, m, e.k1, gw, part, step, a);
+      if (poly) small_gather4<kGatherPoly>(srec, order, start, g, NG, ng, m, e.k1, part, step, a);
+      else if (masked) small_gather4<kGatherMasked>(srec, order, start, g, NG, ng, m, e.k1, part, step, a);
+      else small_gather4<kGatherFree>(srec, order, start, g, NG, ng, m, e.k1, part, step, a);
       for (int o = 1; o < step; o <<= 1) {  // whole warps: see LP
 #pragma unroll
         for (int i = 0; i < 4; ++i) a[i] += __shfl_xor_sync(0xffffffffu, a[i], o);
@@ -540,7 +597,7 @@ __device__ __forceinline__ void nfft_small_body(const double *__restrict__ t, co
   const int pitch = fft_pitch(L, 1);
   C *s = reinterpret_cast<C *>(smem_raw);
   T *sr = reinterpret_cast<T *>(smem_raw);
-  if (sizeof(T) == 4 && cap) {
+  if (small_gathers(cap, n, L, e.ng / e.nf)) {
     if constexpr (sizeof(T) == 4) {
       SRec<float> *srec = reinterpret_cast<SRec<float> *>(smem_raw + ((sizeof(C) * pitch + 15) & ~(size_t)15));
       int *order = reinterpret_cast<int *>(srec + cap);
@@ -576,7 +633,7 @@ __device__ __forceinline__ void nfft_small_body(const double *__restrict__ t, co
     }
   }
   __syncthreads();
-  smem_fft<T, sizeof(T) == 4>(s, pitch, f.logL, 1, f.tw1);
+  smem_fft<T>(s, pitch, f.logL, 1, f.tw1);
   for (int64_t k = threadIdx.x; k <= e.K; k += blockDim.x) {
     const C Zk = s[pad16((int)(k & (L - 1)))];
     const C Zm = cconj(s[pad16((int)((L - k) & (L - 1)))]);

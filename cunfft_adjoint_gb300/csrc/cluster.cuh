@@ -15,7 +15,7 @@
 //      distributed shared memory and, twiddled, written to the CTAs that own
 //      their row pairs;
 //   4. row FFTs, unpack, deconvolution and centring, as ct_rowpass_body.
-// Grids of less than 2^12 points run phases 1 and 2 alike and leave the FFT to
+// Grids of less than 2^13 points run phases 1 and 2 alike and leave the FFT to
 // the first CTA.  n = 10000, Nf = 16384: 19.0 us -> 13.5; with the records
 // exchanged through device memory instead, after an exchange of counts, 16.5.
 // What bounds it is the latency of its phases: the samples' loads and the
@@ -28,7 +28,7 @@
 namespace cuna {
 namespace {
 
-constexpr int kClusterLo = 12, kClusterHi = 15;  // log2 of the packed length, FFT over the cluster
+constexpr int kClusterLo = 13, kClusterHi = 15;  // log2 of the packed length, FFT over the cluster
 constexpr int kClusterN = 16384;
 constexpr int kClusterCtas = 8, kClusterThreads = 512;
 constexpr int kClusterItems = kClusterN / kClusterCtas / kClusterThreads;  // samples per thread
@@ -37,21 +37,25 @@ constexpr int kClusterItems = kClusterN / kClusterCtas / kClusterThreads;  // sa
 constexpr int kClusterCap = kClusterCtas * kClusterThreads;
 constexpr int kClusterSlack = 64;  // places after the sorted list that a gather may read
 
-// grids of less than kClusterLo: the first CTA transforms the whole grid
-constexpr int kClusterSmallN = 1024;
+// Grids of less than 2^kClusterLo points: the first CTA transforms the whole
+// grid.  (2^12 points over the cluster take 2 us less, but its four-step FFT has
+// two more rounded products per point than the one-CTA FFT: 1.76e-7 of the
+// spectrum of n = 300, Nf = 2048, R = 4 against 1.38e-7.)
+constexpr int kClusterSmallN = 640, kClusterSmallN12 = 256;
 
 // a record touches at most two runs of ng/8 cells
 inline bool cluster_fits(int logL, int m) { return logL <= kClusterHi && logL >= 4 && (1 << (logL - 2)) >= 2 * m; }
 // Measured against the other paths (us; n samples, 2^L packed points).  Below
-// 2^12 points one CTA does it all in less while the samples are few, on the
-// device: n = 1000, 2^10: 7.2 against 7.8 here; 2000: 9.7 against 7.8; 10000,
-// 2^11: 47 against 12 per call.  Above, the tiled path, per call: n = 10000,
-// 2^14: 17.5 against 13.5 here; 2^15: n = 8000 17.8 against 16.4, n = 16384
-// 17.5 against 18.5; 2^16: n = 2000 17.5 against 18.5 -- eight SMs are too few
-// for the cells and samples from there on.
+// 2^13 points one CTA does it all in less while the samples are few, on the
+// device: 2^9 points: n = 600 8.0 against 8.1 here, 700 8.7 and 8.2; 2^11: 600
+// 9.0 and 8.9, 1000 10.3 and 9.1; 2^12: 200 11.0 and 11.0, 300 11.4 and 11.0;
+// 10000 samples, 2^11: 47 against 12 per call.  Above, the tiled path, per call:
+// n = 10000, 2^14: 17.5 against 13.5 here; 2^15: n = 8000 17.8 against 16.4, n =
+// 16384 17.5 against 18.5; 2^16: n = 2000 17.5 against 18.5 -- eight SMs are too
+// few for the cells and samples from there on.
 inline bool cluster_takes(int logL, int64_t n, int nslab) {
   return n <= kClusterN && nslab * kClusterCtas <= device_sm_count() &&
-         (logL < kClusterLo ? n > kClusterSmallN : (n << logL) <= (1 << 28));
+         (logL < kClusterLo ? n > (logL == 12 ? kClusterSmallN12 : kClusterSmallN) : (n << logL) <= (1 << 28));
 }
 
 template <int LOGL> struct ClusterCfg {
@@ -164,8 +168,8 @@ __device__ __forceinline__ void cluster_send(int LOGTC, const int *cell, const f
 // list[0, c) sorted by group of four cells, and the sums of the run's TC cells
 // into the tile (onto it unless first).  start: zeroed, NG + 1 group counts.
 // Where there are fewer groups than threads, 2^LP threads share a group's
-// records.
-template <bool MASKED>
+// records.  ONE >= 0: weights one by one, in that form (gauss_acc4).
+template <bool MASKED, int ONE>
 __device__ __forceinline__ void cluster_gather(int TC, const SRec<float> *list, SRec<float> *sorted, int *start, int c,
                                                int m, float k1, float *tile, bool first) {
   constexpr int TH = kClusterThreads, PER = kClusterCap / TH;
@@ -199,7 +203,8 @@ __device__ __forceinline__ void cluster_gather(int TC, const SRec<float> *list, 
     for (; r < re; r += step) {
       const SRec<float> nx = sorted[r + step];
       const int rel = q.lc - cl0;
-      gauss_acc<float, 4, MASKED>(q.y, (float)(m - rel) - q.f, k1, gw, rel, 2 * m, a);
+      if constexpr (ONE >= 0) gauss_acc4<ONE>(q.y, m - rel, q.f, k1, m, a);
+      else gauss_acc<float, 4, MASKED>(q.y, (float)(m - rel) - q.f, k1, gw, rel, 2 * m, a);
       q = nx;
     }
     for (int o = 1; o < step; o <<= 1) {  // a group's threads are in one warp
@@ -217,7 +222,7 @@ __device__ __forceinline__ void cluster_gather(int TC, const SRec<float> *list, 
 // Phases 1 and 2: this CTA's run of TC = 2^LOGTC cells of the grid of n samples
 // into its tile.  tables() runs while the records travel.  Ends without a
 // barrier.
-template <bool MASKED, class Tables>
+template <bool MASKED, int ONE, class Tables>
 __device__ __forceinline__ void cluster_grid(int LOGTC, const double *__restrict__ t, const float *__restrict__ y, int n,
                                              const PhaseMul &pm, const AccParams<float> &e, float *tile,
                                              unsigned char *work, const Tables &tables) {
@@ -252,7 +257,7 @@ __device__ __forceinline__ void cluster_grid(int LOGTC, const double *__restrict
   cluster_wait();
   const int over = threadIdx.x < NC ? cluster_load(&count, threadIdx.x) > kClusterCap : 0;
   if (!__syncthreads_or(over)) {
-    cluster_gather<MASKED>(TC, list, sorted, start, count, m, e.k1, tile, true);
+    cluster_gather<MASKED, ONE>(TC, list, sorted, start, count, m, e.k1, tile, true);
   } else {
     auto round = [&](auto it) {
       constexpr int IT = decltype(it)::value;
@@ -262,7 +267,7 @@ __device__ __forceinline__ void cluster_grid(int LOGTC, const double *__restrict
       cluster_barrier();
       cluster_send<IT, IT + 1>(LOGTC, cell, fr, yv, on, m, gmask, &count, list);
       cluster_barrier();
-      cluster_gather<MASKED>(TC, list, sorted, start, count, m, e.k1, tile, IT == 0);
+      cluster_gather<MASKED, ONE>(TC, list, sorted, start, count, m, e.k1, tile, IT == 0);
     };
     static_assert(kClusterItems == 4, "rounds");
     round(std::integral_constant<int, 0>());
@@ -290,7 +295,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
   F += (int64_t)blockIdx.y * e.nf;
   constexpr int LNS = last_logns<LOG1>(), P = G::B2 / 2;
   const int c0 = rank * G::B1, p0 = rank * P;
-  cluster_grid<MASKED>(G::LOGE + 1, t, y, n, pm, e, tile, work, [&] {
+  cluster_grid<MASKED, -1>(G::LOGE + 1, t, y, n, pm, e, tile, work, [&] {
     for (int i = threadIdx.x; i < 16 * G::B1; i += TH)
       steps[(i >> 4) * 17 + (i & 15)] = twiddle_L(f, (c0 + (i >> 4)) * ((i & 15) << LNS));
     for (int u = threadIdx.x; u < G::B2 + G::L2; u += TH) {
@@ -324,7 +329,7 @@ inline size_t cluster_small_smem(int logL) {
   return sizeof(float) * TC + sizeof(SRec<float>) * (2 * kClusterCap + kClusterSlack) +
          ((sizeof(int) * ((TC + 32) / 4 + 4) + 15) & ~(size_t)15) + sizeof(float2) * fft_pitch(1 << logL, 1);
 }
-template <bool MASKED>
+template <int FORM>
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
     k_nfft_cluster_small(const double *__restrict__ t, const float *__restrict__ y, int n, PhaseMul pm,
                          AccParams<float> e, FftDev<float> f, float2 *F) {
@@ -336,7 +341,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
                                          ((sizeof(int) * ((TC + 32) / 4 + 4) + 15) & ~(size_t)15));
   y += (int64_t)blockIdx.y * n;
   F += (int64_t)blockIdx.y * e.nf;
-  cluster_grid<MASKED>(LOGTC, t, y, n, pm, e, tile, work, [] {});
+  cluster_grid<FORM != kGatherFree, FORM>(LOGTC, t, y, n, pm, e, tile, work, [] {});
   __syncthreads();
   const int z0 = blockIdx.x << (LOGTC - 1);  // first packed point
   for (int i = threadIdx.x; i < TC / 2; i += kClusterThreads) {
@@ -346,23 +351,23 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
   }
   cluster_barrier();
   if (blockIdx.x != 0) return;
-  smem_fft<float, true>(s, pitch, f.logL, 1, f.tw1);
+  smem_fft<float>(s, pitch, f.logL, 1, f.tw1);
   for (int64_t k = threadIdx.x; k <= e.K; k += kClusterThreads) {
     const float2 Zk = s[pad16((int)(k & (L - 1)))];
     const float2 Zm = cconj(s[pad16((int)((L - k) & (L - 1)))]);
     acc_output<float>(e, k, Zk, Zm, F);
   }
 }
-template <bool MASKED>
+template <int FORM>
 int nfft_cluster_small(int logL, const double *t, const float *y, int n, const PhaseMul &pm, const AccParams<float> &e,
                        const FftDev<float> &f, float2 *F, int nslab, cudaStream_t st) {
   static SetupFlag attr;
   if (!setup_done(&attr)) {
-    CUNA_CK(cudaFuncSetAttribute(k_nfft_cluster_small<MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CUNA_CK(cudaFuncSetAttribute(k_nfft_cluster_small<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)cluster_small_smem(kClusterLo - 1)));
     mark_setup_done(&attr);
   }
-  k_nfft_cluster_small<MASKED>
+  k_nfft_cluster_small<FORM>
       <<<dim3(kClusterCtas, nslab), kClusterThreads, cluster_small_smem(logL), st>>>(t, y, n, pm, e, f, F);
   CUNA_CK(cudaGetLastError());
   return CUNA2_SUCCESS;
@@ -387,7 +392,6 @@ template <bool MASKED>
 int nfft_cluster(int logL, const double *t, const float *y, int n, const PhaseMul &pm, const AccParams<float> &e,
                  const FftDev<float> &f, float2 *F, int nslab, cudaStream_t st) {
   switch (logL) {
-    case 12: return nfft_cluster_at<12, MASKED>(t, y, n, pm, e, f, F, nslab, st);
     case 13: return nfft_cluster_at<13, MASKED>(t, y, n, pm, e, f, F, nslab, st);
     case 14: return nfft_cluster_at<14, MASKED>(t, y, n, pm, e, f, F, nslab, st);
     case 15: return nfft_cluster_at<15, MASKED>(t, y, n, pm, e, f, F, nslab, st);

@@ -108,11 +108,8 @@ template <int R, typename C> __device__ __forceinline__ void dftR(C *v) {
 
 // One Stockham stage of radix R over nseq sequences of length 2^logL stored
 // at s[seq*pitch + pad16(i)].  Ns = 2^logNs is the length already
-// transformed.  tw[q] = exp(+2 pi i q / L).  PROD (radix 16): six table reads
-// w_1..w_3, w_4, w_8, w_12 and their products instead of fifteen reads (one
-// rounding more per twiddle), for tables that do not stay in the L1 beside the
-// sequence.
-template <typename T, int R, bool PROD>
+// transformed.  tw[q] = exp(+2 pi i q / L).
+template <typename T, int R>
 __device__ __forceinline__ void fft_stage(typename CxOf<T>::type *s, int pitch, int logL,
                                           int logNs, int total_bf,
                                           const typename CxOf<T>::type *__restrict__ tw) {
@@ -134,24 +131,8 @@ __device__ __forceinline__ void fft_stage(typename CxOf<T>::type *s, int pitch, 
       for (int r = 0; r < R; ++r) v[u][r] = base[pad16(j + (r << logLR))];
       if (logNs > 0) {
         const int k = j & maskNs;
-        if constexpr (PROD && R == 16) {
-          C wa[4];
 #pragma unroll
-          for (int a = 1; a < 4; ++a) {
-            wa[a] = ldtw(&tw[(a * k) << twsh]);
-            v[u][a] = cmul(v[u][a], wa[a]);
-          }
-#pragma unroll
-          for (int b = 4; b < R; b += 4) {
-            const C wb = ldtw(&tw[(b * k) << twsh]);
-            v[u][b] = cmul(v[u][b], wb);
-#pragma unroll
-            for (int a = 1; a < 4; ++a) v[u][a + b] = cmul(v[u][a + b], cmul(wa[a], wb));
-          }
-        } else {
-#pragma unroll
-          for (int r = 1; r < R; ++r) v[u][r] = cmul(v[u][r], ldtw(&tw[(r * k) << twsh]));
-        }
+        for (int r = 1; r < R; ++r) v[u][r] = cmul(v[u][r], ldtw(&tw[(r * k) << twsh]));
       }
       dftR<R>(v[u]);
     }
@@ -174,7 +155,7 @@ __device__ __forceinline__ void fft_stage(typename CxOf<T>::type *s, int pitch, 
 
 // Inverse FFT of nseq sequences of length 2^logL held in shared memory.  All
 // threads of the block must call it; blockDim.x * kFftE >= nseq * L.
-template <typename T, bool PROD = false>
+template <typename T>
 __device__ void smem_fft(typename CxOf<T>::type *s, int pitch, int logL, int nseq,
                          const typename CxOf<T>::type *__restrict__ tw) {
   if (logL == 0) return;
@@ -182,13 +163,13 @@ __device__ void smem_fft(typename CxOf<T>::type *s, int pitch, int logL, int nse
   if (r0 == 0) r0 = 4;
   const int total = nseq << logL;
   switch (r0) {
-    case 1: fft_stage<T, 2, PROD>(s, pitch, logL, 0, total >> 1, tw); break;
-    case 2: fft_stage<T, 4, PROD>(s, pitch, logL, 0, total >> 2, tw); break;
-    case 3: fft_stage<T, 8, PROD>(s, pitch, logL, 0, total >> 3, tw); break;
-    default: fft_stage<T, 16, PROD>(s, pitch, logL, 0, total >> 4, tw); break;
+    case 1: fft_stage<T, 2>(s, pitch, logL, 0, total >> 1, tw); break;
+    case 2: fft_stage<T, 4>(s, pitch, logL, 0, total >> 2, tw); break;
+    case 3: fft_stage<T, 8>(s, pitch, logL, 0, total >> 3, tw); break;
+    default: fft_stage<T, 16>(s, pitch, logL, 0, total >> 4, tw); break;
   }
   for (int logNs = r0; logNs < logL; logNs += 4)
-    fft_stage<T, 16, PROD>(s, pitch, logL, logNs, total >> 4, tw);
+    fft_stage<T, 16>(s, pitch, logL, logNs, total >> 4, tw);
 }
 
 // ---------------------------------------------------------------------------

@@ -339,3 +339,39 @@ def test_double_lomb_scargle_scales(mods, e):
     dy = torch.as_tensor(rng.uniform(0.2, 0.6, n), device="cuda")
     P, Q = (lomb_scargle(t, v, dy, nfreq=5000, df=1 / 500.0, t0=0.0, R=4, m=12) for v in (y, y * 2.0 ** e))
     assert rel_l2(Q.cpu().numpy(), P.cpu().numpy()) < 1e-12
+
+
+def _direct(t, y, T, nf):
+    """F_k, k = -nf/2 .. nf/2 - 1, of one series by 64-bit sums."""
+    x = t / T - 0.5
+    k = torch.arange(-(nf // 2), nf // 2, device="cuda", dtype=torch.float64)
+    ph = k[:, None] * x[None, :]
+    return (y.double() * torch.exp(2j * np.pi * (ph - ph.round()))).sum(dim=1)
+
+
+@pytest.mark.parametrize("n,nf,R,m,bound", [(1000, 2048, 2, 8, 2.13e-7), (500, 512, 2, 8, 2.11e-7), (700, 1024, 4, 6, 1.43e-7),
+                                            (300, 2048, 4, 12, 1.38e-7), (2000, 1024, 4, 12, 1.39e-7),
+                                            (3001, 4096, 2, 8, 2.24e-7)])
+def test_short_float_error(mods, n, nf, R, m, bound):
+    """Mean relative error of short float transforms against 64-bit sums over
+    16 uniform series: one CTA or one cluster each, in a batch of 16 (an SM
+    each) and of 160 (SMs shared; R = 4: gathered and scattered).  Bounds: the
+    mean of 32 series by the scatter with running products and full twiddle
+    tables, and two standard errors of this mean (2.5 %)."""
+    _, nfft = mods
+    T, B, S = 5.0, 160, 16
+    plan = nfft.AdjointNFFT(nf, R, m)
+    rng = np.random.default_rng(n)
+    ts = [torch.as_tensor(np.sort(rng.uniform(0, T, n)), device="cuda") for _ in range(S)]
+    ys = [torch.as_tensor(rng.normal(0, 1, n), device="cuda").float() for _ in range(S)]
+    X = [_direct(t, y, T, nf) for t, y in zip(ts, ys)]
+
+    def error(F):
+        return np.mean([float((f.to(torch.complex128) - x).abs().square().sum().sqrt() / x.abs().square().sum().sqrt())
+                        for f, x in zip(F, X)])
+
+    def batch(B):
+        p = nfft.BatchAdjointNFFT(np.full(B, n), np.full(B, nf), R, m, np.zeros(B), np.full(B, T))
+        return p(torch.cat(ts * (B // S)), torch.cat(ys * (B // S))).view(B, nf)[:S]
+    for F in ([plan(t, y, 0.0, T) for t, y in zip(ts, ys)], batch(S), batch(B)):
+        assert error(F) < 1.025 * bound
