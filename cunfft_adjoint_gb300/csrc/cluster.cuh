@@ -200,12 +200,21 @@ __device__ __forceinline__ void cluster_gather(int TC, const SRec<float> *list, 
     float a[4] = {0.f, 0.f, 0.f, 0.f};
     int r = start[g] + part;
     SRec<float> q = sorted[r];  // up to 2 step - 1 beyond the last record, in the array
-    for (; r < re; r += step) {
-      const SRec<float> nx = sorted[r + step];
-      const int rel = q.lc - cl0;
-      if constexpr (ONE >= 0) gauss_acc4<ONE>(q.y, m - rel, q.f, k1, m, a);
-      else gauss_acc<float, 4, MASKED>(q.y, (float)(m - rel) - q.f, k1, gw, rel, 2 * m, a);
-      q = nx;
+    // sums of up to 32 records: a thousand samples in a few cells lose to one
+    // long sum (10000 in 60 cells: 8e-7 of the spectrum, 3e-7 here; 0.2 us of a
+    // transform of 10000 uniform ones)
+    while (r < re) {
+      const int rs = min(re, r + 32 * step);
+      float b[4] = {0.f, 0.f, 0.f, 0.f};
+      for (; r < rs; r += step) {
+        const SRec<float> nx = sorted[r + step];
+        const int rel = q.lc - cl0;
+        if constexpr (ONE >= 0) gauss_acc4<ONE>(q.y, m - rel, q.f, k1, m, b);
+        else gauss_acc<float, 4, MASKED>(q.y, (float)(m - rel) - q.f, k1, gw, rel, 2 * m, b);
+        q = nx;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] += b[i];
     }
     for (int o = 1; o < step; o <<= 1) {  // a group's threads are in one warp
 #pragma unroll

@@ -375,3 +375,22 @@ def test_short_float_error(mods, n, nf, R, m, bound):
         return p(torch.cat(ts * (B // S)), torch.cat(ys * (B // S))).view(B, nf)[:S]
     for F in ([plan(t, y, 0.0, T) for t, y in zip(ts, ys)], batch(S), batch(B)):
         assert error(F) < 1.025 * bound
+
+
+def test_short_float_burst_error(mods):
+    """10000 samples in 60 of 2^15 cells, a thousand and more terms per cell:
+    mean error of 16 series against 64-bit sums.  Bound: the tiled gather's, which
+    adds up chunks of at most 1024 records, 4.9e-7 (standard deviation of one
+    series 1.2e-7; one sum per cell gives 8e-7)."""
+    _, nfft = mods
+    n, nf, T = 10_000, 1 << 14, 5.0
+    plan = nfft.AdjointNFFT(nf, 2, 8)
+    e = []
+    for seed in range(16):
+        rng = np.random.default_rng(seed)
+        t = torch.as_tensor((0.375 + rng.uniform(0, 60, n) / (2 * nf)) * T, device="cuda")
+        y = torch.as_tensor(rng.normal(0, 1, n), device="cuda").float()
+        X = _direct(t, y, T, nf)
+        F = plan(t, y, 0.0, T).to(torch.complex128)
+        e.append(float((F - X).abs().square().sum().sqrt() / X.abs().square().sum().sqrt()))
+    assert np.mean(e) < 4.9e-7
