@@ -151,9 +151,20 @@ __global__ void __launch_bounds__(kLsPowerThreads) k_ls_power(const typename CxO
   P[k] = ls_value(A[K + q], B[K + q], B[K + 2 * q], yy);
 }
 
+// The plans of one stream, as its workspace: the caller never sees them, so
+// calls on two streams must not share the records and grids of one.  The mutex
+// is held while a call is enqueued: another thread's call on the same stream
+// uses the same buffers and comes after all of it.
+struct LsStream {
+  std::mutex mu;
+  std::map<std::tuple<int, int64_t, int, int>, cuna2_plan> plans;  // (dtype, nf, R, m)
+};
 std::mutex g_ls_mu;
-std::map<std::tuple<int, int, int64_t, int, int>, cuna2_plan> *g_ls_plans =
-    new std::map<std::tuple<int, int, int64_t, int, int>, cuna2_plan>();
+std::map<std::pair<int, cudaStream_t>, LsStream> *g_ls = new std::map<std::pair<int, cudaStream_t>, LsStream>();
+LsStream &ls_stream(int dev, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_ls_mu);
+  return (*g_ls)[std::make_pair(dev, st)];  // never erased: the reference stays valid
+}
 
 template <typename T>
 int ls_run(int dtype, const double *t, const T *y, const T *dy, int64_t n, int64_t nfreq, double df, double t0,
@@ -167,17 +178,16 @@ int ls_run(int dtype, const double *t, const T *y, const T *dy, int64_t n, int64
   while (nf / 2 <= 2 * nfreq) nf *= 2;
   int dev = 0;
   CUNA_CK(cudaGetDevice(&dev));
+  LsStream &ls = ls_stream(dev, st);
+  std::lock_guard<std::mutex> lk(ls.mu);
   cuna2_plan plan = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g_ls_mu);
-    auto key = std::make_tuple(dev, dtype, nf, R, m);
-    auto it = g_ls_plans->find(key);
-    if (it == g_ls_plans->end()) {
-      CUNA_TRY(cuna2_plan_create(&plan, dtype, nf, R, m));
-      (*g_ls_plans)[key] = plan;
-    } else {
-      plan = it->second;
-    }
+  const auto key = std::make_tuple(dtype, nf, R, m);
+  const auto it = ls.plans.find(key);
+  if (it == ls.plans.end()) {
+    CUNA_TRY(cuna2_plan_create(&plan, dtype, nf, R, m));
+    ls.plans[key] = plan;
+  } else {
+    plan = it->second;
   }
   // workspace: partial sums | channels [wy; w] | outputs [A; B]
   const int np = (int)std::min<int64_t>(std::min(kLsMaxBlocks, 4 * device_sm_count()), (n + kLsThreads - 1) / kLsThreads);

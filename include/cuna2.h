@@ -196,7 +196,8 @@ int cuna2_adjoint_multi(cuna2_plan plan, const double *t, const void *y, void *F
  * f_k = (k + 1) df, k < nfreq, written to power (nfreq values of dtype).
  * Built on one two-channel adjoint NFFT (weighted centred values and
  * weights) with period 1/df, Nf the smallest power of two > 4 nfreq,
- * oversampling R and half-width m.  Plans are cached per (device, size). */
+ * oversampling R and half-width m.  Plans are cached per device, stream and
+ * size, so calls on several streams may overlap. */
 int cuna2_lomb_scargle(int dtype, const double *t, const void *y, const void *dy, int64_t n,
                        int64_t nfreq, double df, double t0, int R, int m, void *power,
                        cudaStream_t stream);

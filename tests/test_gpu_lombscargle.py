@@ -71,3 +71,25 @@ def test_lomb_scargle_vs_direct(mods, dtype, tol):
     assert rel_l2(P.cpu().numpy(), D) < tol
     # the injected period is the highest peak
     assert abs(freqs[int(np.argmax(P.cpu().numpy()))] - 1 / 2.1) < 2 * df
+
+
+@pytest.mark.parametrize("n,nfreq", [(40_000, 20_000), (3000, 20_000)])
+def test_lomb_scargle_on_two_streams(mods, n, nfreq):
+    """Periodograms of one size enqueued alternately on two streams, several in
+    flight, equal those of one stream (double: integer sums on the grid and
+    partial sums added up in order, so the same bits)."""
+    _, ls = mods
+    rng = np.random.default_rng(n)
+    data = [(torch.as_tensor(np.sort(rng.uniform(0, 100.0, n)), device="cuda"),
+             torch.as_tensor(rng.normal(0, 1, n), device="cuda")) for _ in range(2)]
+    want = [ls.lomb_scargle(t, y, None, nfreq=nfreq, df=1 / 500.0, t0=0.0, R=4, m=12) for t, y in data]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    out = [[torch.empty(nfreq, dtype=torch.float64, device="cuda") for _ in range(8)] for _ in range(2)]
+    torch.cuda.synchronize()
+    for i in range(8):
+        for (t, y), s, o in zip(data, streams, out):
+            ls.lomb_scargle(t, y, None, nfreq=nfreq, df=1 / 500.0, t0=0.0, R=4, m=12, out=o[i], stream=s)
+    torch.cuda.synchronize()
+    for w, o in zip(want, out):
+        assert all(torch.equal(w, x) for x in o)
