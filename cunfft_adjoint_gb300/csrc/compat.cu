@@ -83,10 +83,11 @@ __global__ void __launch_bounds__(kFilterThreads) k_compat_filter_f32(cuna2_filt
 }
 
 // a / b from r, the reciprocal of b: one correction of the quotient by its exact
-// remainder (Markstein 1990), the correctly rounded quotient for ordinary values
+// remainder (Markstein 1990), the correctly rounded quotient for ordinary
+// values; b is infinite (r = 0) on grids of n / 2 cells
 __device__ __forceinline__ double div_by(double a, double b, double r) {
   const double q = a * r;
-  return fma(fma(-q, b, a), r, q);
+  return r == 0.0 ? q : fma(fma(-q, b, a), r, q);
 }
 // The FP64 pipe bounds this kernel: the square root and the two reciprocals that
 // all samples share are one warp's work (1e5 samples: 15.8 us, 13.3 here).

@@ -394,3 +394,18 @@ def test_short_float_burst_error(mods):
         F = plan(t, y, 0.0, T).to(torch.complex128)
         e.append(float((F - X).abs().square().sum().sqrt() / X.abs().square().sum().sqrt()))
     assert np.mean(e) < 4.9e-7
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [2047, 2048, 2049])
+def test_compat_filter_at_half_the_samples(mods, oracle_lib, dt, n):
+    """Filter coefficients around ng = n / 2, where the reference's b changes sign
+    through infinity: E1 and E2 as the reference's expressions give them (NaN
+    for a negative b, 0 and 1 for an infinite one).  Tolerances of the filter's
+    parity test: 3e-5 and 1e-14."""
+    cuna, _ = mods
+    x = np.random.default_rng(n).uniform(-0.5, 0.5, n).astype(dt)
+    fp = cuna.generate_filter_properties(torch.as_tensor(x, device="cuda"), n, 1024)
+    _, _, _, E1, E2, _ = oracle_lib.compat_filter(x, 1024, "f" if dt == np.float32 else "d")
+    for got, want in ((fp.E1, E1), (fp.E2, E2)):
+        np.testing.assert_allclose(got[:n].cpu().numpy(), want, rtol=3e-5 if dt == np.float32 else 1e-14)
