@@ -54,8 +54,10 @@ struct cuna2_plan_st {
   bool has_split = false;
   bool tiled_single = true;
   // float plans of middling length: a short single transform in one cluster
-  // launch (cluster.cuh), until the caller chooses a schedule
-  bool cluster = false;
+  // launch (cluster.cuh) where cluster_takes its number of samples, unless the
+  // caller chose a schedule or the sort of k_bin_local, or the autotuner found
+  // another path faster for such a series
+  bool has_cluster = false, cluster = false, local_asked = false;
   cuna::FftGeom geom_cl;
   cuna::FftGeom geom4;
   // double plans with four-step passes: the float-float geometry the passes
@@ -266,7 +268,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   // over many CTAs when they can; many slabs take one CTA each
   bool clus = false;
   if constexpr (sizeof(T) == 4)
-    clus = p->cluster && cluster_takes(p->geom.logL, n, nslab) && p->binning == CUNA2_BIN_GLOBAL && !bo && !grep;
+    clus = p->cluster && !p->local_asked && cluster_takes(p->geom.logL, n, nslab) && !bo && !grep;
   const bool small = !clus && p->small && !(p->has_split && p->tiled_single && 2 * nslab <= device_sm_count());
   const FftDev<T> f = to_dev<T>(small || !p->small ? p->geom : p->geom4);
   const int L = 1 << p->geom.logL;
@@ -643,7 +645,7 @@ extern "C" int cuna2_plan_create(cuna2_plan *plan, int dtype, int64_t nf, int R,
     delete p;
     return st;
   }
-  p->cluster = dtype == CUNA2_F32 && cluster_fits(logL, m);
+  p->has_cluster = p->cluster = dtype == CUNA2_F32 && cluster_fits(logL, m);
   if (p->cluster && logL >= kClusterLo && (st = fft_geometry(false, logL, &p->geom_cl, logL <= kSingleLogF32))) {
     delete p;
     return st;
@@ -1006,11 +1008,16 @@ extern "C" int cuna2_plan_autotune(cuna2_plan p, const double *t, const void *y,
     flush = nullptr;
   }
   int s = CUNA2_SUCCESS;
-  bool best_cluster = false;
-  if (p->cluster && cluster_takes(p->geom.logL, n, 1)) {
-    s = time_schedule(p, t, y, F, n, t0, T, st, reps, flush, flush_bytes, &best);
-    best_cluster = !s;
-  }
+  // The cluster path runs by the number of samples, so it keeps the short
+  // series of the plan unless it loses at one of them; the other paths are
+  // chosen among themselves for every longer one.
+  bool best_cluster = p->has_cluster;
+  float cluster_ms = 3.4e38f;
+  const bool had_cluster = p->cluster, had_local = p->local_asked;
+  p->local_asked = false;
+  p->cluster = p->has_cluster;
+  if (p->cluster && cluster_takes(p->geom.logL, n, 1))
+    s = time_schedule(p, t, y, F, n, t0, T, st, reps, flush, flush_bytes, &cluster_ms);
   p->cluster = false;
   if (!s && p->small) {  // the single-CTA path: no tiles to choose
     const bool keep = p->tiled_single;
@@ -1020,7 +1027,7 @@ extern "C" int cuna2_plan_autotune(cuna2_plan p, const double *t, const void *y,
     p->tiled_single = keep;
     if (!s && ms < best) {
       best = ms;
-      best_tiled = best_cluster = false;
+      best_tiled = false;
     }
   }
   if (!s && (!p->small || p->has_split)) {  // tiled schedules
@@ -1042,9 +1049,12 @@ extern "C" int cuna2_plan_autotune(cuna2_plan p, const double *t, const void *y,
             best_method = method;
             best_bin = bin;
             best_tiled = true;
-            best_cluster = false;
           }
         }
+  }
+  if (cluster_ms < 3.4e38f) {
+    best_cluster = cluster_ms <= best;
+    best = std::min(best, cluster_ms);
   }
   drop_graphs(p);
   p->logTL = best_tile;
@@ -1057,7 +1067,11 @@ extern "C" int cuna2_plan_autotune(cuna2_plan p, const double *t, const void *y,
     cudaStreamSynchronize(st);
     cudaFree(flush);
   }
-  if (s) return s;
+  if (s) {
+    p->cluster = had_cluster;
+    p->local_asked = had_local;
+    return s;
+  }
   if (best_ms) *best_ms = best;
   return CUNA2_SUCCESS;
 }
@@ -1116,8 +1130,9 @@ extern "C" int cuna2_plan_set_binning(cuna2_plan p, int mode) {
   if (mode != CUNA2_BIN_GLOBAL && mode != CUNA2_BIN_LOCAL)
     return fail(CUNA2_ERROR_INVALID_VALUE, "binning mode %d", mode);
   std::lock_guard<std::mutex> lk(p->mu);
-  if (mode != p->binning) drop_graphs(p);
+  if (mode != p->binning || p->cluster) drop_graphs(p);
   p->binning = mode;
+  p->local_asked = mode == CUNA2_BIN_LOCAL;
   return CUNA2_SUCCESS;
 }
 

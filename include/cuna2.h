@@ -287,9 +287,11 @@ int cuna2_plan_time_grid(cuna2_plan plan, const double *t, const void *y, void *
  * 2^log_tile >= 2m.
  * New plans start at (11, CUNA2_GRID_GATHER) for float and (12,
  * CUNA2_GRID_FIXED) for double (a grid of at most 8192 cells is one tile).
- * Short float transforms (n <= 16384, R nf <= 2^16 cells; see cluster.cuh) run
- * in one launch without tiles until a schedule is set or autotuned.  Changing
- * the schedule drops the plan's cached graphs.  No counterpart in the reference
+ * Most short float transforms (up to 16384 samples and 2^16 cells, n R nf at
+ * most 2^29, and few channels or resamples: cluster_takes in cluster.cuh) run
+ * in one launch without tiles, until a schedule or CUNA2_BIN_LOCAL is set; the
+ * autotuner keeps that for them unless another path is faster on such a
+ * series.  Changing the schedule drops the plan's cached graphs.  No counterpart in the reference
  * (its gridding kernel, src/gridding.cu:36-65, has a fixed launch shape). */
 enum { CUNA2_GRID_GATHER = 0, CUNA2_GRID_SCATTER = 1, CUNA2_GRID_FIXED = 2 };
 int cuna2_plan_set_schedule(cuna2_plan plan, int log_tile, int grid_method);
@@ -325,8 +327,9 @@ int cuna2_plan_get_binning(cuna2_plan plan, int *mode);
  * taken, with a buffer of twice the L2 size overwritten before each run so
  * the inputs come from HBM), and keeps the fastest; best_ms (may be NULL)
  * receives its time.  Allocates and frees that buffer; synchronises
- * `stream`.  Plans small enough for the single-CTA path have nothing to tune
- * and keep their schedule. */
+ * `stream`.  Series that the one-launch path of short transforms takes are also
+ * timed on it; longer ones leave it to such series.  Plans small enough for the
+ * single-CTA path have no schedule to tune and keep theirs. */
 int cuna2_plan_autotune(cuna2_plan plan, const double *t, const void *y, void *F, int64_t n,
                         double t0, double T, cudaStream_t stream, int reps, float *best_ms);
 

@@ -409,3 +409,44 @@ def test_compat_filter_at_half_the_samples(mods, oracle_lib, dt, n):
     _, _, _, E1, E2, _ = oracle_lib.compat_filter(x, 1024, "f" if dt == np.float32 else "d")
     for got, want in ((fp.E1, E1), (fp.E2, E2)):
         np.testing.assert_allclose(got[:n].cpu().numpy(), want, rtol=3e-5 if dt == np.float32 else 1e-14)
+
+
+def _stages(plan, t, y, T):
+    import ctypes
+    from cunfft_adjoint_gb300 import _lib
+    F = torch.empty(plan.nf, dtype=torch.complex64, device="cuda")
+    ms, names, k = (ctypes.c_float * 16)(), (ctypes.c_char_p * 16)(), ctypes.c_int()
+    _lib.check(_lib.core().cuna2_plan_profile(plan._h, t.data_ptr(), y.data_ptr(), F.data_ptr(), t.numel(), 0.0, T, None,
+                                              ms, names, 16, ctypes.byref(k)))
+    return [names[i].decode() for i in range(k.value)]
+
+
+def test_autotune_leaves_short_series_their_path(mods):
+    """The one-launch path runs by the number of samples: tuning on a long series
+    chooses among the others and leaves short ones on it, also after a chosen
+    schedule or the local sort had turned it off; spectra of both against the
+    double plan (float rounding, 2e-6)."""
+    from cunfft_adjoint_gb300 import _lib
+    _, nfft = mods
+    rng = np.random.default_rng(3)
+    nf, T = 1 << 14, 5.0
+    (ts, ys), (tl, yl) = (((torch.as_tensor(rng.uniform(0, T, n), device="cuda"),
+                            torch.as_tensor(rng.normal(0, 1, n), device="cuda").float())) for n in (9000, 40_000))
+    plan, ref = nfft.AdjointNFFT(nf, 2, 8), nfft.AdjointNFFT(nf, 2, 8, torch.float64)
+
+    def check(cluster):
+        assert ("nfft_cluster" in _stages(plan, ts, ys, T)) == cluster
+        assert "nfft_cluster" not in _stages(plan, tl, yl, T)
+        for t, y in ((ts, ys), (tl, yl)):
+            assert rel_l2(plan(t, y, 0.0, T).cpu().numpy(), ref(t, y.double(), 0.0, T).cpu().numpy()) < 2e-6
+    check(True)
+    plan.autotune(tl, yl, 0.0, T, reps=2)
+    check(True)
+    plan.set_schedule(11, _lib.GRID_GATHER)
+    check(False)
+    plan.autotune(tl, yl, 0.0, T, reps=2)
+    check(True)
+    plan.binning = 1
+    check(False)
+    plan.binning = 0
+    check(True)
