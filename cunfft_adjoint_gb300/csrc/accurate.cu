@@ -111,6 +111,7 @@ template <typename T> AccParams<T> make_params(const cuna2_plan_st *p) {
   e.c0 = (T)(0.5 / sqrt(4.0 * kPi * tau));
   e.c1 = (T)(4.0 * kPi * kPi * tau / ((double)p->ng * (double)p->ng));
   e.twk = (T)(2.0 / (double)p->ng);
+  e.masks = !tail_free_gather(sizeof(T) == 4, p->m, tau) || masked_gather_forced();
   return e;
 }
 
@@ -352,7 +353,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   if (nbs > 0 && !one) CUNA_TRY(boot_weights(false));
   if constexpr (sizeof(T) == 4) {
     if (clus) {
-      const bool masked = !tail_free_gather(true, p->m, p->tau) || masked_gather_forced();
+      const bool masked = e.masks;
       const float *v = wts ? wts : y;
       const int logL = p->geom.logL;
       if (logL < kClusterLo) {
@@ -513,7 +514,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
       const T *wc = wts;
       const int64_t nv = n, sstr = p->ng;
       cudaError_t le;
-      const bool free_ = tail_free_gather(sizeof(T) == 4, p->m, p->tau) && !masked_gather_forced();
+      const bool free_ = !e.masks;
       if (p->grid_method == CUNA2_GRID_GATHER && cw8 && wts && group >= 2) {
         const size_t sm4 = grid_smem_bytes<T>(p->logTL, p->m, 4);
         if (free_) le = launch_pdl(k_grid_acc_sg4<T, false>, ggrid, gb, sm4, st, rc, oc, grid, e, wc, nv, nslab, group, sstr);

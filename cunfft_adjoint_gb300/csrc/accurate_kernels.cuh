@@ -46,6 +46,7 @@ template <typename T> struct AccParams {
   T e3c;              // E3[d] = exp(e3c d^2)
   T c0, c1;           // 0.5 / psi_hat(k) = c0 exp(c1 k^2)
   T twk;              // 2 / ng  (unpack twiddle angle / pi)
+  bool masks;         // the gather masks a record's taps (tail_free_gather)
 };
 
 // fractional cell from the low word of S*ng
@@ -541,8 +542,7 @@ __device__ __forceinline__ void small_grid_gather(const double *__restrict__ t, 
                                                   const PhaseMul &pm, const AccParams<float> &e, float *sr,
                                                   SRec<float> *srec, int *order, int *start, int cap) {
   const int ng = (int)e.ng, NG = ng / 4, m = e.m;
-  // as tail_free_gather: exp(-m^2 / (4 tau)) < 1e-8
-  const bool masked = e.k1 * (float)(m * m) < 26.6f, poly = e.ng >= 4 * e.nf;
+  const bool masked = e.masks, poly = e.ng >= 4 * e.nf;
   // Where there are fewer groups than threads, 2^LP threads share a group's
   // records (NG is a power of two: with LP > 0 either all threads have a group
   // or, at LP = 5, whole warps have none).

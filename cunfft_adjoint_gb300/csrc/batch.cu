@@ -249,6 +249,7 @@ template <typename T> AccParams<T> series_params(int64_t nf, int R, int m, doubl
   e.c0 = (T)(0.5 / sqrt(4.0 * kPi * tau));
   e.c1 = (T)(4.0 * kPi * kPi * tau / ((double)ng * (double)ng));
   e.twk = (T)(2.0 / (double)ng);
+  e.masks = !tail_free_gather(sizeof(T) == 4, m, tau) || masked_gather_forced();
   return e;
 }
 

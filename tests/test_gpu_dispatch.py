@@ -450,3 +450,43 @@ def test_autotune_leaves_short_series_their_path(mods):
     check(False)
     plan.binning = 0
     check(True)
+
+
+_MASKS_SCRIPT = """
+import sys
+import numpy as np, torch
+sys.path.insert(0, sys.argv[1])
+from cunfft_adjoint_gb300 import nfft
+t = torch.tensor([1.2345], dtype=torch.float64, device="cuda")
+y = torch.ones(1, device="cuda")
+out = {}
+for nf, m in ((2048, 8), (2048, 5), (1 << 14, 8)):
+    out["plan_%d_%d" % (nf, m)] = nfft.AdjointNFFT(nf, 2, m)(t, y, 0.0, 3.0).cpu().numpy()
+b = nfft.BatchAdjointNFFT(np.ones(2, int), np.full(2, 2048), 2, 8, np.zeros(2), np.full(2, 3.0))
+out["batch_2048_8"] = b(t.repeat(2), y.repeat(2)).cpu().numpy()
+np.savez(sys.argv[2], **out)
+"""
+
+
+def test_masks_switch_reaches_every_gather(tmp_path, native_built):
+    """CUNA2_GATHER_MASKS=1 keeps the tap masks in the one-CTA, cluster and batch
+    gathers too: one sample's spectrum (no order of sums) differs in some bits
+    from that of whole cell groups, whose cells beyond the window hold below 1e-8
+    of the peak (m = 8), and by no more than float rounding; m = 5 keeps the
+    masks either way."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    script = tmp_path / "masks.py"
+    script.write_text(_MASKS_SCRIPT)
+    res = []
+    for v in "01":
+        out = tmp_path / ("masks%s.npz" % v)
+        r = subprocess.run([sys.executable, str(script), root, str(out)], env={**os.environ, "CUNA2_GATHER_MASKS": v},
+                           capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-2000:]
+        res.append(np.load(out))
+    for key in res[0].files:
+        assert rel_l2(res[0][key], res[1][key]) < 1e-6, key
+        assert np.array_equal(res[0][key], res[1][key]) == key.endswith("_5"), key
