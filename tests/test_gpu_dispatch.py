@@ -490,3 +490,48 @@ def test_masks_switch_reaches_every_gather(tmp_path, native_built):
     for key in res[0].files:
         assert rel_l2(res[0][key], res[1][key]) < 1e-6, key
         assert np.array_equal(res[0][key], res[1][key]) == key.endswith("_5"), key
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dtype,n,nf,R,m", [(torch.float32, 300, 512, 2, 8), (torch.float32, 500, 1024, 4, 6),
+                                            (torch.float32, 2000, 2048, 2, 8), (torch.float32, 9000, 1 << 14, 2, 8),
+                                            (torch.float32, 20_000, 1 << 17, 2, 8), (torch.float64, 800, 1 << 11, 2, 10),
+                                            (torch.float64, 9000, 1 << 15, 2, 10)])
+def test_non_finite_values(mods, bad, dtype, n, nf, R, m):
+    """A non-finite value spreads over the spectrum of its own series and no
+    other's: one transform (one CTA, one cluster, tiled), the other channel, the
+    other series of a batch (an SM each and shared); its gradients stay with
+    the sample or the series it belongs to, the others keep their bits or, where
+    the order of sums is free, float rounding."""
+    _, nfft = mods
+    rng = np.random.default_rng(n)
+    T, B = 5.0, 3
+    t = torch.as_tensor(rng.uniform(0, T, (B, n)), device="cuda")
+    y = torch.as_tensor(rng.normal(0, 1, (B, n)), device="cuda").to(dtype)
+    w = y.clone()
+    w[1, n // 2] = bad
+    plan = nfft.AdjointNFFT(nf, R, m, dtype)
+
+    def lost(F):
+        return bool((~torch.isfinite(torch.view_as_real(F)).all(dim=-1)).all())
+
+    def near(a, b):
+        return rel_l2(a.cpu().numpy(), b.cpu().numpy()) < (1e-6 if dtype == torch.float32 else 1e-13)
+    assert lost(plan(t[1], w[1], 0.0, T))
+    F, M = plan(t[1], y[2], 0.0, T).clone(), plan.multi(t[1], w[1:], 0.0, T)
+    assert lost(M[0]) and near(M[1], F)
+    for reps in (1, 60):
+        batch = nfft.BatchAdjointNFFT(np.full(B * reps, n), np.full(B * reps, nf), R, m, np.zeros(B * reps),
+                                      np.full(B * reps, T), dtype)
+        G, H = (batch(t.repeat(reps, 1), v.repeat(reps, 1)).view(-1, nf) for v in (y, w))
+        assert lost(H[1]) and near(H[0], G[0]) and near(H[2], G[2])
+    g = torch.as_tensor(rng.normal(0, 1, (B, nf)) + 1j * rng.normal(0, 1, (B, nf)), device="cuda").to(plan.cdtype)
+    gy, gt = plan.backward_batch(t, y, g, 0.0, T)
+    hy, ht = plan.backward_batch(t, w, g, 0.0, T)
+    assert torch.equal(gy, hy) and not torch.isfinite(ht[1, n // 2])
+    ok = torch.isfinite(ht)
+    assert int((~ok).sum()) == 1 and torch.equal(ht[ok], gt[ok])
+    g[1, 3] = bad
+    hy, ht = plan.backward_batch(t, y, g, 0.0, T)
+    assert not torch.isfinite(hy[1]).any() and not torch.isfinite(ht[1]).any()
+    assert torch.equal(hy[::2], gy[::2]) and torch.equal(ht[::2], gt[::2])
