@@ -269,7 +269,7 @@ int adjoint_run(cuna2_plan_st *p, const double *t, const T *y, typename CxOf<T>:
   // over many CTAs when they can; many slabs take one CTA each
   bool clus = false;
   if constexpr (sizeof(T) == 4)
-    clus = p->cluster && !p->local_asked && cluster_takes(p->geom.logL, n, nslab) && !bo && !grep;
+    clus = p->cluster && !p->local_asked && cluster_takes(p->geom.logL, p->R, n, nslab) && !bo && !grep;
   const bool small = !clus && p->small && !(p->has_split && p->tiled_single && 2 * nslab <= device_sm_count());
   const FftDev<T> f = to_dev<T>(small || !p->small ? p->geom : p->geom4);
   const int L = 1 << p->geom.logL;
@@ -1017,7 +1017,7 @@ extern "C" int cuna2_plan_autotune(cuna2_plan p, const double *t, const void *y,
   const bool had_cluster = p->cluster, had_local = p->local_asked;
   p->local_asked = false;
   p->cluster = p->has_cluster;
-  if (p->cluster && cluster_takes(p->geom.logL, n, 1))
+  if (p->cluster && cluster_takes(p->geom.logL, p->R, n, 1))
     s = time_schedule(p, t, y, F, n, t0, T, st, reps, flush, flush_bytes, &cluster_ms);
   p->cluster = false;
   if (!s && p->small) {  // the single-CTA path: no tiles to choose

@@ -3,7 +3,7 @@
 //
 // A short transform on the tiled path is a chain of four launches of a few CTAs
 // each, and their gaps and the host's enqueue are most of its time (n = 10000,
-// Nf = 16384: 19 us per call).  Here the steps are phases of one kernel between
+// Nf = 16384: 17.5 us per call).  Here the steps are phases of one kernel between
 // cluster barriers:
 //   1. each CTA takes an eighth of the samples and sends each one's record to
 //      the shared-memory list of the CTA whose run of ng/8 cells it touches
@@ -16,8 +16,9 @@
 //      their row pairs;
 //   4. row FFTs, unpack, deconvolution and centring, as ct_rowpass_body.
 // Grids of less than 2^13 points run phases 1 and 2 alike and leave the FFT to
-// the first CTA.  n = 10000, Nf = 16384: 19.0 us -> 13.5; with the records
-// exchanged through device memory instead, after an exchange of counts, 16.5.
+// the first CTA.  n = 10000, Nf = 16384: 17.5 -> 13.0 us per call; with the
+// records exchanged through device memory instead, after an exchange of counts,
+// 16.5.
 // What bounds it is the latency of its phases: the samples' loads and the
 // remote atomics 6 of about 20 thousand cycles, sort and gather 7, the FFT
 // passes with their remote accesses and the barriers the rest.
@@ -41,21 +42,24 @@ constexpr int kClusterSlack = 64;  // places after the sorted list that a gather
 // grid.  (2^12 points over the cluster take 2 us less, but its four-step FFT has
 // two more rounded products per point than the one-CTA FFT: 1.76e-7 of the
 // spectrum of n = 300, Nf = 2048, R = 4 against 1.38e-7.)
-constexpr int kClusterSmallN = 640, kClusterSmallN12 = 256;
+constexpr int kClusterSmallN = 700, kClusterSmallN12 = 500;
 
 // a record touches at most two runs of ng/8 cells
 inline bool cluster_fits(int logL, int m) { return logL <= kClusterHi && logL >= 4 && (1 << (logL - 2)) >= 2 * m; }
 // Measured against the other paths (us; n samples, 2^L packed points).  Below
 // 2^13 points one CTA does it all in less while the samples are few, on the
-// device: 2^9 points: n = 600 8.0 against 8.1 here, 700 8.7 and 8.2; 2^11: 600
-// 9.0 and 8.9, 1000 10.3 and 9.1; 2^12: 200 11.0 and 11.0, 300 11.4 and 11.0;
-// 10000 samples, 2^11: 47 against 12 per call.  Above, the tiled path, per call:
-// n = 10000, 2^14: 17.5 against 13.5 here; 2^15: n = 8000 17.8 against 16.4, n =
-// 16384 17.5 against 18.5; 2^16: n = 2000 17.5 against 18.5 -- eight SMs are too
-// few for the cells and samples from there on.
-inline bool cluster_takes(int logL, int64_t n, int nslab) {
-  return n <= kClusterN && nslab * kClusterCtas <= device_sm_count() &&
-         (logL < kClusterLo ? n > (logL == 12 ? kClusterSmallN12 : kClusterSmallN) : (n << logL) <= (1 << 28));
+// device, one CTA and here: R = 2, 2^9 points: n = 600 7.9 and 7.8, 700 8.3 and
+// 7.9; 2^11: 700 8.4 and 8.7, 900 8.8 and 8.8; 2^12: 400 11.0 and 11.1, 600 11.3
+// and 11.3, 1000 12.0 and 11.4; R = 4 (dearer weights), 2^10: 300 7.3 and 7.9,
+// 500 7.9 and 8.1; 2^11: 300 8.8 and 8.6, 500 9.5 and 8.7; 2^12: 200 11.3 and
+// 10.9.  Above, the tiled path, per call: n = 10000, 2^14: 17.5 against 13.0
+// here; 2^15: n = 8000 17.8 against 16.4, n = 16384 17.5 against 18.5; 2^16: n =
+// 2000 17.5 against 18.5 -- eight SMs are too few for the cells and samples
+// from there on.
+inline bool cluster_takes(int logL, int R, int64_t n, int nslab) {
+  if (n > kClusterN || nslab * kClusterCtas > device_sm_count()) return false;
+  if (logL >= kClusterLo) return (n << logL) <= (1 << 28);
+  return n > (logL == kClusterLo - 1 ? kClusterSmallN12 : kClusterSmallN) >> (R >= 4);
 }
 
 template <int LOGL> struct ClusterCfg {

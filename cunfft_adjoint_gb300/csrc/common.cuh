@@ -11,7 +11,10 @@ namespace cuna {
 // half an ulp; pairs split from a double by df_from_double are not), about
 // 48 significant bits.  The float64 plan's FFT passes and fixed-point taps
 // compute in it on the FP32 pipe (GB300's FP64 rate is a small fraction of
-// its FP32 rate) and keep double in memory.  Sums by Knuth's two-sum,
+// its FP32 rate); records and spectra are double in memory, a single plan's
+// fixed-point grid and the values between its passes float-float.  Values
+// outside the float range overflow, and below about 1e-30 the low floats lose
+// bits to underflow.  Sums by Knuth's two-sum,
 // products by an FMA-exact product (Dekker's method with fma), both
 // renormalised by a fast two-sum (Dekker 1971; Hida, Li, Bailey 2001).
 struct dfl {
@@ -268,12 +271,9 @@ cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, 
 // Fixed-point accumulation in shared memory: a value w (already scaled so
 // that every cell's sum stays within `range`) is rounded to an integer and
 // added with a native shared-memory integer atomic; integer sums do not
-// depend on the order of the atomics.  Double cells round by adding
-// 1.5 * 2^52 (the integer lands in the low mantissa bits; exact round to
-// nearest for |w| < 2^51), one FP64 add that the multiply before it fuses
-// into, instead of a conversion on the FP64 pipe (gridding of the large
-// float64 workload 354 -> 299 us); hence the 2^50 range, a quantum of 2^-50
-// of each tile's bound.
+// depend on the order of the atomics.  Double cells have a quantum of 2^-50 of
+// their tile's bound, about what a tap's float-float product carries; it is
+// split into its integers from the floats (tap_fix), without the FP64 pipe.
 template <typename T> struct FixAcc;
 template <> struct FixAcc<float> {
   typedef int type;
@@ -296,9 +296,6 @@ template <> struct FixAccWide<double> {
 template <> struct FixAcc<double> {
   typedef long long type;
   static constexpr double range = 1125899906842624.0;  // 2^50
-  __device__ static long long to_fix(double w) {
-    return __double_as_longlong(w + 6755399441055744.0) - 0x4338000000000000ll;
-  }
   __device__ static void add(long long *a, long long v) {
     atomicAdd(reinterpret_cast<unsigned long long *>(a), (unsigned long long)v);
   }
